@@ -1,0 +1,674 @@
+// segsum.cu -- sums over the segments of a contiguous array: segmented_reduce
+// (+) and the CSR SpMV with the default row split.
+//
+// Replaces the LoopSegRedOuter loop of segmented_reduce (Lowering.hs:874-944,
+// `schedule(dynamic)` per CodegenC.hs:1055-1057) and the generate-of-
+// reduce_generate of bench/spmv/spmv.hyd:30-40.  Both are the same problem: an
+// array of values cut by ascending offsets (the segment offsets; row_ptr), one
+// sum per piece.  For the SpMV a value is the product vals[k] * x[col[k]].
+//
+// Every warp takes one contiguous range of values, equal shares of all values
+// whatever the segments' lengths, and walks it in chunks of 256:
+//  * a run of chunks with no boundary (the end of a segment) in it is added
+//    into eight accumulators per lane, one operation per value;
+//  * a chunk with boundaries is summed by a segmented scan: each lane folds
+//    its 8 consecutive values, restarting at each head, one warp scan carries
+//    the sums across lanes, and the sum before each boundary is written out;
+//  * the sum of the piece that was open when the range began, and of the one
+//    open when it ends, go to per-warp partials.
+// A second kernel adds the partials of the pieces that cross warps (a warp per
+// piece, a fixed order).  There is no look-back, no atomic and no flag to wait
+// for; every order is fixed by the data, so results are identical over runs.
+//
+// What bounds it: FP64.  GB300 adds 5.3e11 doubles/s, 254 us for 2^27, against
+// 158 us for reading them.  Measured (start -> now): 2^27 float64 values in
+// segments of 2^U(0,16), 695 -> 317 us (3.4 TB/s); segments of 2^U(0,5), 783 ->
+// 579 us; of one value each, 1136 -> 1014 us.  Before, tiles of 4096 values took
+// 1.6 FP64 operations per value and waited for a look-back.  SpMV, 2^20 rows of
+// Zipf length, 12.9e6 entries: 198 -> 107 us; 8 lanes per row spent about seven
+// FP64 lane slots per entry.  Three blocks per SM (80 registers) beat four (64
+// and spills): 1014 against 1327 us on one-value segments.
+//
+// Offsets that are not an ascending partition of [0, n_vals] are detected on
+// the way (every adjacent pair is looked at by exactly one warp); the second
+// kernel then computes every segment on its own, with the reference's
+// semantics (an invalid segment yields init and is reported; a row takes
+// whatever its two row pointers span).
+#include <climits>
+
+#include "hyd_common.cuh"
+
+namespace hyd {
+
+constexpr int kSegT = 256;
+constexpr int kSegWarps = kSegT / 32;
+constexpr int kSegPer = 8;                  // consecutive values per lane
+constexpr int kSegC = 32 * kSegPer;         // values per chunk
+constexpr int kSegCounterWord = 240;              // stream counters: +0 invalid offsets, +1 finished blocks
+// where a chunk's sum i sits: free of bank conflicts for a lane's 8 consecutive values
+__device__ __forceinline__ int seg_slot(int i) { return i ^ ((i >> 4) & 7); }
+
+__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gsrc, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(smem_dst)),
+                 "l"(gsrc), "r"(bytes)
+                 : "memory");
+}
+// 16-byte units of a staged chunk: unit u sits at seg_unit(u), so that the
+// lanes' reads of their own consecutive units meet few bank conflicts
+__device__ __forceinline__ int seg_unit(int u) { return u ^ ((u >> 3) & 3); }
+
+// One entry per warp of the first kernel.
+template <class T>
+struct SegPartials {
+    T* head;          // the piece open at the range's start, up to its first boundary
+    T* tail;          // after the last boundary (the whole range when it has none)
+    int64_t* closes;  // the boundary that ends that first piece, -1: none, or the piece is empty
+    unsigned* bad;
+    unsigned* done;
+};
+
+// ---- what a position of the array contributes ---------------------------------
+// Plain values; mac() adds one to a running sum.
+template <class T>
+struct SegPlain {
+    static constexpr int kCtasPerSm = 3, kUnroll = 2;  // resident blocks; chunks in flight per warp
+    static constexpr int kStageBytes = 0;
+    static constexpr int kPos = kSegC + 32;  // boundaries of a chunk kept in shared memory; more are read again
+    const T* vals;
+    int64_t n;
+    bool vec;  // 32-byte aligned base
+    struct Item {
+        T x[kSegPer];
+    };
+    __device__ __forceinline__ int64_t first() const { return 0; }
+    __device__ __forceinline__ int64_t end() const { return n; }
+    __device__ __forceinline__ bool check(const Item&) const { return true; }
+    // positions base + i .. base + i + 7, those with i + j outside [lo, hi) zero
+    __device__ __forceinline__ void load(Item& it, int64_t base, int i, int lo, int hi) const {
+        const T* const vals = this->vals + base;
+        if (vec && i >= lo && i + kSegPer <= hi) {
+            const u64x4 a = ldg_stream_u64x4(vals + i), b = ldg_stream_u64x4(vals + i + 4);
+            it.x[0] = from_bits<T>(a.x); it.x[1] = from_bits<T>(a.y);
+            it.x[2] = from_bits<T>(a.z); it.x[3] = from_bits<T>(a.w);
+            it.x[4] = from_bits<T>(b.x); it.x[5] = from_bits<T>(b.y);
+            it.x[6] = from_bits<T>(b.z); it.x[7] = from_bits<T>(b.w);
+        } else {
+#pragma unroll
+            for (int j = 0; j < kSegPer; ++j) it.x[j] = i + j >= lo && i + j < hi ? vals[i + j] : T(0);
+        }
+    }
+    __device__ __forceinline__ T mac(const Item& it, int j, T acc) const { return acc + it.x[j]; }
+};
+
+// Products vals[k] * x[col[k]]; a column outside [0, ncols) contributes
+// nothing and is reported.
+template <class C>
+struct SegProduct {
+    // chunks are staged in shared memory by cp.async, two ahead: the entries'
+    // latency is off the chain entries -> x -> sums
+    static constexpr int kCtasPerSm = 3, kUnroll = 1;
+    static constexpr int kStageBytes = kSegC * (8 + (int)sizeof(C));  // values, then columns
+    // none: three blocks of two staged chunks per warp just fit the 196 KB
+    // setting of shared memory, which leaves 60 KB of L1 for x (at the 228 KB
+    // setting, 28 KB of L1, the 2^20-row case took 142 us instead of 108)
+    static constexpr int kPos = 0;
+    const C* cols;
+    const double* vals;
+    const double* x;
+    const long long* row_ptr;
+    int64_t nrows, ncols;
+    bool vec;
+    struct Item {
+        double v[kSegPer], x[kSegPer];
+        bool ok;
+    };
+    __device__ __forceinline__ int64_t first() const { return row_ptr[0]; }
+    __device__ __forceinline__ int64_t end() const { return row_ptr[nrows]; }
+    __device__ __forceinline__ bool check(const Item& it) const { return it.ok; }
+    __device__ __forceinline__ void load(Item& it, int64_t base, int i, int lo, int hi) const {
+        const C* const cols = this->cols + base;
+        const double* const vals = this->vals + base;
+        unsigned long long c[kSegPer];
+        if (vec && i >= lo && i + kSegPer <= hi) {
+            if (sizeof(C) == 8) {
+                const u64x4 a = ldg_stream_u64x4(cols + i), b = ldg_stream_u64x4(cols + i + 4);
+                c[0] = a.x; c[1] = a.y; c[2] = a.z; c[3] = a.w;
+                c[4] = b.x; c[5] = b.y; c[6] = b.z; c[7] = b.w;
+            } else {
+                const u64x4 a = ldg_stream_u64x4(cols + i);
+                const unsigned long long w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    c[2 * j] = (unsigned long long)(long long)(int)(unsigned)w[j];
+                    c[2 * j + 1] = (unsigned long long)(long long)(int)(unsigned)(w[j] >> 32);
+                }
+            }
+            const f64x4 p = ldg_stream_f64x4(vals + i), q = ldg_stream_f64x4(vals + i + 4);
+            it.v[0] = p.x; it.v[1] = p.y; it.v[2] = p.z; it.v[3] = p.w;
+            it.v[4] = q.x; it.v[5] = q.y; it.v[6] = q.z; it.v[7] = q.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < kSegPer; ++j) {
+                const bool in = i + j >= lo && i + j < hi;
+                c[j] = in ? (unsigned long long)(long long)cols[i + j] : 0ull;
+                it.v[j] = in ? vals[i + j] : 0.0;
+            }
+        }
+        it.ok = true;
+#pragma unroll
+        for (int j = 0; j < kSegPer; ++j) {
+            const bool in = i + j >= lo && i + j < hi;
+            const bool ok = c[j] < (unsigned long long)ncols;
+            it.x[j] = in && ok ? __ldg(x + c[j]) : 0.0;
+            if (!ok) it.v[j] = 0.0;
+            it.ok &= ok || !in;
+        }
+    }
+    __device__ __forceinline__ void stage(unsigned char* buf, int64_t base, int p, int lo, int hi) const {
+        const int lane = threadIdx.x & 31;
+        if (vec) {
+            // a unit that begins before `lo` is fetched whole (lo is inside the array)
+            const double* const gv = vals + base + p;
+            const C* const gc = cols + base + p;
+            constexpr int kPerV = 2, kPerC = 16 / (int)sizeof(C);
+#pragma unroll
+            for (int k = 0; k < kSegC / kPerV / 32; ++k) {
+                const int u = lane + 32 * k, left = hi - (p + kPerV * u);
+                if (left > 0 && p + kPerV * (u + 1) > lo)
+                    cp_async_16(buf + 16 * seg_unit(u), gv + kPerV * u, left >= kPerV ? 16 : left * 8);
+            }
+#pragma unroll
+            for (int k = 0; k < kSegC / kPerC / 32; ++k) {
+                const int u = lane + 32 * k, left = hi - (p + kPerC * u);
+                if (left > 0 && p + kPerC * (u + 1) > lo)
+                    cp_async_16(buf + kSegC * 8 + 16 * seg_unit(u), gc + kPerC * u,
+                                left >= kPerC ? 16 : left * (int)sizeof(C));
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    __device__ __forceinline__ void load_staged(Item& it, const unsigned char* buf, int64_t base, int i, int lo,
+                                                int hi) const {
+        if (!vec) {
+            load(it, base, i, lo, hi);
+            return;
+        }
+        const int lane = threadIdx.x & 31;
+        unsigned long long c[kSegPer];
+        constexpr int kPerC = 16 / (int)sizeof(C);
+#pragma unroll
+        for (int q = 0; q < kSegPer / kPerC; ++q) {
+            const C* const s = reinterpret_cast<const C*>(buf + kSegC * 8 + 16 * seg_unit(kSegPer / kPerC * lane + q));
+            C w[kPerC];
+            *reinterpret_cast<uint4*>(w) = *reinterpret_cast<const uint4*>(s);
+#pragma unroll
+            for (int k = 0; k < kPerC; ++k) c[kPerC * q + k] = (unsigned long long)(long long)w[k];
+        }
+        it.ok = true;
+#pragma unroll
+        for (int j = 0; j < kSegPer; ++j) {
+            const bool in = i + j >= lo && i + j < hi;
+            const bool ok = c[j] < (unsigned long long)ncols;
+            it.x[j] = in && ok ? __ldg(x + c[j]) : 0.0;
+            it.ok &= ok || !in;
+            c[j] = in && ok;
+        }
+#pragma unroll
+        for (int q = 0; q < kSegPer / 2; ++q) {
+            const double2 v = *reinterpret_cast<const double2*>(buf + 16 * seg_unit(kSegPer / 2 * lane + q));
+            it.v[2 * q] = c[2 * q] ? v.x : 0.0;
+            it.v[2 * q + 1] = c[2 * q + 1] ? v.y : 0.0;
+        }
+    }
+    __device__ __forceinline__ double mac(const Item& it, int j, double acc) const {
+        return fma(it.v[j], it.x[j], acc);
+    }
+};
+
+// The split of [first, end) over the warps: ranges of `range` values from
+// `base` (a multiple of the chunk), the last ones possibly empty.  Positions
+// inside a range are kept in 32 bits.
+struct SegSplit {
+    int64_t base, range, lo_valid, hi_valid;
+    bool ok;
+    __device__ __forceinline__ SegSplit(int64_t first, int64_t end, int64_t nwarps) {
+        ok = first >= 0 && end >= first;
+        lo_valid = ok ? first : 0;
+        hi_valid = ok ? end : 0;
+        base = lo_valid / kSegC * kSegC;
+        const int64_t chunks = (hi_valid - base + kSegC - 1) / kSegC;
+        const int64_t per = (chunks + nwarps - 1) / nwarps;
+        range = (per > 0 ? per : 1) * kSegC;
+        if (range > (1 << 30)) ok = false;
+    }
+};
+
+// First indices i in [0, m) with a[i] >= key, for two keys at once (m when
+// there is none).  Warp-wide: 32 probes per key and round narrow the range
+// 33-fold.  Monotone in `key` even for unsorted `a`, so the ranges of
+// different warps never overlap and together cover every boundary.
+__device__ __forceinline__ void warp_lower_bound2(const int64_t* __restrict__ a, int64_t m, int64_t key0,
+                                                  int64_t key1, int64_t& out0, int64_t& out1) {
+    const int lane = threadIdx.x & 31;
+    int64_t lo[2] = {0, 0}, hi[2] = {m, m};
+    const int64_t key[2] = {key0, key1};
+    while (hi[0] - lo[0] > 32 || hi[1] - lo[1] > 32) {
+        int64_t v[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int64_t p = lo[q] + (hi[q] - lo[q]) * (lane + 1) / 33;
+            v[q] = p < hi[q] ? a[p] : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int64_t span = hi[q] - lo[q];
+            if (span > 32) {  // warp-uniform
+                const int k = __popc(__ballot_sync(0xffffffffu, v[q] < key[q]));
+                const int64_t nlo = k ? lo[q] + span * k / 33 + 1 : lo[q];
+                const int64_t nhi = k < 32 ? lo[q] + span * (k + 1) / 33 : hi[q];
+                lo[q] = nlo;
+                hi[q] = nhi;
+            }
+        }
+    }
+    int64_t v[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) v[q] = lo[q] + lane < hi[q] ? a[lo[q] + lane] : key[q];
+    out0 = lo[0] + __popc(__ballot_sync(0xffffffffu, v[0] < key0));
+    out1 = lo[1] + __popc(__ballot_sync(0xffffffffu, v[1] < key1));
+}
+
+// Boundary b is offsets[b], 0 <= b <= nseg; it ends segment b - 1.  A warp
+// with the range (lo, hi] takes the boundaries in it, the first warp those at
+// the array's very start too.  Positions and boundary numbers below are
+// relative to the warp's lo and first boundary b0.
+template <class T, class Src>
+__global__ void __launch_bounds__(kSegT, Src::kCtasPerSm)
+    segsum_kernel(const Src src, const int64_t* __restrict__ offsets, const int64_t nseg, const T init,
+                  T* __restrict__ out, const SegPartials<T> part, unsigned* err) {
+    // per warp: the chunk's sums, or two staged chunks (a chunk's sums then take the place of its values)
+    extern __shared__ __align__(16) unsigned char seg_smem[];
+    constexpr bool kStaged = Src::kStageBytes > 0;
+    __shared__ unsigned sh_bits[kSegWarps][kSegC / 32];
+    __shared__ int sh_pos[kSegWarps][Src::kPos > 0 ? Src::kPos : 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned char* const mine = seg_smem + warp * (kStaged ? 2 * Src::kStageBytes : kSegC * (int)sizeof(T));
+    unsigned* const bits = sh_bits[warp];
+    int* const pos = sh_pos[warp];
+    const int w = blockIdx.x * kSegWarps + warp;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const SegSplit sp(src.first(), src.end(), (int64_t)gridDim.x * kSegWarps);
+    const int64_t lo = sp.base + w * sp.range;
+    if (w > 0 && lo >= sp.hi_valid) {  // no values left for this warp
+        if (lane == 0) {
+            part.tail[w] = T(0);
+            part.closes[w] = -1;
+        }
+        return;
+    }
+    const bool is_last = lo + sp.range >= sp.hi_valid;
+    int64_t b0, b1;
+    warp_lower_bound2(offsets, nseg + 1, lo + 1, lo + sp.range + 1, b0, b1);
+    if (w == 0) b0 = 0;
+    if (is_last) b1 = nseg + 1;
+    bool bad = !sp.ok || b1 < b0 || b1 - b0 > INT_MAX - 64;
+    bool bad_item = false;
+    const int nb = bad ? 0 : (int)(b1 - b0);
+    const int64_t* const off = offsets + b0;  // [nb]
+    T* const outb = out + b0 - 1;             // segment b0 - 1 + r ends at boundary r
+    // a boundary's position: clamped below to "before the range"
+    auto rel = [&](int64_t x) {
+        const int64_t r = x - lo;
+        return r < 0 ? -1 : (r > INT_MAX ? INT_MAX : (int)r);
+    };
+    const int vlo = (int)(sp.lo_valid > lo ? sp.lo_valid - lo : 0);                      // valid positions:
+    const int vhi = (int)(sp.hi_valid - lo < sp.range ? sp.hi_valid - lo : sp.range);  // [vlo, vhi)
+    const int stop_p = vhi;  // chunks start below this (the first one always runs)
+    int bc = 0;                                      // first boundary not yet passed
+    int prev = b0 > 0 ? rel(offsets[b0 - 1]) : -2;   // the one before it
+    bool closes = false;   // this lane ended the piece that was open at lo
+    T carry = T(0);        // sum of the open piece, up to the last boundary chunk's end
+    T acc[kSegPer];        // ... and since then, per lane
+    bool have_acc = false;
+#pragma unroll
+    for (int j = 0; j < kSegPer; ++j) acc[j] = T(0);
+    // a window of the next 32 boundaries
+    int win = lane < nb ? rel(off[lane]) : INT_MAX;
+
+    int p = 0;
+    if constexpr (kStaged) {
+        src.stage(mine, lo, 0, vlo, vhi);
+        src.stage(mine + Src::kStageBytes, lo, kSegC, vlo, vhi);
+    }
+    while (!bad) {
+        typename Src::Item it;
+        unsigned char* buf = mine;
+        if constexpr (kStaged) {
+            buf += (p / kSegC & 1) * Src::kStageBytes;
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+            src.load_staged(it, buf, lo, p + kSegPer * lane, vlo, vhi);
+            __syncwarp();
+        } else {
+            src.load(it, lo, p + kSegPer * lane, vlo, vhi);
+        }
+        T* const sums = reinterpret_cast<T*>(buf);
+        const int next = __shfl_sync(0xffffffffu, win, 0);
+        bad_item |= !src.check(it);
+        if (next > p + kSegC) {
+#pragma unroll
+            for (int j = 0; j < kSegPer; ++j) acc[j] = src.mac(it, j, acc[j]);
+            have_acc = true;
+            if constexpr (kStaged) src.stage(buf, lo, p + 2 * kSegC, vlo, vhi);
+            p += kSegC;
+            // whole chunks before the next boundary, kUnroll at a time
+            const int stop = next - 1 < stop_p ? next - 1 : stop_p;
+            for (; !kStaged && p + Src::kUnroll * kSegC <= stop; p += Src::kUnroll * kSegC) {
+                typename Src::Item iu[Src::kUnroll];
+#pragma unroll
+                for (int u = 0; u < Src::kUnroll; ++u)
+                    src.load(iu[u], lo, p + u * kSegC + kSegPer * lane, vlo, vhi);
+#pragma unroll
+                for (int u = 0; u < Src::kUnroll; ++u) {
+                    bad_item |= !src.check(iu[u]);
+#pragma unroll
+                    for (int j = 0; j < kSegPer; ++j) acc[j] = src.mac(iu[u], j, acc[j]);
+                }
+            }
+            if (p >= stop_p) break;
+            continue;
+        }
+        // a chunk with boundaries: mark the heads
+        if (lane < kSegC / 32) bits[lane] = 0u;
+        __syncwarp();
+        bool at_end = false;
+        int total = 0, pw = prev;  // boundaries of this chunk so far; the last one
+        const int wn = bc + 32 + lane < nb ? rel(off[bc + 32 + lane]) : INT_MAX;
+        // one window of 32: false when it is the chunk's last
+        auto mark = [&](int xw) {
+            const bool in = bc + total + lane < nb && xw <= p + kSegC;
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            const int up = __shfl_up_sync(0xffffffffu, xw, 1);
+            const int before = lane ? up : pw;
+            const int cnt = __popc(m);
+            if (in) {
+                // ascending, inside the values, and not one that an earlier chunk should have met
+                bad |= xw < before || xw > vhi || xw < vlo || !(xw > p || (w == 0 && xw == 0));
+                if (xw > p && xw < p + kSegC) atomicOr(&bits[(xw - p) >> 5], 1u << ((xw - p) & 31));
+                at_end |= xw == p + kSegC;
+                if (total + lane < Src::kPos) pos[total + lane] = xw;
+            }
+            bad |= cnt < 32 && (m >> cnt) != 0u;  // not a prefix of the window
+            if (cnt) pw = __shfl_sync(0xffffffffu, xw, cnt - 1);
+            total += cnt;
+            return cnt == 32;
+        };
+        if (mark(win) && mark(wn)) {
+            // many short segments: four windows' loads at once
+            bool more = true;
+            while (more) {
+                int x4[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int b = bc + total + 32 * u + lane;
+                    x4[u] = b < nb ? rel(off[b]) : INT_MAX;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (more) more = mark(x4[u]);
+            }
+        }
+        bad = __any_sync(0xffffffffu, bad);
+        if (bad) break;
+        at_end = __any_sync(0xffffffffu, at_end);
+        if (have_acc) {
+            T a = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            carry += a;
+#pragma unroll
+            for (int j = 0; j < kSegPer; ++j) acc[j] = T(0);
+            have_acc = false;
+        }
+        __syncwarp();
+        // segmented scan; only segment ends (and the chunk's last value) are
+        // read back, so the carry from the lanes before is added once, at the
+        // last position before the lane's first head
+        const unsigned hb = (bits[lane >> 2] >> ((lane & 3) * 8)) & 0xffu;
+        T r[kSegPer];
+        r[0] = src.mac(it, 0, T(0));
+#pragma unroll
+        for (int j = 1; j < kSegPer; ++j) r[j] = src.mac(it, j, (hb >> j) & 1u ? T(0) : r[j - 1]);
+        bool h = hb != 0u;
+        T v = r[kSegPer - 1];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const bool hu = __shfl_up_sync(0xffffffffu, h, d);
+            const T vu = __shfl_up_sync(0xffffffffu, v, d);
+            if (lane >= d) {
+                if (!h) v = vu + v;
+                h = h || hu;
+            }
+        }
+        const bool hl = __shfl_up_sync(0xffffffffu, h, 1);
+        const T vl = __shfl_up_sync(0xffffffffu, v, 1);
+        const T ve = lane == 0 ? carry : (hl ? vl : carry + vl);
+        const int fix = (hb ? __ffs(hb) - 1 : kSegPer) - 1;  // -1: nothing before the first head
+        T sel = T(0);
+#pragma unroll
+        for (int j = 0; j < kSegPer; ++j)
+            if (j == fix) sel = r[j];
+        const T fixed = ve + sel;
+#pragma unroll
+        for (int j = 0; j < kSegPer; ++j) sums[seg_slot(kSegPer * lane + j)] = j == fix ? fixed : r[j];
+        const T tail = fix == kSegPer - 1 ? fixed : r[kSegPer - 1];
+        carry = at_end ? T(0) : __shfl_sync(0xffffffffu, tail, 31);
+        __syncwarp();
+        // the sums that end here
+        // boundary 0 ends no segment; the piece that was open at lo goes to the partials
+        auto finish = [&](int k, int x, int before) {
+            const T s = x > p ? sums[seg_slot(x - 1 - p)] : T(0);
+            const bool open = before < 0 && before != x;
+            if (open && (b0 > 0 || bc + k > 0)) {
+                part.head[w] = s;
+                part.closes[w] = b0;
+                closes = true;
+            }
+            if (!open) outb[bc + k] = before == x ? init : init + s;
+        };
+        if (Src::kPos == 0 && total <= 32) {
+            const int up = __shfl_up_sync(0xffffffffu, win, 1);
+            if (lane < total) finish(lane, win, lane ? up : prev);
+        } else {
+#pragma unroll 2
+            for (int k = lane; k < total; k += 32) {
+                const int x = k < Src::kPos ? pos[k] : rel(off[bc + k]);
+                const int before = k == 0 ? prev : (k <= Src::kPos ? pos[k - 1] : rel(off[bc + k - 1]));
+                finish(k, x, before);
+            }
+        }
+        prev = pw;
+        bc += total;
+        if (total <= 32) {  // the window moves on by `total`: from the lanes above, then from the next 32
+            const int from = lane + total;
+            const int from_win = __shfl_sync(0xffffffffu, win, from & 31);
+            const int from_next = __shfl_sync(0xffffffffu, wn, from & 31);
+            win = from < 32 ? from_win : from_next;
+        } else {
+            win = bc + lane < nb ? rel(off[bc + lane]) : INT_MAX;
+        }
+        __syncwarp();
+        if constexpr (kStaged) src.stage(buf, lo, p + 2 * kSegC, vlo, vhi);
+        p += kSegC;
+        if (p >= stop_p) break;
+    }
+    if constexpr (kStaged) asm volatile("cp.async.wait_all;" ::: "memory");
+    bad |= bc != nb;
+    T a = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    const bool any = __any_sync(0xffffffffu, closes);
+    if (lane == 0) {
+        if (!any) part.closes[w] = -1;
+        part.tail[w] = carry + a;
+        if (bad) atomicOr(part.bad, 1u);
+    }
+    if (bad_item) raise_error(err, ERRBIT_BOUNDS);
+}
+
+// One segment on its own, by a whole warp; false when it is invalid.
+template <class T>
+__device__ __forceinline__ bool seg_one(const SegPlain<T>& src, int64_t start, int64_t stop, T init, T* o) {
+    const int lane = threadIdx.x & 31;
+    const bool ok = start >= 0 && stop <= src.n && stop >= start;
+    T acc = T(0);
+    if (ok)
+        for (int64_t k = start + lane; k < stop; k += 32) acc += src.vals[k];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+    if (lane == 0) *o = init + acc;
+    return ok;
+}
+template <class C>
+__device__ __forceinline__ bool seg_one(const SegProduct<C>& src, int64_t start, int64_t stop, double init,
+                                        double* o) {
+    const int lane = threadIdx.x & 31;
+    bool ok = true;
+    double acc = 0.0;
+    for (int64_t k = start + lane; k < stop; k += 32) {
+        const unsigned long long c = (unsigned long long)(long long)src.cols[k];
+        if (c < (unsigned long long)src.ncols) acc = fma(src.vals[k], src.x[c], acc);
+        else ok = false;
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+    if (lane == 0) *o = init + acc;
+    return ok;
+}
+
+// Adds up the pieces that cross warps of the first kernel: warp w of this
+// one ends the piece that warp w of that one closed.  With invalid offsets it
+// computes every segment instead.
+template <class T, class Src>
+__global__ void __launch_bounds__(kSegT) segsum_finish_kernel(const Src src, const int64_t* __restrict__ offsets,
+                                                              const int64_t nseg, const T init,
+                                                              T* __restrict__ out, const SegPartials<T> part,
+                                                              const int64_t nwarps, unsigned* err) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t w = (int64_t)blockIdx.x * kSegWarps + warp;
+    // launched while the first kernel runs: wait for its results
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const bool invalid = *(volatile const unsigned*)part.bad != 0u;
+    if (invalid) {
+        bool bad = false;
+        for (int64_t s = w; s < nseg; s += (int64_t)gridDim.x * kSegWarps)
+            bad |= !seg_one(src, offsets[s], offsets[s + 1], init, out + s);
+        if (bad) raise_error(err, ERRBIT_BOUNDS);
+    } else if (w < nwarps) {
+        const int64_t b = part.closes[w];
+        if (b >= 0) {
+            const SegSplit sp(src.first(), src.end(), nwarps);
+            const int64_t start = offsets[b - 1];
+            // the warp whose range (lo, hi] holds the piece's start
+            const int64_t u0 = start > sp.base ? (start - 1 - sp.base) / sp.range : 0;
+            T s = T(0);
+            for (int64_t u = u0 + lane; u < w; u += 32) s += part.tail[u];
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+            if (lane == 0) out[b - 1] = init + (s + part.head[w]);
+        }
+    }
+    // the last block leaves the two words at zero for the next call
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(part.done, 1u) == gridDim.x - 1) {
+            *part.bad = 0u;
+            *part.done = 0u;
+        }
+    }
+}
+
+// `values`: the number of values, or an estimate of it when only the device knows.
+template <class T, class Src>
+static int segsum_launch(const Src& src, const int64_t* offsets, int64_t nseg, int64_t values, T init, T* out,
+                         cudaStream_t s, const char* what) {
+    Device* d = nullptr;
+    HYD_TRY(device(&d));
+    int64_t blocks = (values + (int64_t)kSegC * kSegWarps - 1) / ((int64_t)kSegC * kSegWarps);
+    const int64_t cap = (int64_t)d->sm_count * Src::kCtasPerSm;
+    blocks = blocks < 1 ? 1 : (blocks > cap ? cap : blocks);
+    const int64_t nwarps = blocks * kSegWarps;
+    unsigned* counters = nullptr;
+    void* scratch = nullptr;
+    HYD_TRY(workspace(s, (size_t)nwarps * 24, &counters, &scratch));
+    SegPartials<T> part;
+    part.head = static_cast<T*>(scratch);
+    part.tail = part.head + nwarps;
+    part.closes = reinterpret_cast<int64_t*>(part.tail + nwarps);
+    part.bad = counters + kSegCounterWord;
+    part.done = counters + kSegCounterWord + 1;
+    auto k = segsum_kernel<T, Src>;
+    constexpr size_t kSmem = kSegWarps * (size_t)(Src::kStageBytes ? 2 * Src::kStageBytes : kSegC * (int)sizeof(T));
+    HYD_TRY(configure_kernel((const void*)k, d, false));
+    k<<<(unsigned)blocks, kSegT, kSmem, s>>>(src, offsets, nseg, init, out, part, d->d_err);
+    HYD_TRY(launch_check(what));
+    // programmatic dependent launch: the second kernel's blocks are in place
+    // when the first one ends
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(kSegT);
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    HYD_CUDA_TRY(cudaLaunchKernelEx(&cfg, segsum_finish_kernel<T, Src>, src, offsets, nseg, init, out, part, nwarps,
+                                    d->d_err));
+    return launch_check(what);
+}
+
+// The SpMV with the default row split (sparse.cu checks the arguments).
+template <class C>
+int spmv_segsum(int64_t nrows, int64_t ncols, const long long* row_ptr, const C* cols, const double* vals,
+                const double* x, double* y, cudaStream_t s) {
+    const bool vec = ((reinterpret_cast<uintptr_t>(cols) | reinterpret_cast<uintptr_t>(vals)) & 31) == 0;
+    const SegProduct<C> src{cols, vals, x, row_ptr, nrows, ncols, vec};
+    return segsum_launch<double>(src, reinterpret_cast<const int64_t*>(row_ptr), nrows, INT64_MAX / 2, 0.0, y, s,
+                                 "spmv_csr");
+}
+template int spmv_segsum<long long>(int64_t, int64_t, const long long*, const long long*, const double*,
+                                    const double*, double*, cudaStream_t);
+template int spmv_segsum<int>(int64_t, int64_t, const long long*, const int*, const double*, const double*, double*,
+                              cudaStream_t);
+
+template <class T>
+static int segreduce_launch(const int64_t* offsets, int64_t n_offsets, const T* vals, int64_t n_vals, T init,
+                            T* out, void* stream, const char* what) {
+    HYD_CHECK_ARG(n_offsets >= 1, "%s: need at least one offset", what);
+    HYD_CHECK_ARG(offsets != nullptr, "%s: null offsets", what);
+    HYD_CHECK_ARG(n_vals >= 0 && (n_vals == 0 || vals != nullptr), "%s: bad values", what);
+    const int64_t nseg = n_offsets - 1;
+    HYD_CHECK_ARG(nseg == 0 || out != nullptr, "%s: null output", what);
+    if (nseg == 0) return HYD_CUDA_OK;
+    HYD_CHECK_ARG(n_vals <= (int64_t)4096 * 0x7fffffffLL, "%s: too many values", what);
+    const SegPlain<T> src{vals, n_vals, (reinterpret_cast<uintptr_t>(vals) & 31) == 0};
+    return segsum_launch<T>(src, offsets, nseg, n_vals, init, out, as_stream(stream), what);
+}
+
+}  // namespace hyd
+
+using namespace hyd;
+
+extern "C" int hyd_cuda_segmented_reduce_i64(const int64_t* offsets, int64_t n_offsets, const int64_t* vals,
+                                             int64_t n_vals, int64_t init, int64_t* out, void* stream) {
+    return segreduce_launch<long long>(offsets, n_offsets, reinterpret_cast<const long long*>(vals), n_vals,
+                                       (long long)init, reinterpret_cast<long long*>(out), stream,
+                                       "segmented_reduce_i64");
+}
+
+extern "C" int hyd_cuda_segmented_reduce_f64(const int64_t* offsets, int64_t n_offsets, const double* vals,
+                                             int64_t n_vals, double init, double* out, void* stream) {
+    return segreduce_launch<double>(offsets, n_offsets, vals, n_vals, init, out, stream, "segmented_reduce_f64");
+}

@@ -1,0 +1,101 @@
+"""GPU parity of the evenly split segment sums (segmented_reduce and the SpMV
+with the default row split) where the split can go wrong: boundaries at the
+edges of the 256-value chunks and of the warps' ranges, pieces that cross many
+warps, unaligned bases, row pointers that do not start at 0 or do not ascend."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _seg(hc, orc, dev, offsets, nv, shift):
+    rng = np.random.default_rng(nv + shift)
+    vi = rng.integers(-(1 << 62), 1 << 62, size=nv).astype(np.int64)
+    vf = rng.uniform(-1, 1, size=nv)
+    off = torch.from_numpy(offsets).to(dev)
+    oi = torch.empty(len(offsets) - 1, dtype=torch.int64, device=dev)
+    of = torch.empty(len(offsets) - 1, dtype=torch.float64, device=dev)
+    ti = torch.empty(nv + shift, dtype=torch.int64, device=dev)[shift:]
+    tf = torch.empty(nv + shift, dtype=torch.float64, device=dev)[shift:]
+    ti.copy_(torch.from_numpy(vi))
+    tf.copy_(torch.from_numpy(vf))
+    hc.segmented_reduce(off, ti, oi, init=-5)
+    hc.segmented_reduce(off, tf, of, init=0.5)
+    hc.check(hc.device_check())
+    assert np.array_equal(oi.cpu().numpy(), orc.segmented_reduce_i64(offsets, vi, -5))
+    absum = orc.segmented_reduce_f64(offsets, np.abs(vf), 0.0)
+    ref = orc.segmented_reduce_f64(offsets, vf, 0.5)
+    assert np.all(np.abs(of.cpu().numpy() - ref) <= 1e-12 * np.maximum(absum, 1.0))
+
+
+@pytest.mark.parametrize("shift", [0, 1, 2])  # 32-byte aligned values, and not
+@pytest.mark.parametrize("step", [255, 256, 257, 2047, 2048, 1])
+def test_segment_ends_at_chunk_and_range_edges(hc, orc, dev, step, shift):
+    ends = np.arange(step, 200_001, step, dtype=np.int64)
+    offsets = np.concatenate([[0, 0], np.repeat(ends, 1 + (np.arange(len(ends)) % 3 == 0))])
+    _seg(hc, orc, dev, offsets, int(offsets[-1]) + 3, shift)
+
+
+@pytest.mark.parametrize("n", [1, 256, 257, (1 << 21) + 5])
+def test_one_segment_over_many_warps_between_short_ones(hc, orc, dev, n):
+    lens = np.concatenate([[1, 0, 2], [n], [0, 3, 300]])
+    _seg(hc, orc, dev, np.concatenate([[7], 7 + np.cumsum(lens)]).astype(np.int64), 7 + int(lens.sum()), 0)
+
+
+def _csr(rng, nrows, ncols, kind):
+    lens = np.minimum(rng.zipf(1.5, size=nrows), 256)
+    if kind == "empty":
+        lens[rng.random(nrows) < 0.9] = 0
+    if kind == "long":
+        lens[[3, nrows // 2, nrows - 1]] = [1000, 300_000, 257]
+    row_ptr = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    nnz = int(row_ptr[-1])
+    return row_ptr, rng.integers(0, ncols, size=nnz), rng.uniform(-1, 1, size=nnz), rng.uniform(-1, 1, size=ncols)
+
+
+def _spmv(hc, dev, row_ptr, cols, vals, x, dtype, lanes=0, shift=0):
+    def up(a, dt):
+        t = torch.empty(len(a) + shift, dtype=dt, device=dev)[shift:]
+        t.copy_(torch.from_numpy(a))
+        return t
+    y = torch.full((len(row_ptr) - 1,), -7.0, dtype=torch.float64, device=dev)
+    hc.spmv_csr(torch.from_numpy(row_ptr).to(dev), up(cols, dtype), up(vals, torch.float64),
+                torch.from_numpy(x).to(dev), y, lanes_per_row=lanes)
+    return y
+
+
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32])
+@pytest.mark.parametrize("kind,shift", [("zipf", 0), ("zipf", 1), ("empty", 0), ("long", 0)])
+def test_spmv_even_split(hc, orc, dev, kind, shift, dtype):
+    nrows, ncols = (1 << 18) + 37, 70_001
+    row_ptr, cols, vals, x = _csr(np.random.default_rng(5), nrows, ncols, kind)
+    y = _spmv(hc, dev, row_ptr, cols, vals, x, dtype, shift=shift)
+    hc.check(hc.device_check())
+    assert torch.equal(y, _spmv(hc, dev, row_ptr, cols, vals, x, dtype, shift=shift))
+    ref = orc.spmv_csr(row_ptr, cols, vals, x)
+    bound = orc.spmv_csr(row_ptr, cols, np.abs(vals), np.abs(x))
+    assert np.all(np.abs(y.cpu().numpy() - ref) <= 1e-12 * np.maximum(bound, 1e-300))
+
+
+@pytest.mark.parametrize("case", ["starts_later", "descending_inside", "bad_column"])
+def test_spmv_even_split_matches_the_lane_split(hc, dev, case):
+    """Row pointers that do not start at 0 or do not ascend, and columns out of
+    range, give what the lanes-per-row form gives (rows take what their two
+    pointers span; a bad column is left out and reported)."""
+    nrows, ncols = 1 << 18, 5000
+    row_ptr, cols, vals, x = _csr(np.random.default_rng(6), nrows, ncols, "zipf")
+    if case == "starts_later":
+        row_ptr = row_ptr[1001:]
+    elif case == "descending_inside":
+        row_ptr[[500, 1000]] = row_ptr[[1000, 500]]
+    else:
+        cols[12345] = ncols
+        cols[777] = -1
+    if case == "starts_later":  # still enough rows for the even split
+        row_ptr = np.concatenate([row_ptr, np.full(2000, row_ptr[-1])])
+    y = _spmv(hc, dev, row_ptr, cols, vals, x, torch.int64)
+    st = hc.device_check()
+    want = _spmv(hc, dev, row_ptr, cols, vals, x, torch.int64, lanes=8)
+    assert hc.device_check() == st == (hc.ERR_BOUNDS if case == "bad_column" else hc.OK)
+    assert np.allclose(y.cpu().numpy(), want.cpu().numpy(), rtol=0, atol=1e-12 * 60_000)
