@@ -74,8 +74,9 @@ struct Device {
 // Returns the current device's context, creating it on first use.
 int device(Device** out);
 // Scratch of at least `bytes` beyond the counter area for `stream`.  Growth
-// synchronizes the stream before freeing the old block.
-int workspace(cudaStream_t stream, size_t bytes, unsigned** counters, void** scratch);
+// synchronizes the stream before freeing the old block; *grew tells of it
+// (what the old block held is gone).
+int workspace(cudaStream_t stream, size_t bytes, unsigned** counters, void** scratch, bool* grew = nullptr);
 
 // Runtime-owned device buffer named `key` of at least `bytes` (grows; the
 // caller must not have work in flight on an old block when it grows).

@@ -64,7 +64,8 @@ int device(Device** out) {
     return HYD_CUDA_OK;
 }
 
-int workspace(cudaStream_t stream, size_t bytes, unsigned** counters, void** scratch) {
+int workspace(cudaStream_t stream, size_t bytes, unsigned** counters, void** scratch, bool* grew) {
+    if (grew) *grew = false;
     Device* d = nullptr;
     HYD_TRY(device(&d));
     std::lock_guard<std::mutex> lock(d->mu);
@@ -83,6 +84,7 @@ int workspace(cudaStream_t stream, size_t bytes, unsigned** counters, void** scr
         HYD_CUDA_TRY(cudaMemsetAsync(p, 0, kCounterBytes, stream));
         w.base = static_cast<unsigned char*>(p);
         w.bytes = cap;
+        if (grew) *grew = true;
     }
     if (counters) *counters = reinterpret_cast<unsigned*>(w.base);
     if (scratch) *scratch = w.base + kCounterBytes;
