@@ -9,12 +9,11 @@
 // rows in `omp parallel for`, sequential sum per row).
 //
 // GPU forms:
-//  * coo_sum_duplicates: head flags -> inclusive scan (segment ids) -> heads
-//    write (row, col), every entry adds its value into its segment (int64,
-//    order-independent, bit-exact); entries past the canonical count are
-//    zeroed like the reference's calloc'd outputs.
-//  * csr_from_sorted_coo: row counts by global atomics, exclusive scan
-//    (decoupled look-back), parallel copy of cols/vals.
+//  * coo_sum_duplicates: one pass over tiles with a look-back that carries the
+//    number of runs and the open run's sum (int64, bit-exact); entries past the
+//    canonical count are zeroed like the reference's calloc'd outputs.
+//  * csr_from_sorted_coo: row counts (one atomic per run of equal rows in a
+//    warp) and the copies of cols/vals in one pass, then an exclusive scan.
 //  * SpMV: a group of G lanes per row, lane-strided fma partial sums and a
 //    fixed xor tree, so results are deterministic; within 1e-12 of
 //    sum |v*x| of the C backend's sequential sum.  Large matrices with the
@@ -41,51 +40,269 @@ namespace hyd {
 
 int scan_i64_launch(const long long* in, long long* out, int64_t n, long long init, bool reverse,
                     bool inclusive, cudaStream_t stream);
+size_t scan_i64_scratch_bytes(int64_t n);
+int scan_i64_launch_with(const long long* in, long long* out, int64_t n, long long init, bool reverse,
+                         bool inclusive, void* status_scratch, unsigned* tile_counter, cudaStream_t stream);
 
 // ---------------------------------------------------------------- coo dedup
-__global__ void coo_head_flags_kernel(const long long* __restrict__ rows, const long long* __restrict__ cols,
-                                      int64_t nnz, long long* __restrict__ flags) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * blockDim.x)
-        flags[i] = (i == 0 || rows[i] != rows[i - 1] || cols[i] != cols[i - 1]) ? 1 : 0;
+// One pass over the entries: a tile of 2048 finds its heads (entries that
+// differ from the one before), sums each run of equal entries and looks back
+// over the earlier tiles' words for the number of heads before it and the sum
+// of the run that was open at its start.  A run is written once, by the tile
+// it ends in, through shared memory so that the stores are whole sectors.
+// HBM bounds it: 24 bytes read per entry and 24 written, 119 us at 2^24
+// entries.  Measured there (runs of 4): 160 us, and 47 us for the zeros; head
+// flags, a scan of them, three fills and a merge with atomics took 300 us.
+constexpr int kCooT = 256;
+constexpr int kCooPer = 8;
+constexpr int kCooTile = kCooT * kCooPer;
+
+// 8 consecutive entries, those past the end zero.
+__device__ __forceinline__ void coo_load8(const long long* __restrict__ a, int64_t i, int64_t n, bool vec,
+                                          long long (&v)[kCooPer]) {
+    if (vec && i + kCooPer <= n) {
+        const u64x4 x = ldg_stream_u64x4(a + i), y = ldg_stream_u64x4(a + i + 4);
+        v[0] = (long long)x.x; v[1] = (long long)x.y; v[2] = (long long)x.z; v[3] = (long long)x.w;
+        v[4] = (long long)y.x; v[5] = (long long)y.y; v[6] = (long long)y.z; v[7] = (long long)y.w;
+    } else {
+#pragma unroll
+        for (int j = 0; j < kCooPer; ++j) v[j] = i + j < n ? a[i + j] : 0;
+    }
 }
 
-__global__ void coo_merge_kernel(const long long* __restrict__ rows, const long long* __restrict__ cols,
-                                 const long long* __restrict__ vals, int64_t nnz,
-                                 const long long* __restrict__ seg_incl, long long* __restrict__ out_rows,
-                                 long long* __restrict__ out_cols, unsigned long long* __restrict__ out_vals) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * blockDim.x) {
-        const long long s = seg_incl[i] - 1;
-        const bool head = (i == 0) || seg_incl[i] != seg_incl[i - 1];
-        if (head) {
-            out_rows[s] = rows[i];
-            out_cols[s] = cols[i];
+// Tile word: {state | heads << 2, sum since the last head}; state 1 the tile's
+// own, 2 of all entries up to the tile's end (TileWord, one 16-byte access).
+__global__ void __launch_bounds__(kCooT, 3)
+    coo_sum_kernel(const long long* __restrict__ rows, const long long* __restrict__ cols,
+                   const long long* __restrict__ vals, int64_t nnz, bool vec, long long* __restrict__ out_rows,
+                   long long* __restrict__ out_cols, long long* __restrict__ out_vals, long long* __restrict__ out_nnz,
+                   TileWord* words, unsigned* ticket, unsigned* err) {
+    __shared__ long long sh_out[kCooTile];
+    __shared__ long long sh_sum[kCooT / 32];   // per warp: the sum since its last head
+    __shared__ int sh_heads[kCooT / 32];
+    __shared__ long long sh_carry, sh_before;  // of the tile: the open run's sum, the heads before
+    __shared__ unsigned sh_tile;
+    __shared__ int sh_head0, sh_end;
+    typedef unsigned long long U;  // sums wrap
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) sh_tile = atomicAdd(ticket, 1u);
+    __syncthreads();
+    const int64_t tile = sh_tile;
+    const int64_t base = tile * kCooTile, i0 = base + kCooPer * threadIdx.x;
+    long long r[kCooPer], c[kCooPer], v[kCooPer];
+    coo_load8(rows, i0, nnz, vec, r);
+    coo_load8(cols, i0, nnz, vec, c);
+    coo_load8(vals, i0, nnz, vec, v);
+    // heads of entries i0 .. i0 + 8 (bit 8: the next thread's first entry, so
+    // bit j + 1 says that entry j ends its run; past the end counts as a head)
+    long long pr = __shfl_up_sync(0xffffffffu, r[kCooPer - 1], 1), pc = __shfl_up_sync(0xffffffffu, c[kCooPer - 1], 1);
+    if (lane == 0 && i0 > 0 && i0 < nnz) {
+        pr = rows[i0 - 1];
+        pc = cols[i0 - 1];
+    }
+    unsigned hb = 0;
+    if (i0 < nnz && (i0 == 0 || r[0] != pr || c[0] != pc)) hb |= 1u;
+#pragma unroll
+    for (int j = 1; j < kCooPer; ++j)
+        if (i0 + j < nnz && (r[j] != r[j - 1] || c[j] != c[j - 1])) hb |= 1u << j;
+    const unsigned first_next = __shfl_down_sync(0xffffffffu, hb, 1) & 1u;
+    unsigned ends = hb >> 1;  // bit j: entry j ends its run
+    {
+        const int64_t nx = i0 + kCooPer;
+        unsigned e = first_next;
+        if (lane == 31 && nx < nnz) e = rows[nx] != r[kCooPer - 1] || cols[nx] != c[kCooPer - 1];
+        if (nx >= nnz) e = 1u;
+        ends |= e << (kCooPer - 1);
+        if (i0 < nnz && nnz - i0 < kCooPer) ends |= 1u << (nnz - 1 - i0);
+        const int64_t left = nnz - i0;
+        ends &= left >= kCooPer ? 0xffu : (left > 0 ? (1u << left) - 1u : 0u);
+    }
+    // this thread: heads, and the sum since its last head
+    const int nh = __popc(hb);
+    U s = 0;
+#pragma unroll
+    for (int j = 0; j < kCooPer; ++j) s = ((hb >> j) & 1u ? 0ull : s) + (U)v[j];
+    int hs = nh;
+    U ss = s;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int hu = __shfl_up_sync(0xffffffffu, hs, d);
+        const U su = __shfl_up_sync(0xffffffffu, ss, d);
+        if (lane >= d) {
+            if (hs == 0) ss += su;
+            hs += hu;
         }
-        atomicAdd(&out_vals[s], (unsigned long long)vals[i]);
+    }
+    int hx = __shfl_up_sync(0xffffffffu, hs, 1);  // exclusive, within the warp
+    U sx = __shfl_up_sync(0xffffffffu, ss, 1);
+    if (lane == 0) {
+        hx = 0;
+        sx = 0;
+    }
+    if (lane == 31) {
+        sh_heads[warp] = hs;
+        sh_sum[warp] = (long long)ss;
+    }
+    if (threadIdx.x == 0) sh_head0 = (int)(hb & 1u);
+    const int64_t last = (nnz - base < kCooTile ? nnz - base : kCooTile) - 1;  // the tile's last entry
+    if (threadIdx.x == last / kCooPer) sh_end = (int)((ends >> (last % kCooPer)) & 1u);
+    __syncthreads();
+    int heads = 0;  // of the tile
+    int hw = 0;     // of the warps before this one
+    U sw = 0;       // sum of the run open at this warp's start, within the tile
+    U tsum = 0;     // of the tile: the sum since its last head
+#pragma unroll
+    for (int w = 0; w < kCooT / 32; ++w) {
+        if (w == warp) {
+            hw = heads;
+            sw = tsum;
+        }
+        tsum = (sh_heads[w] ? 0ull : tsum) + (U)sh_sum[w];
+        heads += sh_heads[w];
+    }
+    if (warp == 0) {
+        U before = 0, carry = 0;
+        if (tile > 0) {
+            if (lane == 0) tile_word_store(&words[tile], 1ull | (U)heads << 2, tsum);
+            bool open = true;  // the carry is not complete
+            int64_t p = tile - 1;
+            for (;;) {
+                const int64_t q = p - lane;
+                U f = 2ull, b = 0ull;  // before the first tile: no heads, no sum
+                if (q >= 0) tile_word_load(&words[q], f, b);
+                unsigned spins = 0;
+                bool ok = true;
+                while (__any_sync(0xffffffffu, (f & 3ull) == 0ull)) {
+                    if (++spins > kSpinLimit) {
+                        ok = false;
+                        break;
+                    }
+                    if ((f & 3ull) == 0ull) tile_word_load(&words[q], f, b);
+                }
+                if (!ok) {
+                    if (lane == 0) raise_error(err, ERRBIT_TIMEOUT);
+                    break;
+                }
+                const unsigned incl = __ballot_sync(0xffffffffu, (f & 3ull) == 2ull);
+                const int stop = incl ? __ffs(incl) - 1 : 31;
+                const unsigned with_head = __ballot_sync(0xffffffffu, (f >> 2) != 0ull);
+                // the run's sum reaches back to the nearest tile with a head
+                const int reach = with_head ? min(stop, __ffs(with_head) - 1) : stop;
+                U h = lane <= stop ? f >> 2 : 0ull;
+                U x = open && lane <= reach ? b : 0ull;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    h += __shfl_xor_sync(0xffffffffu, h, o);
+                    x += __shfl_xor_sync(0xffffffffu, x, o);
+                }
+                before += h;
+                carry += x;
+                if (with_head) open = false;
+                if (incl) break;
+                p -= 32;
+            }
+        }
+        if (lane == 0) {
+            tile_word_store(&words[tile], 2ull | (before + (U)heads) << 2, heads ? tsum : carry + tsum);
+            sh_before = (long long)before;
+            sh_carry = (long long)carry;
+            if (base + kCooTile >= nnz) *out_nnz = (long long)before + heads;
+        }
+    }
+    __syncthreads();
+    const int head0 = sh_head0;
+    const int nruns = heads - head0 + sh_end;                            // runs that end here
+    const int64_t at = sh_before - (head0 ? 0 : 1);                      // the first of them
+    // the run open at this thread's start: from the lanes, the warps, the tiles before
+    U run = sx;
+    if (hx == 0) {
+        run += sw;
+        if (hw == 0) run += (U)sh_carry;
+    }
+    int slot = hw + hx - head0;  // of the run of the entry before this thread's first
+    int my[kCooPer];
+#pragma unroll
+    for (int j = 0; j < kCooPer; ++j) {
+        if ((hb >> j) & 1u) {
+            ++slot;
+            run = 0ull;
+        }
+        run += (U)v[j];
+        my[j] = slot;
+        if ((ends >> j) & 1u) sh_out[slot] = (long long)run;
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < nruns; k += kCooT) out_vals[at + k] = sh_out[k];
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kCooPer; ++j)
+        if ((ends >> j) & 1u) sh_out[my[j]] = r[j];
+    __syncthreads();
+    for (int k = threadIdx.x; k < nruns; k += kCooT) out_rows[at + k] = sh_out[k];
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kCooPer; ++j)
+        if ((ends >> j) & 1u) sh_out[my[j]] = c[j];
+    __syncthreads();
+    for (int k = threadIdx.x; k < nruns; k += kCooT) out_cols[at + k] = sh_out[k];
+}
+
+// Zeros past the canonical count, as in the reference's calloc'd result.
+__global__ void __launch_bounds__(256) coo_zero_tail_kernel(long long* __restrict__ rows, long long* __restrict__ cols,
+                                                            long long* __restrict__ vals, int64_t nnz,
+                                                            const long long* __restrict__ count) {
+    const int64_t k = *count;
+    for (int64_t i = k + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * blockDim.x) {
+        rows[i] = 0;
+        cols[i] = 0;
+        vals[i] = 0;
     }
 }
 
 // ---------------------------------------------------------------- csr build
-__global__ void csr_count_kernel(const long long* __restrict__ rows, int64_t nnz, int64_t nrows,
-                                 unsigned long long* __restrict__ counts, unsigned* err) {
+// Row counts and the copies in one pass.  Sorted entries come in runs of equal
+// rows: a warp adds each run of its 32 entries with one atomic.
+__global__ void __launch_bounds__(256) csr_count_copy_kernel(const long long* __restrict__ rows,
+                                                             const long long* __restrict__ cols,
+                                                             const long long* __restrict__ vals, int64_t nnz,
+                                                             int64_t nrows, unsigned long long* __restrict__ counts,
+                                                             long long* __restrict__ col_idx,
+                                                             long long* __restrict__ out_vals, unsigned* err) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     bool bad = false;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * blockDim.x) {
-        const long long r = rows[i];
-        if ((unsigned long long)r < (unsigned long long)nrows) atomicAdd(&counts[r], 1ULL);
-        else bad = true;
+    // warp-uniform trips: every lane takes part in the shuffles
+    for (int64_t b = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); b < nnz; b += 2 * stride) {
+        long long r[2], c[2], v[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int64_t i = b + u * stride + lane;
+            const bool in = i < nnz;
+            r[u] = in ? __ldg(rows + i) : -1;
+            c[u] = in ? __ldg(cols + i) : 0;
+            v[u] = in ? __ldg(vals + i) : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int64_t i = b + u * stride + lane;
+            const bool in = i < nnz;
+            if (in && nrows > 0) {  // with no rows every entry is out of range: nothing is copied
+                col_idx[i] = c[u];
+                out_vals[i] = v[u];
+            }
+            const bool ok = (unsigned long long)r[u] < (unsigned long long)nrows;
+            bad |= in && !ok;
+            const long long up = __shfl_up_sync(0xffffffffu, r[u], 1);
+            const bool head = lane == 0 || up != r[u];
+            const unsigned hm = __ballot_sync(0xffffffffu, head);
+            if (head && ok) {
+                const unsigned later = lane == 31 ? 0u : hm & (0xfffffffeu << lane);
+                const int len = (later ? __ffs(later) - 1 : 32) - lane;
+                atomicAdd(&counts[r[u]], (unsigned long long)len);
+            }
+        }
     }
     if (bad) raise_error(err, ERRBIT_BOUNDS);
-}
-
-template <class T>
-__global__ void copy_kernel(const T* __restrict__ src, T* __restrict__ dst, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        dst[i] = src[i];
-}
-
-__global__ void set_last_kernel(long long* row_ptr, int64_t nrows, const long long* scan_in, const long long* scan_out) {
-    // row_ptr[nrows] = total = exclusive prefix of the last row + its count
-    if (threadIdx.x == 0 && blockIdx.x == 0)
-        row_ptr[nrows] = nrows > 0 ? scan_out[nrows - 1] + scan_in[nrows - 1] : 0;
 }
 
 // ---------------------------------------------------------------- SpMV
@@ -492,24 +709,25 @@ extern "C" int hyd_cuda_coo_sum_duplicates_i64(const int64_t* rows, const int64_
     }
     Device* d = nullptr;
     HYD_TRY(device(&d));
-    void* dev_flags = nullptr;
-    HYD_TRY(device_buffer(d, "coo_flags", 2 * (size_t)nnz * 8, &dev_flags));
-    long long* flags = static_cast<long long*>(dev_flags);
-    long long* seg = flags + nnz;
+    const int64_t ntiles = (nnz + kCooTile - 1) / kCooTile;
+    HYD_CHECK_ARG(ntiles <= 0x7fffffffLL, "coo_sum_duplicates: too long");
+    const size_t bytes = 256 + sizeof(TileWord) * (size_t)ntiles;  // the ticket, then the tile words
+    void* scratch = nullptr;
+    HYD_TRY(workspace(s, bytes, nullptr, &scratch));
+    HYD_CUDA_TRY(cudaMemsetAsync(scratch, 0, bytes, s));
+    const bool vec = ((reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(cols) |
+                       reinterpret_cast<uintptr_t>(vals)) & 31) == 0;
+    coo_sum_kernel<<<(unsigned)ntiles, kCooT, 0, s>>>(
+        (const long long*)rows, (const long long*)cols, (const long long*)vals, nnz, vec, (long long*)out_rows,
+        (long long*)out_cols, (long long*)out_vals, (long long*)out_nnz,
+        reinterpret_cast<TileWord*>(static_cast<unsigned char*>(scratch) + 256), static_cast<unsigned*>(scratch),
+        d->d_err);
+    HYD_TRY(launch_check("coo_sum_duplicates"));
     int64_t blocks = (nnz + 255) / 256;
     if (blocks > d->sm_count * 8) blocks = d->sm_count * 8;
-    coo_head_flags_kernel<<<(unsigned)blocks, 256, 0, s>>>((const long long*)rows, (const long long*)cols, nnz, flags);
-    HYD_TRY(launch_check("coo_head_flags"));
-    HYD_TRY(scan_i64_launch(flags, seg, nnz, 0, false, true, s));
-    HYD_CUDA_TRY(cudaMemsetAsync(out_rows, 0, (size_t)nnz * 8, s));
-    HYD_CUDA_TRY(cudaMemsetAsync(out_cols, 0, (size_t)nnz * 8, s));
-    HYD_CUDA_TRY(cudaMemsetAsync(out_vals, 0, (size_t)nnz * 8, s));
-    coo_merge_kernel<<<(unsigned)blocks, 256, 0, s>>>((const long long*)rows, (const long long*)cols,
-                                                      (const long long*)vals, nnz, seg, (long long*)out_rows,
-                                                      (long long*)out_cols, (unsigned long long*)out_vals);
-    HYD_TRY(launch_check("coo_merge"));
-    HYD_CUDA_TRY(cudaMemcpyAsync(out_nnz, seg + nnz - 1, 8, cudaMemcpyDeviceToDevice, s));
-    return HYD_CUDA_OK;
+    coo_zero_tail_kernel<<<(unsigned)blocks, 256, 0, s>>>((long long*)out_rows, (long long*)out_cols,
+                                                          (long long*)out_vals, nnz, (const long long*)out_nnz);
+    return launch_check("coo_sum_duplicates");
 }
 
 extern "C" int hyd_cuda_csr_from_sorted_coo_i64(int64_t nrows, int64_t nnz, const int64_t* rows, const int64_t* cols,
@@ -521,31 +739,26 @@ extern "C" int hyd_cuda_csr_from_sorted_coo_i64(int64_t nrows, int64_t nnz, cons
     cudaStream_t s = as_stream(stream);
     Device* d = nullptr;
     HYD_TRY(device(&d));
-    if (nrows == 0) {
-        HYD_CUDA_TRY(cudaMemsetAsync(row_ptr, 0, 8, s));
-        if (nnz > 0) {
-            // every entry's row is out of range
-            csr_count_kernel<<<1, 32, 0, s>>>((const long long*)rows, nnz, 0, nullptr, d->d_err);
-            HYD_TRY(launch_check("csr_count"));
-        }
-        return HYD_CUDA_OK;
-    }
-    void* buf = nullptr;
-    HYD_TRY(device_buffer(d, "csr_counts", (size_t)nrows * 8, &buf));
-    unsigned long long* counts = static_cast<unsigned long long*>(buf);
-    HYD_CUDA_TRY(cudaMemsetAsync(counts, 0, (size_t)nrows * 8, s));
-    int64_t blocks = (nnz + 255) / 256;
-    if (blocks > d->sm_count * 8) blocks = d->sm_count * 8;
-    if (blocks < 1) blocks = 1;
+    // nrows + 1 counts (the last stays zero), so that their exclusive scan is
+    // the whole row_ptr, the total included
+    const int64_t m = nrows + 1;
+    auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t count_bytes = al((size_t)m * 8);
+    unsigned* counters = nullptr;
+    void* scratch = nullptr;
+    HYD_TRY(workspace(s, count_bytes + al(scan_i64_scratch_bytes(m)), &counters, &scratch));
+    unsigned long long* counts = static_cast<unsigned long long*>(scratch);
+    HYD_CUDA_TRY(cudaMemsetAsync(counts, 0, count_bytes, s));
     if (nnz > 0) {
-        csr_count_kernel<<<(unsigned)blocks, 256, 0, s>>>((const long long*)rows, nnz, nrows, counts, d->d_err);
+        int64_t blocks = (nnz + 255) / 256;
+        if (blocks > d->sm_count * 8) blocks = d->sm_count * 8;
+        csr_count_copy_kernel<<<(unsigned)blocks, 256, 0, s>>>((const long long*)rows, (const long long*)cols,
+                                                               (const long long*)vals, nnz, nrows, counts,
+                                                               (long long*)col_idx, (long long*)out_vals, d->d_err);
         HYD_TRY(launch_check("csr_count"));
-        copy_kernel<long long><<<(unsigned)blocks, 256, 0, s>>>((const long long*)cols, (long long*)col_idx, nnz);
-        copy_kernel<long long><<<(unsigned)blocks, 256, 0, s>>>((const long long*)vals, (long long*)out_vals, nnz);
     }
-    HYD_TRY(scan_i64_launch((const long long*)counts, (long long*)row_ptr, nrows, 0, false, false, s));
-    set_last_kernel<<<1, 32, 0, s>>>((long long*)row_ptr, nrows, (const long long*)counts, (const long long*)row_ptr);
-    return launch_check("csr_from_sorted_coo");
+    return scan_i64_launch_with((const long long*)counts, (long long*)row_ptr, m, 0, false, false,
+                                static_cast<unsigned char*>(scratch) + count_bytes, counters + 8, s);
 }
 
 extern "C" int hyd_cuda_spmv_csr_f64(int64_t nrows, int64_t ncols, const int64_t* row_ptr, const int64_t* col_idx,
