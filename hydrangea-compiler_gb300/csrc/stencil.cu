@@ -15,9 +15,14 @@
 // is exact -- `t3 - 4e` and `t3 + e*-4` are one fma because 4e is exact (for
 // |e| < DBL_MAX/4), and /4.0 is *0.25 (both correctly rounded, same value).
 //
-// GB300 design.  fp64 runs at ~1.9 DFMA/clk/SM on this part, so a 5-point fp64
-// step is bound by the FP64 pipe (6 DP ops per point for HEAT), not by HBM.
-// The kernel therefore spends nothing but DP ops in its inner loop:
+// GB300 design.  FP64 runs at 1.7 operations per clock and SM on this part, so
+// a 5-point fp64 step is bound by the FP64 pipe (6 operations per point for
+// HEAT: 768 us per step at 8192^2), not by HBM (158 us).  The default kernel
+// therefore does the neighbour sum on the integer pipe, exactly (fp64_emu.cuh),
+// sweeping rows of a column per thread: HEAT 369 us per step, its FP64 pipe
+// (2.75 operations per point) and its ALU pipe both near 90% busy, JACOBI 312,
+// HEAT_EXAMPLE 415; with two additions emulated one by one they took 528, 418
+// and 895.  The tiled kernels bring each tile through shared memory:
 //  * a persistent grid walks 16 x 128 output tiles; each tile plus its halo
 //    (rows -1..+1, columns -2..+2 so the TMA x coordinate stays 16-byte
 //    aligned) is brought into shared memory by a 2-D TMA load
@@ -46,13 +51,17 @@ namespace hyd {
 
 enum { ST_LAPLACIAN = 0, ST_JACOBI = 1, ST_HEAT = 2, ST_HEAT_EXAMPLE = 3 };
 
-// EMU: how many of the three additions a + b, + c, + d run on the integer
-// pipe (dadd_pos, bit-identical to __dadd_rn); the rest use the FP64 unit.
+// EMU: how much of the body runs on the integer pipe, bit-identical to the
+// FP64 unit.  0: nothing; 2: two of the three additions a + b, + c, + d, each on
+// its own (dadd_pos); 3: the whole sum on one grid (fp64_emu.cuh), with the
+// divisions of JACOBI and HEAT_EXAMPLE; 4: HEAT's `- 4e` too.
 template <int KIND, int EMU>
 __device__ __forceinline__ double stencil_body(double a, double b, double c, double d, double e) {
-    const double t1 = EMU >= 1 ? dadd_pos(a, b) : __dadd_rn(a, b);
-    const double t2 = EMU >= 2 ? dadd_pos(t1, c) : __dadd_rn(t1, c);
-    const double t3 = EMU >= 3 ? dadd_pos(t2, d) : __dadd_rn(t2, d);
+    if (EMU >= 3 && KIND == ST_JACOBI) return dmean4_pos(a, b, c, d);
+    if (EMU >= 3 && KIND == ST_HEAT_EXAMPLE) return dmean5_pos(a, b, c, d, e);
+    if (EMU >= 4 && KIND == ST_HEAT) return __dadd_rn(e, __dmul_rn(0.1, dlap4_pos(a, b, c, d, e)));
+    const double t3 = EMU >= 3 ? dsum4_pos(a, b, c, d)
+                               : __dadd_rn(EMU >= 2 ? dadd_pos(dadd_pos(a, b), c) : __dadd_rn(__dadd_rn(a, b), c), d);
     if (KIND == ST_LAPLACIAN) return __fma_rn(e, -4.0, t3);
     if (KIND == ST_JACOBI) return __dmul_rn(t3, 0.25);
     if (KIND == ST_HEAT) {
@@ -63,17 +72,32 @@ __device__ __forceinline__ double stencil_body(double a, double b, double c, dou
 }
 
 // ---------------------------------------------------------------- plain path
-template <int KIND, int EMU>
+// A thread sweeps kRows rows of one column, carrying the rows above and at the
+// point in registers: three loads per point.
+template <int KIND, int EMU, int kRows>
 __global__ void __launch_bounds__(256) stencil_plain_kernel(const double* __restrict__ in,
                                                             double* __restrict__ out, int64_t h,
                                                             int64_t w) {
     const int64_t j = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
-    const int64_t i = (int64_t)blockIdx.y * 8 + (threadIdx.x >> 5);
-    if (i >= h || j >= w) return;
-    const int64_t im = i > 0 ? i - 1 : 0, ip = i + 1 < h ? i + 1 : h - 1;
+    const int64_t i0 = ((int64_t)blockIdx.y * 8 + (threadIdx.x >> 5)) * kRows;
+    if (i0 >= h || j >= w) return;
     const int64_t jm = j > 0 ? j - 1 : 0, jp = j + 1 < w ? j + 1 : w - 1;
-    out[i * w + j] = stencil_body<KIND, EMU>(in[im * w + j], in[ip * w + j], in[i * w + jm],
-                                        in[i * w + jp], in[i * w + j]);
+    const double* row = in + i0 * w;
+    double* o = out + i0 * w + j;
+    double up = in[(i0 > 0 ? i0 - 1 : 0) * w + j], mid = row[j];
+#pragma unroll
+    for (int k = 0; k < kRows; ++k) {
+        if (kRows > 1 && i0 + k >= h) break;
+        const double* const next = i0 + k + 1 < h ? row + w : row;
+        const double dn = next[j];
+        // HEAT: `- 4e` on the integer pipe in one row of four balances the pipes
+        *o = KIND == ST_HEAT && EMU == 3 && (k & 3) == 3 ? stencil_body<KIND, 4>(up, dn, row[jm], row[jp], mid)
+                                                    : stencil_body<KIND, EMU>(up, dn, row[jm], row[jp], mid);
+        up = mid;
+        mid = dn;
+        row = next;
+        o += w;
+    }
 }
 
 // ---------------------------------------------------------------- TMA path
@@ -253,8 +277,8 @@ constexpr int kPlainShape = kNumTiles;
 constexpr int kEmuLevels[] = {0, 2, 3};
 constexpr int kNumLevels = sizeof(kEmuLevels) / sizeof(kEmuLevels[0]);
 constexpr int kNumVariants = kShapes * kNumLevels;
-constexpr int kDefaultVariant = kPlainShape + kShapes;  // plain kernel, 2 integer-pipe sums
-                                                        // (fastest at 8192^2 heat on GB300)
+constexpr int kDefaultVariant = kPlainShape + 2 * kShapes;  // plain kernel, all three sums on the integer pipe
+                                                            // (fastest at 8192^2 heat on GB300)
 
 template <int KIND, int TH, int TW, int EMU>
 static int launch_tma(const CUtensorMap* map, double* out, int64_t h, int64_t w, const Device* d, cudaStream_t stream) {
@@ -282,8 +306,15 @@ static int launch_shape(const CUtensorMap* map, const double* in, double* out, i
         case 4: HYD_TRY((launch_tma<KIND, 8, 128, EMU>(map, out, h, w, d, stream))); break;
         case 5: HYD_TRY((launch_tma<KIND, 32, 128, EMU>(map, out, h, w, d, stream))); break;
         default: {
-            dim3 grid((unsigned)((w + 31) / 32), (unsigned)((h + 7) / 8));
-            stencil_plain_kernel<KIND, EMU><<<grid, 256, 0, stream>>>(in, out, h, w);
+            // four rows per thread once that still gives every SM its eight
+            // blocks, eight when there are ten waves of them (HEAT: 8192^2 369 us
+            // with eight rows, 375 with four; 3000^2 54.8 and 53.2)
+            const int64_t points = h * w, fill = (int64_t)d->sm_count * 8 * 256;
+            const int rows = points >= 80 * fill ? 8 : points >= 4 * fill ? 4 : 1;
+            dim3 grid((unsigned)((w + 31) / 32), (unsigned)((h + 8 * rows - 1) / (8 * rows)));
+            if (rows == 8) stencil_plain_kernel<KIND, EMU, 8><<<grid, 256, 0, stream>>>(in, out, h, w);
+            else if (rows == 4) stencil_plain_kernel<KIND, EMU, 4><<<grid, 256, 0, stream>>>(in, out, h, w);
+            else stencil_plain_kernel<KIND, EMU, 1><<<grid, 256, 0, stream>>>(in, out, h, w);
         }
     }
     return launch_check("stencil2d_f64");

@@ -265,8 +265,9 @@ void hyd_cuda_stencil_release_graphs(void);
  * TMA tile shapes (0 = 32x32, the reference's fixed polyhedral tile,
  * Polyhedral.hs:196-204; 1 = 16x128, 2 = 16x64, 3 = 32x64, 4 = 8x128,
  * 5 = 32x128), 6 = the plain non-TMA kernel.  Levels 0, 1, 2 run 0, 2, 3 of
- * the three additions of the 4-neighbour sum on the integer pipe (exact
- * round-to-nearest-even; FP64 is the scarce pipe on GB300).  All 21 variants
+ * the three additions of the 4-neighbour sum on the integer pipe, level 2 with
+ * the divisions too (exact round-to-nearest-even; FP64 is the scarce pipe on
+ * GB300).  All 21 variants
  * give identical bits. */
 int hyd_cuda_stencil2d_f64_variant(int kind, const double* in, double* out, int64_t h, int64_t w,
                                    int variant, void* stream);
