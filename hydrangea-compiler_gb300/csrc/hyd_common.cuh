@@ -209,6 +209,14 @@ __device__ __forceinline__ void bulk_load_1d(unsigned dst, const void* src, unsi
         : "memory");
 }
 
+// Asks for the 16-byte units that lie inside [p, p + bytes) to be brought into
+// L2 (one thread; nothing waits for it).
+__device__ __forceinline__ void l2_prefetch(const void* p, int64_t bytes) {
+    const uint64_t a = (reinterpret_cast<uint64_t>(p) + 15) & ~15ull;
+    const int64_t n = (int64_t)((reinterpret_cast<uint64_t>(p) + (uint64_t)bytes) & ~15ull) - (int64_t)a;
+    if (n > 0) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)n) : "memory");
+}
+
 // ---- decoupled look-back: tile status words and the bounded window wait ------
 constexpr unsigned kSpinLimit = 1u << 22;  // polls before a look-back gives up
 

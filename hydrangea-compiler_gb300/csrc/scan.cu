@@ -3,18 +3,21 @@
 // Replaces the serial LoopFold of lowerScanFamily (Lowering.hs:3563-3612; the
 // C backend never parallelises a fold, Parallelize.hs:517).
 //
-// int64: single-pass decoupled look-back (Merrill & Garland, "Single-pass
-// Parallel Prefix Scan with Decoupled Look-back", 2016).  Tiles of 4096
-// elements take their id from an atomic counter in launch order, so every
-// predecessor a tile waits on has already started; a tile publishes its
-// aggregate, a warp looks back 32 predecessors at a time, then publishes its
-// inclusive prefix.  A tile's status is one 16-byte {flag, value} word
-// (TileWord), written and read whole, so a look-back window costs one memory
-// round trip.  Every spin is bounded (error bit, no hang).  int64 adds wrap
-// and commute, so the result is bit-identical to the serial C fold.  One
-// read and one write per element: 16 B/element of HBM traffic.
+// int64: two launches over contiguous ranges, one per warp: the ranges' sums,
+// then the scans.  int64 adds wrap and commute, so the result is bit-identical
+// to the serial C fold.  Measured against the single-pass look-back this took
+// the place of (start -> now): 2^22 elements 30.3 -> 22.6 us, 2e7 94 -> 84 us,
+// 2^27 540 -> 512 us; 24 bytes of traffic per element bound it.  float64 takes
+// the same form up to 2^17 elements (12.3 -> 10.2 us); above, its third pass of
+// FP64 additions costs more than the look-back (1e6: 28.7 against 16.9 us).
 //
-// float64: single pass, deterministic in two levels.  Within a block of 32
+// float64 above that: single pass, a decoupled look-back (Merrill & Garland,
+// "Single-pass Parallel Prefix Scan with Decoupled Look-back", 2016),
+// deterministic in two levels.  Tiles of 4096 elements take their id from an
+// atomic counter in launch order, so every predecessor a tile waits on has
+// already started.  A tile's status is one 16-byte {flag, value} word
+// (TileWord), written and read whole, so a look-back window costs one memory
+// round trip.  Every spin is bounded (error bit, no hang).  Within a block of 32
 // tiles a tile's prefix over its block-mates comes from a fixed warp scan of
 // their aggregates; across blocks the block totals are folded left to right
 // through the same kind of look-back (lookback_fold).  Every value is defined
@@ -22,6 +25,9 @@
 // a tile the order is fixed too (per-thread serial sums, a fixed shuffle
 // tree).  A parallel prefix cannot reproduce the serial fold's roundings; the
 // tolerance is |gpu - c| <= 1e-12 * prefix sum of |x| (stated in the tests).
+// FP64 bounds it: 2.3 additions per element (15 + 5 + 2 + 16 per thread of 16),
+// 586 us of the 744 us at 2^27 (812 with 8 per thread, 2.6 additions, the two
+// levels of the look-back one after the other and no prefetch).
 //
 // Tiles pass through shared memory padded with one slot per 16 elements, so
 // the blocked (8 consecutive elements per thread) and striped accesses are
@@ -33,80 +39,43 @@
 
 namespace hyd {
 
-constexpr int kScanT = 512;
-constexpr int kScanIPT = 8;
-constexpr int kScanTile = kScanT * kScanIPT;  // 4096 (32 KiB of static shared memory for int64)
-constexpr int kScanCtasPerSm = 4;  // resident CTAs per SM (32 registers per thread)
+constexpr int kScanT = 256;
+constexpr int kScanWarps = kScanT / 32;
+constexpr int kScanIPT = 16;
+constexpr int kScanTile = kScanT * kScanIPT;  // 4096
+constexpr int kScanCtasPerSm = 4;  // resident CTAs per SM (64 registers per thread)
 // Tiles sit in shared memory with one 8-byte pad after every 16 elements: a
-// thread's blocked run of 8 (stride 64 B between lanes) and the striped
+// thread's blocked run of 16 (an odd stride between lanes) and the striped
 // accesses then both meet no bank conflict.  Unpadded, the blocked accesses
 // were 16-way conflicted and the tile copy alone ran at half the copy rate.
 constexpr int kScanTileP = kScanTile + kScanTile / 16;
 __device__ __forceinline__ int scan_pad(int i) { return i + (i >> 4); }
 
-// --- block-wide exclusive scan of one value per thread (int64, wrapping) ------
+// Inclusive scan of one value per lane, fixed order.
 template <class T>
-__device__ __forceinline__ T block_exclusive_scan(T v, T* sh /*[32]*/, T& total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    T incl = v;
+__device__ __forceinline__ T warp_inclusive_scan(T v) {
+    const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        T y = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += y;
+        const T y = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v = y + v;
     }
-    if (lane == 31) sh[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        T w = lane < nw ? sh[lane] : T(0);
-        T wi = w;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            T y = __shfl_up_sync(0xffffffffu, wi, d);
-            if (lane >= d) wi += y;
-        }
-        sh[lane] = wi - w;  // exclusive warp offsets
-        if (lane == 31) sh[32] = wi;
-    }
-    __syncthreads();
-    total = sh[32];
-    T r = sh[warp] + incl - v;
-    __syncthreads();
-    return r;
+    return v;
 }
-
-// The same for float64, without the subtraction the integer form uses for the
-// exclusive value (one FP64 operation fewer per thread; the FP64 pipe bounds
-// the float64 scan): the exclusive value of a lane is its left neighbour's
-// inclusive one.  Fixed order, so run-to-run identical.
+// Warp 0: the exclusive prefixes of the warps' totals (lane w gets warp w's,
+// computed without a subtraction) and the block's total.
 template <class T>
-__device__ __forceinline__ T block_exclusive_scan_shift(T v, T* sh /*[33]*/, T& total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    T incl = v;
+__device__ __forceinline__ T scan_warp_totals(const T* totals, T& total) {
+    const int lane = threadIdx.x & 31;
+    T w = lane < kScanWarps ? totals[lane] : T(0);
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const T y = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl = y + incl;
+    for (int d = 1; d < kScanWarps; d <<= 1) {
+        const T y = __shfl_up_sync(0xffffffffu, w, d);
+        if (lane >= d) w = y + w;
     }
-    if (lane == 31) sh[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        const T w = lane < nw ? sh[lane] : T(0);
-        T wi = w;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const T y = __shfl_up_sync(0xffffffffu, wi, d);
-            if (lane >= d) wi = y + wi;
-        }
-        const T wx = __shfl_up_sync(0xffffffffu, wi, 1);
-        sh[lane] = lane == 0 ? T(0) : wx;  // exclusive warp offsets
-        if (lane == 31) sh[32] = wi;
-    }
-    __syncthreads();
-    total = sh[32];
-    const T lx = __shfl_up_sync(0xffffffffu, incl, 1);
-    const T r = lane == 0 ? sh[warp] : sh[warp] + lx;
-    __syncthreads();
-    return r;
+    total = __shfl_sync(0xffffffffu, w, kScanWarps - 1);
+    const T x = __shfl_up_sync(0xffffffffu, w, 1);
+    return lane == 0 ? T(0) : x;
 }
 
 // Tile load/store in blocked arrangement through shared memory: global
@@ -129,6 +98,17 @@ __device__ __forceinline__ void tile_load(const T* in, int64_t n, int64_t base, 
     __syncthreads();
 }
 
+// Brings the tile `ahead` tiles further on into L2: a tile's look-back waits for
+// the slowest load among the tiles in flight before it, and L2 hits vary less
+// (755 -> 744 us at 2^27, one wave of tiles ahead).
+template <class T>
+__device__ __forceinline__ void tile_prefetch(const T* in, int64_t n, int64_t base, int64_t ahead, bool reverse) {
+    const int64_t k = base + ahead * kScanTile;
+    if (k >= n) return;
+    const int64_t cnt = n - k < kScanTile ? n - k : kScanTile;
+    l2_prefetch(in + (reverse ? n - k - cnt : k), cnt * (int64_t)sizeof(T));
+}
+
 template <class T>
 __device__ __forceinline__ void tile_store(T* out, int64_t n, int64_t base, bool reverse, T* sh,
                                            const T (&items)[kScanIPT]) {
@@ -141,89 +121,169 @@ __device__ __forceinline__ void tile_store(T* out, int64_t n, int64_t base, bool
     }
 }
 
-// ---- int64 decoupled look-back ----------------------------------------------------
-// One TileWord per tile (flag 0 none, 1 aggregate, 2 inclusive prefix).
-struct ScanStatus {
-    TileWord* word;
-    unsigned* tile_counter;
-};
+// ---- two launches: sums, then scans ---------------------------------------------
+// Every warp takes one contiguous range of the elements, in steps of 256.  The
+// first launch sums the ranges (no output); in the second a warp adds up the
+// sums of the ranges before its own and scans its range step by step, carrying
+// the prefix along.  24 bytes per element instead of the look-back's 16, but
+// no tile waits for another: with a look-back a tile spent 40% of its time on
+// the slowest of the 600 tiles in flight before it.
+constexpr int kRangeT = 256;
+constexpr int kRangeWarps = kRangeT / 32;
+constexpr int kRangePer = 8;                   // elements per lane and step
+constexpr int kRangeStep = 32 * kRangePer;
+constexpr int kRangeCtasPerSm = 4;
+constexpr int64_t kScanRangesF64 = 1 << 17;
+constexpr int kRangeSlots = kRangeStep + kRangeStep / 16;
+// per-warp staging, one 8-byte pad after every 16: blocked and striped accesses
+// are both free of bank conflicts
 
-__global__ void __launch_bounds__(kScanT, kScanCtasPerSm) scan_i64_lookback_kernel(const long long* __restrict__ in,
-                                                                    long long* __restrict__ out, int64_t n,
-                                                                    long long init, bool reverse,
-                                                                    bool inclusive, ScanStatus st,
-                                                                    unsigned* err) {
-    __shared__ long long sh_tile[kScanTileP];
-    __shared__ long long sh_scan[33];
-    __shared__ unsigned sh_tile_id;
-    __shared__ long long sh_prefix;
-    if (threadIdx.x == 0) sh_tile_id = atomicAdd(st.tile_counter, 1u);
-    __syncthreads();
-    const unsigned tile = sh_tile_id;
-    const int64_t base = (int64_t)tile * kScanTile;
-
-    long long items[kScanIPT];
-    tile_load(in, n, base, reverse, sh_tile, items);
-    long long tsum = 0;
+// Elements k0 + lane + 32 j (logical positions; past `end` zero).
+template <class T>
+__device__ __forceinline__ void range_load(const T* __restrict__ in, int64_t n, int64_t k0, int64_t end, bool reverse,
+                                           T (&v)[kRangePer]) {
+    const int lane = threadIdx.x & 31;
+    const T* const p = reverse ? in + (n - 1 - k0) - lane : in + k0 + lane;
+    if (k0 + kRangeStep <= end) {
+        if (reverse) {
 #pragma unroll
-    for (int j = 0; j < kScanIPT; ++j) tsum += items[j];
-    long long agg;
-    const long long texcl = block_exclusive_scan(tsum, sh_scan, agg);
-
-    // publish and look back (warp 0)
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        if (tile == 0) {
-            if (lane == 0) {
-                tile_word_store(&st.word[0], 2ull, to_bits(init + agg));
-                sh_prefix = init;
-            }
+            for (int j = 0; j < kRangePer; ++j) v[j] = __ldg(p - 32 * j);
         } else {
-            if (lane == 0) tile_word_store(&st.word[tile], 1ull, to_bits(agg));
-            long long running = 0;
-            int64_t p = (int64_t)tile - 1;  // window covers p, p-1, ..., p-31
-            for (;;) {
-                const int64_t q = p - lane;
-                // wait until every tile of the window has published something
-                unsigned long long bits;
-                const unsigned f = lookback_wait_words(st.word, p, lane, bits);
-                if (f == 0u) {
-                    if (lane == 0) raise_error(err, ERRBIT_TIMEOUT);
-                    break;
-                }
-                const unsigned incl_mask = __ballot_sync(0xffffffffu, f == 2u);
-                // nearest predecessor with an inclusive prefix (lowest lane):
-                // the aggregates of the lanes before it, then its prefix (before
-                // tile 0: the fold's initial value)
-                const int stop = incl_mask ? (__ffs(incl_mask) - 1) : 32;
-                long long v = 0;
-                if (lane <= stop) v = q >= 0 ? from_bits<long long>(bits) : init;
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                running += v;
-                if (stop < 32) break;
-                p -= 32;
-            }
-            if (lane == 0) {
-                tile_word_store(&st.word[tile], 2ull, to_bits(running + agg));
-                sh_prefix = running;
-            }
+            for (int j = 0; j < kRangePer; ++j) v[j] = __ldg(p + 32 * j);
         }
-    }
-    __syncthreads();
-    long long acc = sh_prefix + texcl;
+    } else {
 #pragma unroll
-    for (int j = 0; j < kScanIPT; ++j) {
-        const long long x = items[j];
+        for (int j = 0; j < kRangePer; ++j)
+            v[j] = k0 + lane + 32 * j < end ? __ldg(reverse ? p - 32 * j : p + 32 * j) : T(0);
+    }
+}
+
+template <class T>
+__global__ void __launch_bounds__(kRangeT, kRangeCtasPerSm)
+    scan_sums_kernel(const T* __restrict__ in, int64_t n, bool reverse, int64_t range, T* __restrict__ sums) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int64_t w = (int64_t)blockIdx.x * kRangeWarps + (threadIdx.x >> 5);
+    const int64_t lo = w * range, end = lo + range < n ? lo + range : n;
+    T acc[kRangePer];
+#pragma unroll
+    for (int j = 0; j < kRangePer; ++j) acc[j] = T(0);
+    // from the range's end to its start: what was read last is still in L2 when
+    // the second launch reads it first
+    int64_t k = end > lo ? lo + (end - lo - 1) / kRangeStep * kRangeStep : lo - kRangeStep;
+    for (; k > lo; k -= 2 * kRangeStep) {
+        T a[kRangePer], b[kRangePer];
+        range_load(in, n, k, end, reverse, a);
+        range_load(in, n, k - kRangeStep, end, reverse, b);
+#pragma unroll
+        for (int j = 0; j < kRangePer; ++j) acc[j] += a[j];
+#pragma unroll
+        for (int j = 0; j < kRangePer; ++j) acc[j] += b[j];
+    }
+    if (k == lo) {
+        T a[kRangePer];
+        range_load(in, n, k, end, reverse, a);
+#pragma unroll
+        for (int j = 0; j < kRangePer; ++j) acc[j] += a[j];
+    }
+    T s = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) sums[w] = s;
+}
+
+template <class T>
+__global__ void __launch_bounds__(kRangeT, kRangeCtasPerSm)
+    scan_ranges_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t n, T init, bool reverse, bool inclusive,
+                       int64_t range, const T* __restrict__ sums) {
+    __shared__ T sh[kRangeWarps][kRangeSlots];
+    __shared__ T sh_part[kRangeWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T* const st = sh[warp];
+    const int64_t w = (int64_t)blockIdx.x * kRangeWarps + warp;
+    const int64_t lo = w * range, end = lo + range < n ? lo + range : n;
+    T v[kRangePer];
+    if (lo < end) range_load(in, n, lo, end, reverse, v);  // does not depend on the sums
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // the sums of all ranges before this block's (fixed order), then before this warp's
+    T part = T(0);
+    for (int64_t u = threadIdx.x; u < (int64_t)blockIdx.x * kRangeWarps; u += kRangeT) part += __ldcg(sums + u);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    if (lane == 0) sh_part[warp] = part;
+    __syncthreads();
+    T carry = T(0);
+#pragma unroll
+    for (int u = 0; u < kRangeWarps; ++u) carry += sh_part[u];
+    for (int u = 0; u < warp; ++u) carry += __ldcg(sums + (int64_t)blockIdx.x * kRangeWarps + u);
+    carry = init + carry;
+    for (int64_t k = lo; k < end; k += kRangeStep) {
+        // to blocked: lane l then holds elements k + 8l .. k + 8l + 7
+#pragma unroll
+        for (int j = 0; j < kRangePer; ++j) st[scan_pad(lane + 32 * j)] = v[j];
+        __syncwarp();
+        T x[kRangePer];
+#pragma unroll
+        for (int j = 0; j < kRangePer; ++j) x[j] = st[scan_pad(kRangePer * lane + j)];
+        __syncwarp();
+        if (k + kRangeStep < end) range_load(in, n, k + kRangeStep, end, reverse, v);  // the next step's
+#pragma unroll
+        for (int j = 1; j < kRangePer; ++j) x[j] = x[j - 1] + x[j];
+        const T incl = warp_inclusive_scan(x[kRangePer - 1]);
+        const T left = __shfl_up_sync(0xffffffffu, incl, 1);
+        const T p = lane == 0 ? carry : carry + left;
+        carry = carry + __shfl_sync(0xffffffffu, incl, 31);
         if (inclusive) {
-            acc += x;
-            items[j] = acc;
+#pragma unroll
+            for (int j = 0; j < kRangePer; ++j) x[j] = p + x[j];
         } else {
-            items[j] = acc;
-            acc += x;
+#pragma unroll
+            for (int j = kRangePer - 1; j > 0; --j) x[j] = p + x[j - 1];
+            x[0] = p;
         }
+#pragma unroll
+        for (int j = 0; j < kRangePer; ++j) st[scan_pad(kRangePer * lane + j)] = x[j];
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < kRangePer; ++j) {
+            const int64_t q = k + lane + 32 * j;
+            if (q < end) out[reverse ? n - 1 - q : q] = st[scan_pad(lane + 32 * j)];
+        }
+        __syncwarp();
     }
-    tile_store(out, n, base, reverse, sh_tile, items);
+}
+
+// Bytes of scratch, and the launches (`scratch`: 8-byte aligned).
+static int64_t range_blocks(const Device* d, int64_t n) {
+    const int64_t want = (n + kRangeStep * kRangeWarps - 1) / (kRangeStep * kRangeWarps);
+    const int64_t cap = (int64_t)d->sm_count * kRangeCtasPerSm;
+    return want < cap ? want : cap;
+}
+template <class T>
+static int scan_ranges_launch(const T* in, T* out, int64_t n, T init, bool reverse, bool inclusive, void* scratch,
+                              cudaStream_t stream, const char* what) {
+    Device* d = nullptr;
+    HYD_TRY(device(&d));
+    const int64_t blocks = range_blocks(d, n), warps = blocks * kRangeWarps;
+    const int64_t steps = (n + kRangeStep - 1) / kRangeStep;
+    const int64_t range = (steps + warps - 1) / warps * kRangeStep;
+    T* const sums = static_cast<T*>(scratch);
+    scan_sums_kernel<T><<<(unsigned)blocks, kRangeT, 0, stream>>>(in, n, reverse, range, sums);
+    HYD_TRY(launch_check(what));
+    // programmatic dependent launch: the scans' blocks load their first steps
+    // while the sums finish
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(kRangeT);
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    HYD_CUDA_TRY(cudaLaunchKernelEx(&cfg, scan_ranges_kernel<T>, in, out, n, init, reverse, inclusive, range,
+                                    (const T*)sums));
+    return launch_check(what);
 }
 
 // ---- deterministic decoupled look-back (left fold) -----------------------------------
@@ -302,27 +362,34 @@ __device__ bool lookback_fold(const FoldStatus<T>& st, int64_t tile, T before, T
 template <class T>
 __global__ void __launch_bounds__(kScanT, kScanCtasPerSm) scan_fold_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t n,
                                                             T init, bool reverse, bool inclusive, FoldStatus<T> st,
-                                                            FoldStatus<T> bst, unsigned* err) {
+                                                            FoldStatus<T> bst, int ahead, unsigned* err) {
     __shared__ T sh_tile[kScanTileP];
-    __shared__ T sh_scan[33];
+    __shared__ T sh_total[kScanWarps];  // the warps' totals, then their offsets in the tile
     __shared__ T sh_fold[kFoldBuf];
     __shared__ unsigned sh_tile_id;
-    __shared__ T sh_prefix;
-    if (threadIdx.x == 0) sh_tile_id = atomicAdd(st.tile_counter, 1u);
+    __shared__ T sh_within, sh_before;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        sh_tile_id = atomicAdd(st.tile_counter, 1u);
+        tile_prefetch(in, n, (int64_t)sh_tile_id * kScanTile, ahead, reverse);
+    }
     __syncthreads();
     const unsigned tile = sh_tile_id;
     const int64_t base = (int64_t)tile * kScanTile;
+    const int64_t blk = tile >> 5;
+    const int pos = (int)(tile & 31u);
     T items[kScanIPT];
     tile_load(in, n, base, reverse, sh_tile, items);
     // the thread's running sums, in place: items[j] = x_0 + ... + x_j
 #pragma unroll
     for (int j = 1; j < kScanIPT; ++j) items[j] = items[j - 1] + items[j];
-    T agg;
-    const T texcl = block_exclusive_scan_shift(items[kScanIPT - 1], sh_scan, agg);
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        const int64_t blk = tile >> 5;
-        const int pos = (int)(tile & 31u);
+    const T incl = warp_inclusive_scan(items[kScanIPT - 1]);
+    if (lane == 31) sh_total[warp] = incl;
+    __syncthreads();
+    T off = T(0), total = T(0);
+    if (warp == 0) {
+        T agg;
+        off = scan_warp_totals(sh_total, agg);
         if (lane == 0) tile_word_store(&st.word[tile], 1ull, to_bits(agg));
         // the aggregates of the block's tiles before this one (earlier tickets)
         unsigned long long f = 1ull, bits = 0ull;
@@ -337,23 +404,29 @@ __global__ void __launch_bounds__(kScanT, kScanCtasPerSm) scan_fold_kernel(const
             if (f == 0ull) tile_word_load(&st.word[(blk << 5) + lane], f, bits);
         }
         if (!ok && lane == 0) raise_error(err, ERRBIT_TIMEOUT);
-        T sc = lane < pos ? from_bits<T>(bits) : (lane == pos ? agg : T(0));
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const T y = __shfl_up_sync(0xffffffffu, sc, d);
-            if (lane >= d) sc = y + sc;
-        }
+        const T sc = warp_inclusive_scan(lane < pos ? from_bits<T>(bits) : (lane == pos ? agg : T(0)));
         const T within = __shfl_sync(0xffffffffu, sc, pos > 0 ? pos - 1 : 0);
-        const T total = __shfl_sync(0xffffffffu, sc, 31);
-        if (pos == 31 && lane == 0) tile_word_store(&bst.word[blk], 1ull, to_bits(total));
+        total = __shfl_sync(0xffffffffu, sc, 31);
+        if (lane == 0) {
+            if (pos == 31) tile_word_store(&bst.word[blk], 1ull, to_bits(total));
+            sh_within = within;
+        }
+    } else if (warp == 1) {
         T before = init;  // B(blk - 1)
         if (!lookback_fold(bst, blk, init, sh_fold, before) && lane == 0) raise_error(err, ERRBIT_TIMEOUT);
+        if (lane == 0) sh_before = before;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const T before = sh_before;
         if (pos == 31 && lane == 0) tile_word_store(&bst.word[blk], 2ull, to_bits(before + total));
-        if (lane == 0) sh_prefix = pos == 0 ? before : before + within;
+        const T prefix = pos == 0 ? before : before + sh_within;
+        if (lane < kScanWarps) sh_total[lane] = prefix + off;
     }
     __syncthreads();
     // outputs: the thread's prefix plus its running sums (one addition each)
-    const T p = sh_prefix + texcl;
+    const T left = __shfl_up_sync(0xffffffffu, incl, 1);
+    const T p = lane == 0 ? sh_total[warp] : sh_total[warp] + left;
     if (inclusive) {
 #pragma unroll
         for (int j = 0; j < kScanIPT; ++j) items[j] = p + items[j];
@@ -370,38 +443,27 @@ __global__ void __launch_bounds__(kScanT, kScanCtasPerSm) scan_fold_kernel(const
 using namespace hyd;
 
 namespace hyd {
-// Scratch bytes the decoupled look-back needs for n elements.
+// Scratch bytes of an int64 scan, at most.
 size_t scan_i64_scratch_bytes(int64_t n) {
-    const int64_t ntiles = (n + kScanTile - 1) / kScanTile;
-    return sizeof(TileWord) * (size_t)ntiles + 256;  // + room to align the words to 16 bytes
+    const int64_t steps = (n + kRangeStep - 1) / kRangeStep + kRangeWarps;
+    const int64_t most = 1 << 16;  // more warps than any grid here has
+    return sizeof(long long) * (size_t)(steps < most ? steps : most);
 }
 
-// int64 scan with caller-provided status scratch (scan_i64_scratch_bytes(n))
-// and a 4-byte tile counter; both are reset here on the stream.
+// int64 scan with caller-provided scratch (scan_i64_scratch_bytes(n)).
 int scan_i64_launch_with(const long long* in, long long* out, int64_t n, long long init, bool reverse,
-                         bool inclusive, void* status_scratch, unsigned* tile_counter, cudaStream_t stream) {
+                         bool inclusive, void* scratch, cudaStream_t stream) {
     if (n == 0) return HYD_CUDA_OK;
-    Device* d = nullptr;
-    HYD_TRY(device(&d));
-    const int64_t ntiles = (n + kScanTile - 1) / kScanTile;
-    ScanStatus st;
-    st.word = reinterpret_cast<TileWord*>((reinterpret_cast<uintptr_t>(status_scratch) + 15) & ~(uintptr_t)15);
-    st.tile_counter = tile_counter;
-    HYD_CUDA_TRY(cudaMemsetAsync(st.word, 0, sizeof(TileWord) * (size_t)ntiles, stream));
-    HYD_CUDA_TRY(cudaMemsetAsync(st.tile_counter, 0, 4, stream));
-    scan_i64_lookback_kernel<<<(unsigned)ntiles, kScanT, 0, stream>>>(in, out, n, init, reverse, inclusive, st,
-                                                                       d->d_err);
-    return launch_check("scan_i64");
+    return scan_ranges_launch<long long>(in, out, n, init, reverse, inclusive, scratch, stream, "scan_i64");
 }
 
 // Same, with scratch from the stream's workspace.
 int scan_i64_launch(const long long* in, long long* out, int64_t n, long long init, bool reverse,
                     bool inclusive, cudaStream_t stream) {
     if (n == 0) return HYD_CUDA_OK;
-    unsigned* counters = nullptr;
     void* scratch = nullptr;
-    HYD_TRY(workspace(stream, scan_i64_scratch_bytes(n), &counters, &scratch));
-    return scan_i64_launch_with(in, out, n, init, reverse, inclusive, scratch, counters + 8, stream);
+    HYD_TRY(workspace(stream, scan_i64_scratch_bytes(n), nullptr, &scratch));
+    return scan_i64_launch_with(in, out, n, init, reverse, inclusive, scratch, stream);
 }
 }  // namespace hyd
 
@@ -445,9 +507,14 @@ extern "C" int hyd_cuda_scan_f64(const double* in, double* out, int64_t n, doubl
     HYD_CHECK_ARG(ntiles <= 0x7fffffffLL, "scan_f64: too long");
     Device* d = nullptr;
     HYD_TRY(device(&d));
+    if (n <= kScanRangesF64) {
+        void* scratch = nullptr;
+        HYD_TRY(workspace(s, scan_i64_scratch_bytes(n), nullptr, &scratch));
+        return scan_ranges_launch<double>(in, out, n, init, reverse != 0, inclusive != 0, scratch, s, "scan_f64");
+    }
     FoldStatus<double> st, bst;
     HYD_TRY(fold_status(s, ntiles, &st, &bst));
     scan_fold_kernel<double><<<(unsigned)ntiles, kScanT, 0, s>>>(in, out, n, init, reverse != 0, inclusive != 0, st,
-                                                                 bst, d->d_err);
+                                                                 bst, d->sm_count * kScanCtasPerSm, d->d_err);
     return launch_check("scan_f64");
 }

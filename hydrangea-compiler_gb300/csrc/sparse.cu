@@ -42,7 +42,7 @@ int scan_i64_launch(const long long* in, long long* out, int64_t n, long long in
                     bool inclusive, cudaStream_t stream);
 size_t scan_i64_scratch_bytes(int64_t n);
 int scan_i64_launch_with(const long long* in, long long* out, int64_t n, long long init, bool reverse,
-                         bool inclusive, void* status_scratch, unsigned* tile_counter, cudaStream_t stream);
+                         bool inclusive, void* scratch, cudaStream_t stream);
 
 // ---------------------------------------------------------------- coo dedup
 // One pass over the entries: a tile of 2048 finds its heads (entries that
@@ -744,9 +744,8 @@ extern "C" int hyd_cuda_csr_from_sorted_coo_i64(int64_t nrows, int64_t nnz, cons
     const int64_t m = nrows + 1;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
     const size_t count_bytes = al((size_t)m * 8);
-    unsigned* counters = nullptr;
     void* scratch = nullptr;
-    HYD_TRY(workspace(s, count_bytes + al(scan_i64_scratch_bytes(m)), &counters, &scratch));
+    HYD_TRY(workspace(s, count_bytes + al(scan_i64_scratch_bytes(m)), nullptr, &scratch));
     unsigned long long* counts = static_cast<unsigned long long*>(scratch);
     HYD_CUDA_TRY(cudaMemsetAsync(counts, 0, count_bytes, s));
     if (nnz > 0) {
@@ -758,7 +757,7 @@ extern "C" int hyd_cuda_csr_from_sorted_coo_i64(int64_t nrows, int64_t nnz, cons
         HYD_TRY(launch_check("csr_count"));
     }
     return scan_i64_launch_with((const long long*)counts, (long long*)row_ptr, m, 0, false, false,
-                                static_cast<unsigned char*>(scratch) + count_bytes, counters + 8, s);
+                                static_cast<unsigned char*>(scratch) + count_bytes, s);
 }
 
 extern "C" int hyd_cuda_spmv_csr_f64(int64_t nrows, int64_t ncols, const int64_t* row_ptr, const int64_t* col_idx,
