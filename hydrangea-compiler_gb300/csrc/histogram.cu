@@ -70,8 +70,9 @@ struct WeightedHistSourceT {
     // Routes of four elements; true when all four are in [0, bins).  For a
     // power of two the only way out of range is a negative x, so one test of the
     // four sign bits replaces four per-element checks.
-    __device__ __forceinline__ bool four(int64_t v, long long bins, long long bin[4], u64 val[4]) const {
-        u64x4 q = ldg_stream_u64x4(data + 4 * v);
+    typedef u64x4 Raw;
+    __device__ __forceinline__ Raw load4(int64_t v) const { return ldg_stream_u64x4(data + 4 * v); }
+    __device__ __forceinline__ bool four(const Raw& q, long long bins, long long bin[4], u64 val[4]) const {
         const u64 x[4] = {q.x, q.y, q.z, q.w};
         if (kPow2) {
 #pragma unroll
@@ -83,6 +84,14 @@ struct WeightedHistSourceT {
 #pragma unroll
             for (int k = 0; k < 4; ++k) route(x[k], bin[k], val[k]);
             return false;
+        }
+        if (((x[0] | x[1] | x[2] | x[3]) >> 31) == 0) {  // small values: 32-bit remainders, always in range
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                bin[k] = (long long)dm.rem31((unsigned)x[k]);
+                val[k] = (u64)(unsigned)x[k] * (unsigned)x[k];
+            }
+            return true;
         }
         bool ok = true;
 #pragma unroll
@@ -106,9 +115,12 @@ struct ScatterI64Source {
         bin = idx[i];
         val = (u64)vals[i];
     }
-    __device__ __forceinline__ bool four(int64_t v, long long bins, long long bin[4], u64 val[4]) const {
-        u64x4 a = ldg_stream_u64x4(idx + 4 * v);
-        u64x4 b = ldg_stream_u64x4(vals + 4 * v);
+    struct Raw { u64x4 a, b; };
+    __device__ __forceinline__ Raw load4(int64_t v) const {
+        return Raw{ldg_stream_u64x4(idx + 4 * v), ldg_stream_u64x4(vals + 4 * v)};
+    }
+    __device__ __forceinline__ bool four(const Raw& q, long long bins, long long bin[4], u64 val[4]) const {
+        const u64x4 &a = q.a, &b = q.b;
         bin[0] = (long long)a.x; bin[1] = (long long)a.y; bin[2] = (long long)a.z; bin[3] = (long long)a.w;
         val[0] = b.x; val[1] = b.y; val[2] = b.z; val[3] = b.w;
         return ((a.x | a.y | a.z | a.w) < (u64)bins) ||
@@ -136,10 +148,12 @@ struct GuardedScatterI64Source {
         bin = on ? idx[i] : 0LL;
         val = on ? (u64)vals[i] : 0ULL;
     }
-    __device__ __forceinline__ bool four(int64_t v, long long bins, long long bin[4], u64 val[4]) const {
-        const u64x4 g = ldg_stream_u64x4(guard + 4 * v);
-        const u64x4 a = ldg_stream_u64x4(idx + 4 * v);
-        const u64x4 b = ldg_stream_u64x4(vals + 4 * v);
+    struct Raw { u64x4 g, a, b; };
+    __device__ __forceinline__ Raw load4(int64_t v) const {
+        return Raw{ldg_stream_u64x4(guard + 4 * v), ldg_stream_u64x4(idx + 4 * v), ldg_stream_u64x4(vals + 4 * v)};
+    }
+    __device__ __forceinline__ bool four(const Raw& q, long long bins, long long bin[4], u64 val[4]) const {
+        const u64x4 &g = q.g, &a = q.a, &b = q.b;
         bin[0] = g.x ? (long long)a.x : 0LL; bin[1] = g.y ? (long long)a.y : 0LL;
         bin[2] = g.z ? (long long)a.z : 0LL; bin[3] = g.w ? (long long)a.w : 0LL;
         val[0] = g.x ? b.x : 0ULL; val[1] = g.y ? b.y : 0ULL; val[2] = g.z ? b.z : 0ULL; val[3] = g.w ? b.w : 0ULL;
@@ -168,8 +182,9 @@ __device__ __forceinline__ void for_each_element(const Src& src, int64_t n, bool
         for (; v + S < nv; v += 2 * S) {
             long long b0[4], b1[4];
             u64 v0[4], v1[4];
-            const bool ok0 = src.four(v, bins, b0, v0);
-            const bool ok1 = src.four(v + S, bins, b1, v1);
+            const typename Src::Raw q0 = src.load4(v), q1 = src.load4(v + S);  // both before the first branch
+            const bool ok0 = src.four(q0, bins, b0, v0);
+            const bool ok1 = src.four(q1, bins, b1, v1);
             if (ok0 && ok1) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) fast(b0[k], v0[k]);
@@ -185,7 +200,7 @@ __device__ __forceinline__ void for_each_element(const Src& src, int64_t n, bool
         if (v < nv) {
             long long b0[4];
             u64 v0[4];
-            src.four(v, bins, b0, v0);
+            src.four(src.load4(v), bins, b0, v0);
 #pragma unroll
             for (int k = 0; k < 4; ++k) checked(b0[k], v0[k]);
         }

@@ -141,23 +141,43 @@ __device__ __forceinline__ void stg_f64x4(double* p, f64x4 v) {
 
 __device__ __forceinline__ void raise_error(unsigned* err, unsigned bit) { atomicOr(err, bit); }
 
-// Divide/remainder by a runtime-invariant positive int64 divisor with C's
-// truncating semantics.  Power-of-two divisors use shifts/masks; others fall
-// back to the hardware-emulated 64-bit divide.
+// Remainder by a runtime-invariant positive int64 divisor d <= 2^31 with C's
+// truncating semantics.  Power-of-two divisors use a mask; others a multiply by
+// the rounded-up reciprocal (Granlund and Montgomery, "Division by invariant
+// integers using multiplication", 1994): with 2^(l-1) < d < 2^l and
+// m = floor(2^(63+l) / d) + 1 (below 2^64), floor(u / d) is the high word of
+// m * u shifted right by l - 1 for every u <= 2^63; and the same with 31 for 63
+// in 32 bits.  (The compiler's 64-bit division is a loop of about a hundred
+// instructions: it, not memory, bound the histogram over 1000 bins.)
 struct DivMod64 {
     long long d;
     unsigned long long mask;
+    unsigned long long m64;
+    unsigned m32;
     int shift;  // >= 0 when d is a power of two
+    int l1;     // l - 1
     __host__ void init(long long dv) {
         d = dv;
         shift = -1;
         mask = 0;
+        m64 = 0;
+        m32 = 0;
+        l1 = 0;
         if (dv > 0 && (dv & (dv - 1)) == 0) {
             int s = 0;
             while ((1LL << s) != dv) ++s;
             shift = s;
             mask = (unsigned long long)dv - 1ULL;
+        } else if (dv > 0) {
+            while ((1LL << (l1 + 1)) < dv) ++l1;
+            const unsigned __int128 one = 1;
+            m64 = (unsigned long long)((one << (64 + l1)) / (unsigned long long)dv + 1);
+            m32 = (unsigned)((one << (32 + l1)) / (unsigned long long)dv + 1);
         }
+    }
+    // 0 <= x < 2^31, d no power of two
+    __device__ __forceinline__ unsigned rem31(unsigned x) const {
+        return x - (__umulhi(x, m32) >> l1) * (unsigned)d;
     }
     __device__ __forceinline__ long long rem(long long x) const {
         if (shift >= 0) {
@@ -165,7 +185,9 @@ struct DivMod64 {
             // C: the remainder takes the sign of the dividend.
             return -(long long)((0ULL - (unsigned long long)x) & mask);
         }
-        return x % d;
+        const unsigned long long u = x < 0 ? 0ULL - (unsigned long long)x : (unsigned long long)x;
+        const long long r = (long long)(u - (__umul64hi(u, m64) >> l1) * (unsigned long long)d);
+        return x < 0 ? -r : r;
     }
 };
 
