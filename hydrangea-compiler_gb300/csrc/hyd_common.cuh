@@ -185,6 +185,7 @@ struct DivMod64 {
             // C: the remainder takes the sign of the dividend.
             return -(long long)((0ULL - (unsigned long long)x) & mask);
         }
+        if (((unsigned long long)x >> 31) == 0) return rem31((unsigned)x);
         const unsigned long long u = x < 0 ? 0ULL - (unsigned long long)x : (unsigned long long)x;
         const long long r = (long long)(u - (__umul64hi(u, m64) >> l1) * (unsigned long long)d);
         return x < 0 ? -r : r;
