@@ -8,8 +8,9 @@
 // Here the generated element body -- C statements over the inputs' elements
 // x0..x7 and the index i that assign `v` -- is compiled once per body and
 // device with NVRTC into a kernel that:
-//   * walks the elements as a grid-stride loop over pairs, with 128-bit
-//     (double2) loads and stores when every pointer is 16-byte aligned;
+//   * walks the elements as a grid-stride loop over pairs of 32-byte vectors
+//     when every pointer is 32-byte aligned, of 16-byte ones when all are
+//     16-byte aligned;
 //   * evaluates the body with IEEE round-to-nearest operations and no
 //     contraction (--fmad=false), so each element equals the C backend's;
 //   * optionally writes the elements and/or reduces them with (+): per-thread
@@ -20,6 +21,7 @@
 #include <dlfcn.h>
 #include <nvrtc.h>
 
+#include <climits>
 #include <cstdlib>
 #include <map>
 #include <mutex>
@@ -74,11 +76,14 @@ constexpr int kMapThreads = 256;
 // Kernel source for `body` over `nin` inputs of element type T ("double" or
 // "long long").  int64 sums wrap (accumulated as unsigned), as the C backend's
 // int64 arithmetic does on every target it runs on.
-static std::string map_source(const std::string& body, int nin, bool i64) {
+static std::string map_source(const std::string& body, int nin, bool i64, bool with_sum) {
     const std::string T = i64 ? "long long" : "double";
     const std::string T2 = i64 ? "longlong2" : "double2";
     const std::string A = i64 ? "unsigned long long" : "double";  // accumulator
     const std::string zero = i64 ? "0LL" : "0.0";
+    // without a reduction no element is added up: FP64 additions bind these
+    // kernels before memory does (see map_launch)
+    auto add = [&](const std::string& v) { return with_sum ? "acc += (" + A + ")" + v + ";" : std::string(";"); };
     std::string s;
     s += "__device__ __forceinline__ " + T + " hyd_elem(long long i";
     for (int k = 0; k < kMapMaxInputs; ++k) s += ", " + T + " x" + std::to_string(k);
@@ -94,9 +99,9 @@ static std::string map_source(const std::string& body, int nin, bool i64) {
          "  const long long nt = (long long)gridDim.x * blockDim.x;\n"
          "  if (vec == 2) {\n"
          "    const long long nq = n >> 2;\n"
-         "    long long q = t;\n"
+         "    long long q = 2LL * blockIdx.x * blockDim.x + threadIdx.x;\n"
          "    for (; q < nq; q += 2 * nt) {\n"
-         "      const bool two = q + nt < nq;\n";
+         "      const bool two = q + 256 < nq;\n";
     // 32-byte vectors, two per lane per step (8 elements), all loads first
     const std::string LD = i64 ? "ld.global.nc.L1::no_allocate.v4.u64" : "ld.global.nc.L1::no_allocate.v4.f64";
     const std::string ST = i64 ? "st.global.v4.u64" : "st.global.v4.f64";
@@ -111,7 +116,7 @@ static std::string map_source(const std::string& body, int nin, bool i64) {
                      " {%0,%1,%2,%3}, [%4];\" : \"=" + RC + "\"(a" + ks + "[" + std::to_string(4 * h) + "]), \"=" + RC +
                      "\"(a" + ks + "[" + std::to_string(4 * h + 1) + "]), \"=" + RC + "\"(a" + ks + "[" +
                      std::to_string(4 * h + 2) + "]), \"=" + RC + "\"(a" + ks + "[" + std::to_string(4 * h + 3) +
-                     "]) : \"l\"(p" + ks + " + 4 * (q + " + hs + " * nt)));\n";
+                     "]) : \"l\"(p" + ks + " + 4 * (q + " + hs + " * 256)));\n";
                 if (h) s += "      else { a" + ks + "[4] = a" + ks + "[5] = a" + ks + "[6] = a" + ks + "[7] = " + zero + "; }\n";
             }
         } else {
@@ -120,20 +125,20 @@ static std::string map_source(const std::string& body, int nin, bool i64) {
     }
     s += "      " + T + " w[8];\n"
          "      #pragma unroll\n"
-         "      for (int u = 0; u < 8; ++u) w[u] = hyd_elem(4 * (q + (u >> 2) * nt) + (u & 3)";
+         "      for (int u = 0; u < 8; ++u) w[u] = hyd_elem(4 * (q + (u >> 2) * 256) + (u & 3)";
     for (int k = 0; k < kMapMaxInputs; ++k) s += ", a" + std::to_string(k) + "[u]";
     s += ");\n"
          "      if (out) {\n"
          "        asm volatile(\"" + ST + " [%0], {%1,%2,%3,%4};\" :: \"l\"(out + 4 * q), \"" + RC + "\"(w[0]), \"" +
          RC + "\"(w[1]), \"" + RC + "\"(w[2]), \"" + RC + "\"(w[3]) : \"memory\");\n"
-         "        if (two) asm volatile(\"" + ST + " [%0], {%1,%2,%3,%4};\" :: \"l\"(out + 4 * (q + nt)), \"" + RC +
+         "        if (two) asm volatile(\"" + ST + " [%0], {%1,%2,%3,%4};\" :: \"l\"(out + 4 * (q + 256)), \"" + RC +
          "\"(w[4]), \"" + RC + "\"(w[5]), \"" + RC + "\"(w[6]), \"" + RC + "\"(w[7]) : \"memory\");\n"
          "      }\n"
          "      #pragma unroll\n"
-         "      for (int u = 0; u < 4; ++u) acc += (" + A + ")w[u];\n"
+         "      for (int u = 0; u < 4; ++u) " + add("w[u]") + "\n"
          "      if (two) {\n"
          "        #pragma unroll\n"
-         "        for (int u = 4; u < 8; ++u) acc += (" + A + ")w[u];\n"
+         "        for (int u = 4; u < 8; ++u) " + add("w[u]") + "\n"
          "      }\n"
          "    }\n"
          "    for (long long i = 4 * nq + t; i < n; i += nt) {\n"
@@ -141,7 +146,7 @@ static std::string map_source(const std::string& body, int nin, bool i64) {
     for (int k = 0; k < kMapMaxInputs; ++k) s += k < nin ? ", p" + std::to_string(k) + "[i]" : ", " + zero;
     s += ");\n"
          "      if (out) out[i] = v;\n"
-         "      acc += (" + A + ")v;\n"
+         "      " + add("v") + "\n"
          "    }\n"
          "  } else if (vec) {\n"
          "    const long long np = n >> 1;\n"
@@ -158,8 +163,7 @@ static std::string map_source(const std::string& body, int nin, bool i64) {
     for (int k = 0; k < kMapMaxInputs; ++k) s += ", a" + std::to_string(k) + ".y";
     s += ");\n"
          "      if (out) { " + T2 + " w; w.x = v0; w.y = v1; ((" + T2 + "*)out)[q] = w; }\n"
-         "      acc += (" + A + ")v0;\n"
-         "      acc += (" + A + ")v1;\n"
+         "      " + add("v0") + add("v1") + "\n"
          "    }\n"
          "    if (t == 0 && (n & 1)) {\n"
          "      const long long i = n - 1;\n"
@@ -167,7 +171,7 @@ static std::string map_source(const std::string& body, int nin, bool i64) {
     for (int k = 0; k < kMapMaxInputs; ++k) s += k < nin ? ", p" + std::to_string(k) + "[i]" : ", " + zero;
     s += ");\n"
          "      if (out) out[i] = v;\n"
-         "      acc += (" + A + ")v;\n"
+         "      " + add("v") + "\n"
          "    }\n"
          "  } else {\n"
          "    for (long long i = t; i < n; i += nt) {\n"
@@ -175,7 +179,7 @@ static std::string map_source(const std::string& body, int nin, bool i64) {
     for (int k = 0; k < kMapMaxInputs; ++k) s += k < nin ? ", p" + std::to_string(k) + "[i]" : ", " + zero;
     s += ");\n"
          "      if (out) out[i] = v;\n"
-         "      acc += (" + A + ")v;\n"
+         "      " + add("v") + "\n"
          "    }\n"
          "  }\n"
          "  if (sum == 0) return;\n"
@@ -208,11 +212,11 @@ struct MapKernel {
     cudaLibrary_t lib = nullptr;
     cudaKernel_t kern = nullptr;
 };
-static std::map<std::tuple<int, int, bool, std::string>, MapKernel> g_map_kernels;
+static std::map<std::tuple<int, int, bool, bool, std::string>, MapKernel> g_map_kernels;
 
-static int compile_map(Device* d, const std::string& body, int nin, bool i64, MapKernel* out) {
+static int compile_map(Device* d, const std::string& body, int nin, bool i64, bool with_sum, MapKernel* out) {
     std::lock_guard<std::mutex> lock(g_jit_mu);
-    auto key = std::make_tuple(d->id, nin, i64, body);
+    auto key = std::make_tuple(d->id, nin, i64, with_sum, body);
     auto it = g_map_kernels.find(key);
     if (it != g_map_kernels.end()) {
         *out = it->second;
@@ -222,7 +226,7 @@ static int compile_map(Device* d, const std::string& body, int nin, bool i64, Ma
     int major = 0, minor = 0;
     HYD_CUDA_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, d->id));
     HYD_CUDA_TRY(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, d->id));
-    const std::string src = map_source(body, nin, i64);
+    const std::string src = map_source(body, nin, i64, with_sum);
     nvrtcProgram prog = nullptr;
     if (g_nvrtc.create(&prog, src.c_str(), "hyd_map.cu", 0, nullptr, nullptr) != NVRTC_SUCCESS)
         return set_error(HYD_CUDA_ERR_CUDA, "map_f64: nvrtcCreateProgram failed");
@@ -277,7 +281,7 @@ static int map_launch(const char* body, const T* const* inputs, int ninputs, int
     HYD_TRY(device(&d));
     MapKernel mk;
     // compile errors surface even for n == 0
-    HYD_TRY(compile_map(d, body, ninputs, std::is_integral<T>::value, &mk));
+    HYD_TRY(compile_map(d, body, ninputs, std::is_integral<T>::value, sum != nullptr, &mk));
     if (n == 0) {
         if (sum) HYD_CUDA_TRY(cudaMemsetAsync(sum, 0, sizeof(T), s));
         return HYD_CUDA_OK;
@@ -295,13 +299,28 @@ static int map_launch(const char* body, const T* const* inputs, int ninputs, int
     }
     const int64_t pairs = (n + 1) / 2;
     int64_t grid = (pairs + kMapThreads - 1) / kMapThreads;
-    const int64_t cap = (int64_t)d->sm_count * 8;
-    if (grid > cap) grid = cap;
-    unsigned* counters = nullptr;
-    void* scratch = nullptr;
-    HYD_TRY(workspace(s, (size_t)grid * sizeof(T), &counters, &scratch));
-    unsigned* counter = counters + 200;  // reset by the kernel's last block
-    void* partials = scratch;
+    if (!sum && (vec || vec32) && ninputs <= 4) {
+        // no partials: a block per 512 vectors (two per thread), none of them
+        // staying on for more; x0 * x1 + x2 over 2^27 583 us, against 607 with
+        // 8 blocks per SM that stay.  (It took 784 with the additions of a sum
+        // nobody asked for: three FP64 operations per element, 762 us of that
+        // pipe.)  Scalar elements and many inputs, whose few loads or many
+        // registers leave less in flight, keep the 8 blocks per SM: 607
+        // against 671 us, and 2045 against 2364 with eight inputs.
+        const int64_t per = vec32 ? 8 : 2;
+        grid = (n + kMapThreads * per - 1) / (kMapThreads * per);
+        if (grid > INT_MAX) grid = INT_MAX;
+    } else {
+        const int64_t cap = (int64_t)d->sm_count * 8;
+        if (grid > cap) grid = cap;
+    }
+    unsigned* counter = nullptr;
+    void* partials = nullptr;
+    if (sum) {
+        unsigned* counters = nullptr;
+        HYD_TRY(workspace(s, (size_t)grid * sizeof(T), &counters, &partials));
+        counter = counters + 200;  // reset by the kernel's last block
+    }
     long long nn = n;
     int v = vec32 ? 2 : (vec ? 1 : 0);
     void* args[kMapMaxInputs + 6];
