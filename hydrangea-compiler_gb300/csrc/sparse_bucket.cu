@@ -16,11 +16,13 @@
 //             region as a 32-bit key (row_in_bucket << 24 | col) plus its value
 //             (the tile's values are prefetched into shared memory with
 //             cp.async while the ranks and reservations are computed);
-//  4. bucket  one warp per bucket (at most 2048 entries, ncols <= 2^18): a
-//             stable LSD radix sort of the packed (row, col) keys in shared
-//             memory, the CSR columns/values written in sorted order and the
-//             row pointers from the row changes.  Larger buckets go to an
-//             overflow list sorted by a block-wide bitonic network;
+//  4. bucket  one block per bucket (at most 2048 entries, ncols <= 2^18): a
+//             counting pass into as many bins as entries, in (row, col) order,
+//             and comparisons inside the bins; the CSR columns/values written
+//             in sorted order and the row pointers from the row counts.
+//             Buckets with clustered columns are sorted by a warp each, with a
+//             stable LSD radix sort of the packed keys; larger buckets by a
+//             block-wide bitonic network;
 //  5. spmv    one warp per 256-row chunk of an instance: the rows are ordered
 //             by length in shared memory and each lane sums one row's fma
 //             chain in column order, 32 rows of similar length at a time.
@@ -307,10 +309,11 @@ __device__ __forceinline__ void bk_order_equal_keys(const unsigned* key, IdxT* p
     }
 }
 
-// One warp per bucket: a warp sorts its own bucket with no block barrier, so
-// fifteen independent buckets are in flight per SM.  (A CTA per ~800-entry
-// bucket pays its fixed work -- zeroing and scanning a counter set per warp,
-// five block barriers per radix pass -- once per bucket.)
+// The radix form, for buckets with clustered columns.  One warp per bucket: a
+// warp sorts its own bucket with no block barrier, so fifteen independent
+// buckets are in flight per SM.  (A CTA per ~800-entry bucket pays its fixed
+// work -- zeroing and scanning a counter set per warp, five block barriers per
+// radix pass -- once per bucket.)
 //  * key24 = row_in_bucket << cbits | col, kept to its 6 + cbits <= 24 bits,
 //    sorted by stable LSD passes of 8 bits (at most three);
 //  * the digit counts of every pass are taken in one sweep when the keys are
@@ -328,20 +331,19 @@ __device__ __forceinline__ void bk_order_equal_keys(const unsigned* key, IdxT* p
 //    then put in COO order.
 // Row starts come from the masked keys, which are sorted on every bit they
 // have whatever the records hold, so every row range stays inside [0, E].
-// The pipeline runs it with room for 1536 entries per warp (fifteen warps per
-// SM; 0.5% of the workload's buckets are larger).  Buckets above kCap, or of
-// instances with more than 2^18
-// columns, go to `overflow` (the block-wide kernel below).
+// It has room for 1536 entries per warp (fifteen warps per SM).
+constexpr int kBkRadixCap = 1536;    // entries a bucket of the radix form may have
 constexpr int kBkWarpIdxBits = 11;   // entry index bits: buckets of at most 2048 entries
 constexpr unsigned kBkWarpIdxMask = (1u << kBkWarpIdxBits) - 1u;
 constexpr int kBkWarpMaxCbits = 24 - kBkShift;
-constexpr int kBkWarpPerSm = 3;  // resident CTAs per SM
+constexpr int kBkWarpPerSm = 3;  // resident CTAs of the radix form per SM
+constexpr int kBkWarps = 5;
 // per warp (32-bit words): two key buffers, packed digit counts of three
 // passes, the running digit bases (later the row starts)
 template <int kCap>
 __host__ __device__ constexpr int bk_warp_words() { return 2 * kCap + 3 * 128 + 256; }
-template <int kCap, int kWarps>
-constexpr size_t bk_warp_smem() { return (size_t)kWarps * bk_warp_words<kCap>() * 4; }
+template <int kCap>
+constexpr size_t bk_warp_smem() { return (size_t)kBkWarps * bk_warp_words<kCap>() * 4; }
 
 // The sort key of a record: row_in_bucket << cbits | col, kept to its 6 + cbits
 // bits (which change nothing for a valid entry, and keep every key's row
@@ -381,20 +383,275 @@ __device__ __forceinline__ void bk_rank_pass(const unsigned* src, unsigned* dst,
     }
 }
 
-template <int kCap, int kWarps>
-__global__ void __launch_bounds__(kWarps * 32, kBkWarpPerSm) bk_bucket_warp_kernel(
+// The bucket sort of the 512-instance batch (2.9e8 entries): 5.22 + 0.21 ms with
+// the radix form for every bucket and the block-wide kernel, 1.77 + 0.70 + 0.04
+// ms now.  Buckets whose columns are not clustered take no rank chain: one
+// counting pass puts every entry into a bin, the bins being in (row, column)
+// order, and the few entries that share a bin are ordered by comparing them.
+//  * row r owns as many bins as it has entries, its columns spread evenly over
+//    them: bin = start + (col - first) * L / width, in float, which is monotone
+//    in col.  First the width is the whole row (scattered columns: a bin holds
+//    one entry on average); when a bin gets more entries than a rank can count, the
+//    row's own smallest and largest column (bands);
+//  * an atomic gives each entry its (arbitrary) rank in its bin; a scan of the
+//    bin counts gives the bins' starts;
+//  * an entry's final place is its bin's start plus the number of entries in
+//    the bin that sort before it (equal keys: by COO position).
+// The bucket's records come to shared memory in one bulk copy, and four warps
+// share the bucket.  The L1 pipe bounds the kernel (about 55 wavefronts per 32
+// entries); with a warp per bucket shared memory left 14 warps per SM and the
+// phases' latencies bound it, and reading the values from global memory in
+// sorted order, a line per lane, was a third of the pipe's work.  A bucket
+// whose bins overflow both ways goes to `clustered` (the radix form below), a
+// bucket above kCap, or of an instance with more than 2^18 columns, to
+// `overflow`.  The kernel runs twice: over all buckets with room for 1024
+// entries (nine per SM), and over the larger ones with room for 2048.
+template <int kCap>
+constexpr int bk_place_threads() { return kCap <= 1024 ? 128 : 256; }
+template <int kCap>
+constexpr int bk_place_per_sm() { return kCap <= 1024 ? 9 : 4; }
+// A packed word holds an 18-bit column, a bin or entry number and, in the bits
+// that are left, a rank in a bin: bins of at most 16 entries, or 8.
+template <int kCap>
+constexpr int bk_place_idx_bits() { return kCap <= 1024 ? 10 : 11; }
+constexpr int kBkColBits = 24 - kBkShift;
+// 32-bit words: the records | entries by bin | bin counts, later starts (16
+// bits) | row starts and lengths | row minima | row maxima, later scales
+template <int kCap>
+__host__ __device__ constexpr int bk_place_words() { return 4 * kCap + kCap + 4 + kCap / 2 + 3 * kBkRows; }
+template <int kCap>
+constexpr size_t bk_place_smem() { return (size_t)bk_place_words<kCap>() * 4; }
+
+// kList: the items are a list that another kernel filled (its length in device
+// memory); otherwise every bucket of the batch, in order.
+template <int kCap, bool kList>
+__global__ void __launch_bounds__(bk_place_threads<kCap>(), bk_place_per_sm<kCap>()) bk_bucket_place_kernel(
     const BkInst* __restrict__ inst, const BkItem* __restrict__ items, unsigned nitems_host,
     const unsigned* nitems_dev, unsigned* cursor,
     const long long* __restrict__ bstart, const unsigned* __restrict__ bcount, const uint4* __restrict__ rec_in,
-    BkItem* __restrict__ overflow, unsigned* overflow_count, unsigned* err) {
+    BkItem* __restrict__ overflow, unsigned* overflow_count, BkItem* __restrict__ clustered,
+    unsigned* clustered_count, unsigned* err) {
+    extern __shared__ __align__(128) unsigned bkw_smem[];
+    __shared__ __align__(8) unsigned long long sh_bar;
+    __shared__ unsigned sh_next, sh_part[bk_place_threads<kCap>() / 32];
+    __shared__ BkItem sh_item;    // the next bucket, ...
+    __shared__ int sh_entries;    // ... its entries
+    __shared__ long long sh_slot;  // and its first slot: read ahead by thread 0
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int T = bk_place_threads<kCap>(), kIdx = bk_place_idx_bits<kCap>();
+    constexpr int kRankAt = kIdx + kBkColBits, kRankBits = 32 - kRankAt;
+    constexpr unsigned kBinMax = 1u << kRankBits, kIdxMask = (1u << kIdx) - 1u;
+    constexpr unsigned kColMask = (1u << kBkColBits) - 1u, kRankMask = (kBinMax - 1u) << kRankAt;
+    static_assert(kCap <= (1 << kIdx), "entry and bin numbers must fit their field");
+    uint4* const rec = reinterpret_cast<uint4*>(bkw_smem);
+    unsigned* const ord = reinterpret_cast<unsigned*>(rec + kCap);  // rank << 29 | col << 11 | entry, by bin
+    unsigned* const cntw = ord + kCap + 4;                          // two 16-bit counts per word
+    const unsigned short* const start = reinterpret_cast<const unsigned short*>(cntw);
+    unsigned* const rowinfo = cntw + kCap / 2;  // start | length << 16
+    unsigned* const rowmin = rowinfo + kBkRows;
+    unsigned* const rowmax = rowmin + kBkRows;
+    const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh_bar);
+    const unsigned nitems = kList ? *(volatile const unsigned*)nitems_dev : nitems_host;
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    // thread 0: draws a bucket and reads what the block needs to start on it
+    auto draw = [&]() {
+        const unsigned nx = atomicAdd(cursor, 1u);
+        sh_next = nx;
+        if (nx >= nitems) return;
+        const BkItem nw = items[nx];
+        const long long gb = kList ? inst[nw.inst].bucket_base + nw.tile : (long long)nx;  // its number in the batch
+        const int nE = (int)bcount[gb];
+        const long long ns = bstart[gb];
+        sh_item = nw;
+        sh_entries = nE;
+        sh_slot = ns;
+        if (nE <= kCap) l2_prefetch(rec_in + ns, (int64_t)nE * 16);
+    };
+    if (tid == 0) draw();
+    unsigned parity = 0;
+    int last_inst = -1, skip = 0;
+    for (;;) {
+        __syncthreads();
+        const unsigned it = sh_next;
+        if (it >= nitems) break;
+        const BkItem w = sh_item;
+        const int E = sh_entries;
+        const long long s0 = sh_slot;
+        const BkInst& I = inst[w.inst];
+        const long long ncols = I.ncols;
+        // bits of the largest column: the smallest c with 2^c >= ncols
+        const int cbits = ncols > 1 ? 64 - __clzll((unsigned long long)(ncols - 1)) : 0;
+        const bool fits = E <= kCap && cbits <= kBkWarpMaxCbits;
+        // after a clustered bucket the next 31 that this block draws of its
+        // instance go the same way untried
+        if (w.inst != last_inst) skip = 0;
+        last_inst = w.inst;
+        const bool tried = skip == 0 || E > kBkRadixCap;
+        if (!tried) --skip;
+        const bool copied = E > 0 && fits && tried;
+        if (copied && tid == 0) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the last bucket's accesses are over
+            mbar_expect_tx(bar, (unsigned)E * 16u);
+            bulk_load_1d((unsigned)__cvta_generic_to_shared(rec), rec_in + s0, (unsigned)E * 16u, bar);
+        }
+        const unsigned cmask = (1u << (cbits & 31)) - 1u;
+        if (tid < kBkRows) rowinfo[tid] = 0u;
+        for (int i = tid; i < (E + 1) / 2 && i < kCap / 2; i += T) cntw[i] = 0u;
+        bool ok = true;
+        if (copied) {
+            ok = mbar_wait_bounded(bar, parity);
+            parity ^= 1u;
+        }
+        if (__syncthreads_or(!ok)) {
+            if (tid == 0) {
+                raise_error(err, ERRBIT_TIMEOUT);
+                mbar_wait_bounded(bar, parity ^ 1u);  // let the copy land before the memory is released
+            }
+            return;
+        }
+        if (tid == 0) draw();  // (everyone has read the current one)
+        bool big = !tried;
+        if (fits && tried) {
+#pragma unroll 4
+            for (int p = tid; p < E; p += T) atomicAdd(&rowinfo[bk_key24(rec[p].x, cbits) >> cbits], 1u);
+            __syncthreads();
+            if (warp == 0) {  // lane l owns rows 2l, 2l + 1
+                const unsigned n0 = rowinfo[2 * lane], n1 = rowinfo[2 * lane + 1];
+                unsigned incl = n0 + n1;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                const unsigned st = incl - n0 - n1;
+                rowinfo[2 * lane] = st | n0 << 16;
+                rowinfo[2 * lane + 1] = (st + n0) | n1 << 16;
+            }
+            __syncthreads();
+            const float whole = 1.0f / (float)(cmask + 1u);  // a power of two: exact
+            for (int tier = 0; tier < 2; ++tier) {
+                if (tier == 1) {  // the rows' own widths
+                    if (tid < kBkRows) {
+                        rowmin[tid] = 0xFFFFFFFFu;
+                        rowmax[tid] = 0u;
+                    }
+                    for (int i = tid; i < (E + 1) / 2; i += T) cntw[i] = 0u;
+                    __syncthreads();
+#pragma unroll 4
+                    for (int p = tid; p < E; p += T) {
+                        const unsigned k = bk_key24(rec[p].x, cbits), r = k >> cbits, c = k & cmask;
+                        atomicMin(&rowmin[r], c);
+                        atomicMax(&rowmax[r], c);
+                    }
+                    __syncthreads();
+                    if (tid < kBkRows) {
+                        const unsigned L = rowinfo[tid] >> 16;
+                        const float f = L ? (float)L / (float)(rowmax[tid] - rowmin[tid] + 1u) : 0.0f;
+                        rowmax[tid] = __float_as_uint(f);
+                    }
+                    __syncthreads();
+                }
+                big = false;
+#pragma unroll 4
+                for (int p = tid; p < E; p += T) {
+                    const unsigned k = bk_key24(rec[p].x, cbits), r = k >> cbits, c = k & cmask;
+                    const unsigned ri = rowinfo[r], L = ri >> 16;
+                    const float f = tier == 0 ? (float)c * ((float)L * whole)
+                                              : (float)(c - rowmin[r]) * __uint_as_float(rowmax[r]);
+                    const unsigned o = (unsigned)f;
+                    const unsigned bb = (ri & 0xFFFFu) + (o < L ? o : L - 1u);
+                    const unsigned sh = (bb & 1u) << 4;
+                    const unsigned rank = (atomicAdd(&cntw[bb >> 1], 1u << sh) >> sh) & 0xFFFFu;
+                    big |= rank >= kBinMax;
+                    ord[p] = rank << kRankAt | bb << kBkColBits | c;  // (the keys stay for a second try)
+                }
+                big = __syncthreads_or(big);
+                if (!big) break;
+            }
+            if (big) skip = 31;
+        }
+        if (!fits || big) {  // block-uniform
+            if (tid == 0) {
+                if (!fits || E > kBkRadixCap) overflow[atomicAdd(overflow_count, 1u)] = w;
+                else clustered[atomicAdd(clustered_count, 1u)] = w;
+            }
+            continue;
+        }
+        // counts -> starts; a thread owns an odd number of words (no bank conflicts)
+        const int words = (E + 1) >> 1, W = ((words + T - 1) / T) | 1;
+        const int w0 = tid * W < words ? tid * W : words, w1 = w0 + W < words ? w0 + W : words;
+        unsigned sum = 0;
+        for (int q = w0; q < w1; ++q) sum += cntw[q];  // both halves at once: at most kCap in all
+        sum = (sum & 0xFFFFu) + (sum >> 16);
+        unsigned incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) sh_part[warp] = incl;
+        // the packed words take the place of the keys
+#pragma unroll 4
+        for (int p = tid; p < E; p += T) rec[p].x = ord[p];
+        __syncthreads();
+        unsigned run = incl - sum;
+#pragma unroll
+        for (int u = 0; u < T / 32; ++u) run += u < warp ? sh_part[u] : 0u;
+        for (int q = w0; q < w1; ++q) {
+            const unsigned c = cntw[q], lo = run + (c & 0xFFFFu);
+            cntw[q] = run | lo << 16;
+            run = lo + (c >> 16);
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int p = tid; p < E; p += T) {
+            const unsigned v = rec[p].x, rank = v & kRankMask;
+            ord[start[(v >> kBkColBits) & kIdxMask] + (rank >> kRankAt)] = rank | (v & kColMask) << kIdx | (unsigned)p;
+        }
+        if (tid == 0) ord[E] = 0u;  // the end of the last bin
+        __syncthreads();
+        const long long e0 = s0 - I.scan_base;
+        int* const csr_cols = I.csr_cols + e0;
+        double* const csr_vals = I.csr_vals + e0;
+#pragma unroll 2
+        for (int q = tid; q < E; q += T) {
+            const unsigned me = ord[q];
+            const uint2 v = *reinterpret_cast<const uint2*>(&rec[me & kIdxMask].z);
+            // the bin is the slots from the one of rank 0 to before the next of rank 0
+            int k = q - (int)(me >> kRankAt), at = k;
+            unsigned other = ord[k];
+            do {
+                if ((other ^ me) << kRankBits >> (kRankBits + kIdx)) at += other << kRankBits < me << kRankBits;
+                else if (k != q)  // equal (row, col): COO order
+                    at += rec[other & kIdxMask].y < rec[me & kIdxMask].y;
+                other = ord[++k];
+            } while (other >> kRankAt);
+            csr_cols[at] = (int)((me >> kIdx) & kColMask);
+            csr_vals[at] = __hiloint2double((int)v.y, (int)v.x);
+        }
+        const long long r0 = (long long)w.tile << kBkShift;
+        const int nr = (int)((I.nrows - r0) < kBkRows ? (I.nrows - r0) : kBkRows);
+        for (int r = tid; r <= nr; r += T) {
+            if (r < nr) I.row_ptr[r0 + r] = e0 + (rowinfo[r] & 0xFFFFu);
+            else if (r0 + nr == I.nrows) I.row_ptr[I.nrows] = I.nnz;
+        }
+    }
+}
+
+template <int kCap>
+__global__ void __launch_bounds__(kBkWarps * 32, kBkWarpPerSm) bk_bucket_radix_kernel(
+    const BkInst* __restrict__ inst, const BkItem* __restrict__ items, const unsigned* nitems_dev, unsigned* cursor,
+    const long long* __restrict__ bstart, const unsigned* __restrict__ bcount, const uint4* __restrict__ rec_in) {
     extern __shared__ __align__(16) unsigned bkw_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     static_assert(kCap <= (1 << kBkWarpIdxBits), "entry indices must fit their field");
     unsigned* const a = bkw_smem + (size_t)warp * bk_warp_words<kCap>();
     unsigned* const b = a + kCap;
     unsigned* const hist = b + kCap;  // [3][128]
-    // the item count: given, or read from device memory (a list another kernel filled)
-    const unsigned nitems = nitems_dev ? *(volatile const unsigned*)nitems_dev : nitems_host;
+    const unsigned nitems = *(volatile const unsigned*)nitems_dev;  // a list another kernel filled
     unsigned* const base = hist + 3 * 128;  // [256]; row starts [65] after the sort
     unsigned lt;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
@@ -409,10 +666,6 @@ __global__ void __launch_bounds__(kWarps * 32, kBkWarpPerSm) bk_bucket_warp_kern
         const int E = (int)bcount[gb];
         // bits of the largest column: the smallest c with 2^c >= ncols
         const int cbits = I.ncols > 1 ? 64 - __clzll((unsigned long long)(I.ncols - 1)) : 0;
-        if (E > kCap || cbits > kBkWarpMaxCbits) {
-            if (lane == 0) overflow[atomicAdd(overflow_count, 1u)] = w;
-            continue;  // warp-uniform
-        }
         const long long s0 = bstart[gb];
         const long long e0 = s0 - I.scan_base;
         const long long r0 = (long long)w.tile << kBkShift;
@@ -793,7 +1046,7 @@ int batch_pipeline_bucketed(std::vector<BatchInst>& bi, const char* key, cudaStr
     const size_t cnt_b = al((size_t)nb_total * 4), wide_b = al((size_t)nb_total * 8);
     const size_t vals_b = al((size_t)entries * 8);
     void* buf = nullptr;
-    HYD_TRY(device_buffer(d, key, inst_b + tiles_b + 2 * bk_b + ch_b + 2 * cnt_b + 2 * wide_b + vals_b + vals_b + 256,
+    HYD_TRY(device_buffer(d, key, inst_b + tiles_b + 4 * bk_b + ch_b + 2 * cnt_b + 2 * wide_b + vals_b + vals_b + 256,
                           &buf));
     unsigned char* b = static_cast<unsigned char*>(buf);
     size_t off = 0;
@@ -810,7 +1063,9 @@ int batch_pipeline_bucketed(std::vector<BatchInst>& bi, const char* key, cudaStr
     long long* wide = reinterpret_cast<long long*>(take(wide_b));
     long long* bstart = reinterpret_cast<long long*>(take(wide_b));
     uint4* recs = reinterpret_cast<uint4*>(take(2 * vals_b));  // (key, COO position, value) per entry
-    BkItem* overflow = reinterpret_cast<BkItem*>(take(bk_b));  // buckets above 1536 entries
+    BkItem* overflow = reinterpret_cast<BkItem*>(take(bk_b));  // buckets for the block-wide kernel
+    BkItem* large = reinterpret_cast<BkItem*>(take(bk_b));      // buckets above 1024 entries
+    BkItem* clustered = reinterpret_cast<BkItem*>(take(bk_b));  // buckets for the radix form
     BkItem* d_chunks = reinterpret_cast<BkItem*>(take(ch_b));
     unsigned* cursors = reinterpret_cast<unsigned*>(take(256));
     // only the instance table crosses from the host; the work lists are
@@ -847,16 +1102,26 @@ int batch_pipeline_bucketed(std::vector<BatchInst>& bi, const char* key, cudaStr
                                                              bfill, recs, d->d_err);
         HYD_TRY(launch_check("bk_split"));
     }
-    // cursors: 2 the warp sort, 3 the block-wide kernel, 4 the overflow count.
-    // (A second warp run over the overflow, with room for 2048 entries, took
-    // 0.33 ms against the block-wide kernel's 0.21.)
+    // cursors: 2 the buckets of at most 1024 entries, 9 the larger ones (8: how
+    // many), 7 the radix form (6: how many), 3 the block-wide kernel (4: how many)
     {
-        auto k1 = bk_bucket_warp_kernel<1536, 5>;
+        auto k0 = bk_bucket_place_kernel<1024, false>;
+        HYD_TRY(configure_kernel((const void*)k0, d, false));
+        k0<<<(unsigned)(d->sm_count * bk_place_per_sm<1024>()), bk_place_threads<1024>(), bk_place_smem<1024>(), s>>>(
+            d_inst, d_bk, (unsigned)n_buckets, nullptr, cursors + 2, bstart, bcount, recs, large, cursors + 8,
+            clustered, cursors + 6, d->d_err);
+        HYD_TRY(launch_check("bk_bucket_place"));
+        auto k1 = bk_bucket_place_kernel<2048, true>;
         HYD_TRY(configure_kernel((const void*)k1, d, false));
-        k1<<<(unsigned)(d->sm_count * kBkWarpPerSm), 5 * 32, bk_warp_smem<1536, 5>(), s>>>(
-            d_inst, d_bk, (unsigned)n_buckets, nullptr, cursors + 2, bstart, bcount, recs, overflow, cursors + 4,
-            d->d_err);
-        HYD_TRY(launch_check("bk_bucket_warp"));
+        k1<<<(unsigned)(d->sm_count * bk_place_per_sm<2048>()), bk_place_threads<2048>(), bk_place_smem<2048>(), s>>>(
+            d_inst, large, 0u, cursors + 8, cursors + 9, bstart, bcount, recs, overflow, cursors + 4, clustered,
+            cursors + 6, d->d_err);
+        HYD_TRY(launch_check("bk_bucket_place"));
+        auto k2 = bk_bucket_radix_kernel<kBkRadixCap>;
+        HYD_TRY(configure_kernel((const void*)k2, d, false));
+        k2<<<(unsigned)(d->sm_count * kBkWarpPerSm), kBkWarps * 32, bk_warp_smem<kBkRadixCap>(), s>>>(
+            d_inst, clustered, cursors + 6, cursors + 7, bstart, bcount, recs);
+        HYD_TRY(launch_check("bk_bucket_radix"));
     }
     HYD_TRY(configure_kernel((const void*)bk_bucket_kernel, d, false));
     bk_bucket_kernel<<<grid, kBkThreads, kBkSmem, s>>>(d_inst, overflow, cursors + 4, cursors + 3, bstart, bcount,
