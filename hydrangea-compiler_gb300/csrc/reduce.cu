@@ -5,13 +5,14 @@
 // (CodegenC.hs:1328-1353; emitted `omp parallel for simd reduction(+:acc)`,
 // README.md:25-33) for the 1-D reduce_generate of Lowering.hs:771-804.
 //
-// Design (HBM-bound streaming reduction, one launch):
+// Design (HBM-bound streaming reduction, one launch; dot of 2^24 elements 48.9 ->
+// 46.4 us, of 10^6 14.0 -> 12.3 us since the combining steps take a quarter of
+// the FP64 instructions):
 //  * a fixed grid of 2 blocks x 512 threads per SM; thread t owns the 32-byte
-//    vectors t, t+S, t+2S, ... (S = total threads) and keeps two independent
-//    sets of four fp64 accumulators, so four 256-bit loads are in flight per
-//    thread and the DFMA latency chains stay short;
-//  * per-thread order, the xor-butterfly warp tree, the cross-warp tree and the
-//    final combine are all fixed, so a given (n, device) always produces the
+//    vectors t, t+S, t+2S, ... (S = total threads) in two chains of
+//    multiply-adds, with four 256-bit loads in flight per thread;
+//  * per-thread order, the halving through shared memory, the last warp's tree
+//    and the final combine are all fixed, so a given (n, device) always produces the
 //    same bits (the C backend's result instead depends on the thread count);
 //  * the block partials go to per-stream scratch; the last block to finish
 //    (completion counter) sums them in index order and resets the counter,
@@ -31,18 +32,23 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// Fixed-order block reduction; result valid in thread 0.
-__device__ __forceinline__ double block_sum(double v, double* sh) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    v = warp_sum(v);
-    if (lane == 0) sh[warp] = v;
-    __syncthreads();
-    double r = 0.0;
-    if (warp == 0) {
-        r = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0.0;
-        r = warp_sum(r);
+// Fixed-order block reduction; result valid in thread 0.  The sums are halved
+// through shared memory down to one warp: 20 FP64 instructions per block of 512
+// threads, where a shuffle tree in every warp takes 85, each holding the SM's
+// FP64 pipe for 19 cycles.
+template <int T>
+__device__ __forceinline__ double block_sum(double v, double* sh /*[T]*/) {
+    const int t = threadIdx.x;
+    sh[t] = v;
+#pragma unroll
+    for (int half = T / 2; half >= 32; half >>= 1) {
+        __syncthreads();
+        if (t < half) {
+            v += sh[t + half];
+            sh[t] = v;
+        }
     }
-    return r;
+    return t < 32 ? warp_sum(v) : 0.0;
 }
 
 // Last-block combine of the per-block partials, in index order.
@@ -61,7 +67,7 @@ __device__ __forceinline__ void finish_partials(double bsum, double* partials, u
     double v = 0.0;
     for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x)
         v += *((volatile double*)&partials[i]);
-    double total = block_sum(v, sh);
+    double total = block_sum<kRedThreads>(v, sh);
     if (threadIdx.x == 0) {
         *out = total;
         *counter = 0u;  // leave the counter ready for the next launch
@@ -72,67 +78,133 @@ template <bool kDot, bool kVec>
 __global__ void __launch_bounds__(kRedThreads, kRedBlocksPerSM)
     reduce_f64_kernel(const double* __restrict__ xs, const double* __restrict__ ys, int64_t n,
                       double* partials, unsigned* counter, double* out) {
-    __shared__ double sh[32];
+    __shared__ double sh[kRedThreads];
     const int64_t S = (int64_t)gridDim.x * blockDim.x;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    double b0 = 0.0, b1 = 0.0, b2 = 0.0, b3 = 0.0;
-    int64_t tail_start = 0;
+    double a = 0.0, b = 0.0;  // 32 warps per SM hide the chains' latency
     if (kVec) {
         const int64_t nv = n >> 2;  // 32-byte vectors
+        // the up to three elements after them: on their way from the start
+        const bool tail = 4 * nv + t < n;
+        const double tx = tail ? xs[4 * nv + t] : 0.0, ty = kDot && tail ? ys[4 * nv + t] : 0.0;
         int64_t v = t;
         for (; v + S < nv; v += 2 * S) {
-            f64x4 x0 = ldg_stream_f64x4(xs + 4 * v);
-            f64x4 x1 = ldg_stream_f64x4(xs + 4 * (v + S));
+            const f64x4 x0 = ldg_stream_f64x4(xs + 4 * v);
+            const f64x4 x1 = ldg_stream_f64x4(xs + 4 * (v + S));
             if (kDot) {
-                f64x4 y0 = ldg_stream_f64x4(ys + 4 * v);
-                f64x4 y1 = ldg_stream_f64x4(ys + 4 * (v + S));
-                a0 = fma(x0.x, y0.x, a0); a1 = fma(x0.y, y0.y, a1);
-                a2 = fma(x0.z, y0.z, a2); a3 = fma(x0.w, y0.w, a3);
-                b0 = fma(x1.x, y1.x, b0); b1 = fma(x1.y, y1.y, b1);
-                b2 = fma(x1.z, y1.z, b2); b3 = fma(x1.w, y1.w, b3);
+                const f64x4 y0 = ldg_stream_f64x4(ys + 4 * v);
+                const f64x4 y1 = ldg_stream_f64x4(ys + 4 * (v + S));
+                a = fma(x0.x, y0.x, a); b = fma(x1.x, y1.x, b);
+                a = fma(x0.y, y0.y, a); b = fma(x1.y, y1.y, b);
+                a = fma(x0.z, y0.z, a); b = fma(x1.z, y1.z, b);
+                a = fma(x0.w, y0.w, a); b = fma(x1.w, y1.w, b);
             } else {
-                a0 += x0.x; a1 += x0.y; a2 += x0.z; a3 += x0.w;
-                b0 += x1.x; b1 += x1.y; b2 += x1.z; b3 += x1.w;
+                a += x0.x; b += x1.x;
+                a += x0.y; b += x1.y;
+                a += x0.z; b += x1.z;
+                a += x0.w; b += x1.w;
             }
         }
         if (v < nv) {
-            f64x4 x0 = ldg_stream_f64x4(xs + 4 * v);
+            const f64x4 x0 = ldg_stream_f64x4(xs + 4 * v);
             if (kDot) {
-                f64x4 y0 = ldg_stream_f64x4(ys + 4 * v);
-                a0 = fma(x0.x, y0.x, a0); a1 = fma(x0.y, y0.y, a1);
-                a2 = fma(x0.z, y0.z, a2); a3 = fma(x0.w, y0.w, a3);
+                const f64x4 y0 = ldg_stream_f64x4(ys + 4 * v);
+                a = fma(x0.x, y0.x, a);
+                a = fma(x0.y, y0.y, a);
+                a = fma(x0.z, y0.z, a);
+                a = fma(x0.w, y0.w, a);
             } else {
-                a0 += x0.x; a1 += x0.y; a2 += x0.z; a3 += x0.w;
+                a += x0.x;
+                a += x0.y;
+                a += x0.z;
+                a += x0.w;
             }
         }
-        tail_start = nv * 4;
+        if (tail) a = kDot ? fma(tx, ty, a) : a + tx;
+    } else {  // pointers that are not 32-byte aligned
+        for (int64_t i = t; i < n; i += S) a = kDot ? fma(xs[i], ys[i], a) : a + xs[i];
     }
-    // scalar remainder (or the whole array when the pointers are not 32-byte aligned)
-    for (int64_t i = tail_start + t; i < n; i += S) {
-        if (kDot) a0 = fma(xs[i], ys[i], a0);
-        else a0 += xs[i];
-    }
-    double v = ((a0 + a1) + (a2 + a3)) + ((b0 + b1) + (b2 + b3));
-    double bsum = block_sum(v, sh);
+    const double v = a + b;
+    double bsum = block_sum<kRedThreads>(v, sh);
     __syncthreads();
     finish_partials(bsum, partials, counter, out, sh);
 }
 
+// Short arrays, by one block: no partials through memory and no completion
+// counter.  What counts here is the FP64 pipe of the one SM (a warp instruction
+// holds it for 19 cycles), so there are few warps and each thread keeps one
+// chain of multiply-adds, all its loads in flight.  Per call: 4099 elements 8.2
+// -> 4.1 us, 8192 9.4 -> 6.1, 16384 9.7 -> 8.2 (512 or 1024 threads with eight
+// accumulators each and a tree in every warp: 8.2 at 4099).
+constexpr int kRedOneThreads = 256;
+constexpr int64_t kRedOneBlock = 16384;
+template <bool kDot, bool kVec>
+__global__ void __launch_bounds__(kRedOneThreads) reduce_one_kernel(const double* __restrict__ xs,
+                                                                    const double* __restrict__ ys, int n,
+                                                                    double* out) {
+    __shared__ double sh[kRedOneThreads];
+    constexpr int T = kRedOneThreads, kIn = 4;
+    const int t = threadIdx.x;
+    double acc = 0.0;
+    if (kVec) {
+        const int nv = n >> 2;
+        const bool tail = 4 * nv + t < n;
+        const double tx = tail ? xs[4 * nv + t] : 0.0, ty = kDot && tail ? ys[4 * nv + t] : 0.0;
+        for (int v = t; v < nv; v += kIn * T) {
+            f64x4 x[kIn], y[kIn];
+#pragma unroll
+            for (int u = 0; u < kIn; ++u)
+                if (v + u * T < nv) {
+                    x[u] = ldg_stream_f64x4(xs + 4 * (v + u * T));
+                    if (kDot) y[u] = ldg_stream_f64x4(ys + 4 * (v + u * T));
+                }
+#pragma unroll
+            for (int u = 0; u < kIn; ++u)
+                if (v + u * T < nv) {
+                    acc = kDot ? fma(x[u].x, y[u].x, acc) : acc + x[u].x;
+                    acc = kDot ? fma(x[u].y, y[u].y, acc) : acc + x[u].y;
+                    acc = kDot ? fma(x[u].z, y[u].z, acc) : acc + x[u].z;
+                    acc = kDot ? fma(x[u].w, y[u].w, acc) : acc + x[u].w;
+                }
+        }
+        if (tail) acc = kDot ? fma(tx, ty, acc) : acc + tx;
+    } else {
+#pragma unroll 8
+        for (int i = t; i < n; i += T) acc = kDot ? fma(__ldg(xs + i), __ldg(ys + i), acc) : acc + __ldg(xs + i);
+    }
+    acc = block_sum<T>(acc, sh);
+    if (t == 0) *out = acc;
+}
+
+// Blocks for n elements on `sms` SMs: two vectors per thread until every SM has
+// two blocks.
+static int64_t reduce_blocks(int64_t n, int sms) {
+    const int64_t want = ((n + 3) / 4 + 2LL * kRedThreads - 1) / (2LL * kRedThreads);
+    const int64_t most = (int64_t)sms * kRedBlocksPerSM;
+    return want < most ? want : most;
+}
+static void reduce_one(bool dot, bool vec, const double* xs, const double* ys, int64_t n, double* out,
+                       cudaStream_t s) {
+    auto k = dot ? (vec ? reduce_one_kernel<true, true> : reduce_one_kernel<true, false>)
+                 : (vec ? reduce_one_kernel<false, true> : reduce_one_kernel<false, false>);
+    k<<<1, kRedOneThreads, 0, s>>>(xs, ys, (int)n, out);
+}
+
 static int reduce_launch(bool dot, const double* xs, const double* ys, int64_t n, double* out,
                          cudaStream_t stream) {
+    const bool vec = ((reinterpret_cast<uintptr_t>(xs) | (dot ? reinterpret_cast<uintptr_t>(ys) : 0)) & 31) == 0;
     Device* d = nullptr;
     HYD_TRY(device(&d));
-    const int64_t units = (n + 3) / 4;
-    int64_t blocks = (int64_t)d->sm_count * kRedBlocksPerSM;
-    int64_t want = (units + 2LL * kRedThreads - 1) / (2LL * kRedThreads);
-    if (want < blocks) blocks = want < 1 ? 1 : want;
+    if (n <= kRedOneBlock) {
+        reduce_one(dot, vec, xs, dot ? ys : xs, n, out, stream);
+        return launch_check(dot ? "dot_f64" : "sum_f64");
+    }
+    const int64_t blocks = reduce_blocks(n, d->sm_count);
     unsigned* counters = nullptr;
     void* scratch = nullptr;
     HYD_TRY(workspace(stream, sizeof(double) * (size_t)blocks, &counters, &scratch));
     double* partials = static_cast<double*>(scratch);
     unsigned* counter = counters + (dot ? 0 : 1);
-    const bool vec = ((reinterpret_cast<uintptr_t>(xs) | (dot ? reinterpret_cast<uintptr_t>(ys) : 0)) & 31) == 0;
     dim3 grid((unsigned)blocks), block(kRedThreads);
     if (dot) {
         if (vec) reduce_f64_kernel<true, true><<<grid, block, 0, stream>>>(xs, ys, n, partials, counter, out);
@@ -230,11 +302,13 @@ extern "C" int hyd_cuda_dot_f64_noalloc(const double* xs, const double* ys, int6
     unsigned char* scratch = nullptr;
     int sms = 0;
     HYD_TRY(noalloc_setup(dev, &scratch, &sms));
-    // Same grid rule as hyd_cuda_dot_f64, so both give the same bits.
-    const int64_t units = (n + 3) / 4;
-    int64_t blocks = (int64_t)sms * kRedBlocksPerSM;
-    const int64_t want = (units + 2LL * kRedThreads - 1) / (2LL * kRedThreads);
-    if (want < blocks) blocks = want < 1 ? 1 : want;
+    // Same kernels and grid rule as hyd_cuda_dot_f64, so both give the same bits.
+    const bool vec = ((reinterpret_cast<uintptr_t>(xs) | reinterpret_cast<uintptr_t>(ys)) & 31) == 0;
+    if (n <= kRedOneBlock) {
+        reduce_one(true, vec, xs, ys, n, out, as_stream(stream));
+        return launch_check("dot_f64_noalloc");
+    }
+    const int64_t blocks = reduce_blocks(n, sms);
     if (blocks > kNoAllocMaxBlocks)
         return set_error(HYD_CUDA_ERR_UNSUPPORTED,
                          "dot_f64_noalloc: needs %lld CTAs of scratch but the static scratch holds %d",
@@ -244,7 +318,6 @@ extern "C" int hyd_cuda_dot_f64_noalloc(const double* xs, const double* ys, int6
     cudaStream_t st = as_stream(stream);
     // The array keeps whatever the previous call left; the counter must start at 0.
     HYD_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned), st));
-    const bool vec = ((reinterpret_cast<uintptr_t>(xs) | reinterpret_cast<uintptr_t>(ys)) & 31) == 0;
     if (vec)
         reduce_f64_kernel<true, true><<<(unsigned)blocks, kRedThreads, 0, st>>>(xs, ys, n, partials, counter, out);
     else
