@@ -229,9 +229,13 @@ def ptr(t):
 
 
 def stream_handle(stream=None):
+    if stream is not None:
+        return stream.cuda_stream
     import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    if not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    # the same handle without the Stream object (0.3 us instead of 3, on every call)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def call(name, *args):
