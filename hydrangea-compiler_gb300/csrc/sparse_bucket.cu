@@ -3,7 +3,7 @@
 // Same contract as batch_pipeline in sparse.cu (per instance: CSR of the
 // entries sorted by (row, col), y = A x), organised so that no stage walks
 // rows one dependent memory chain at a time:
-//  1. count   per CTA, a contiguous range of (instance, 8192-entry tile)
+//  1. count   per CTA, a contiguous range of (instance, 6144-entry tile)
 //             items: a shared-memory histogram of 64-row buckets (row >> 6),
 //             flushed with one global red per non-empty bucket when the
 //             instance changes;
@@ -12,10 +12,10 @@
 //             each instance's entry offsets);
 //  3. split   per tile again: each entry gets its rank inside (tile, bucket)
 //             from a shared-memory atomic, each (tile, bucket) reserves its run
-//             with one global atomic, and the entry is written to the bucket's
-//             region as a 32-bit key (row_in_bucket << 24 | col) plus its value
-//             (the tile's values are prefetched into shared memory with
-//             cp.async while the ranks and reservations are computed);
+//             with one global atomic, and the tile, put into bucket order in
+//             shared memory, is written to the buckets' regions as 16-byte
+//             records: a 32-bit key (row_in_bucket << 24 | col), the COO
+//             position and the value;
 //  4. bucket  one block per bucket (at most 2048 entries, ncols <= 2^18): a
 //             counting pass into as many bins as entries, in (row, col) order,
 //             and comparisons inside the bins; the CSR columns/values written
@@ -46,7 +46,11 @@ constexpr int kBkThreads = 512;
 constexpr int kBkShift = 6;                  // 64 rows per bucket
 constexpr int kBkRows = 1 << kBkShift;
 constexpr int kBkCap = kBkRows * 256;        // entries per bucket at most (256 per row)
-constexpr int kTileEntries = 8192;           // entries per count/split work item
+constexpr int kSplitThreads = 512;
+constexpr int kSplitPerSm = 2;
+constexpr int kSplitPer = 12;                // entries per thread of the split
+constexpr int kTileEntries = kSplitThreads * kSplitPer;  // entries per count/split work item
+constexpr int kCountEntries = kBkThreads * 12;           // entries the count loads at once
 constexpr int kMaxSmemBuckets = 4096;        // per instance (2^18 rows)
 
 struct BkInst {
@@ -128,22 +132,24 @@ __global__ void __launch_bounds__(kBkThreads, kCountPerSm) bk_count_kernel(const
         // all of this thread's rows first (read-only loads, all in flight at
         // once), then the counting: a load next to an atomic would otherwise
         // wait for it, one memory round trip per entry
-        int rr[kTileEntries / kBkThreads];
+        for (long long c0 = t0; c0 < t1; c0 += kCountEntries) {
+            int rr[kCountEntries / kBkThreads];
 #pragma unroll
-        for (int j = 0; j < kTileEntries / kBkThreads; ++j) {
-            const long long k = t0 + threadIdx.x + (long long)j * kBkThreads;
-            rr[j] = k < t1 ? __ldg(I.rows + k) : INT_MIN;
-        }
-#pragma unroll
-        for (int j = 0; j < kTileEntries / kBkThreads; ++j) {
-            const int r = rr[j];  // columns are checked by the split, which reads them anyway
-            if (r == INT_MIN && t0 + threadIdx.x + (long long)j * kBkThreads >= t1) continue;
-            if (r < 0 || r >= I.nrows) {
-                bad = true;
-                continue;
+            for (int j = 0; j < kCountEntries / kBkThreads; ++j) {
+                const long long k = c0 + threadIdx.x + (long long)j * kBkThreads;
+                rr[j] = k < t1 ? __ldg(I.rows + k) : INT_MIN;
             }
-            if (smem) atomicAdd(&hist[r >> kBkShift], 1u);
-            else atomicAdd(&bcount[I.bucket_base + (r >> kBkShift)], 1u);
+#pragma unroll
+            for (int j = 0; j < kCountEntries / kBkThreads; ++j) {
+                const int r = rr[j];  // columns are checked by the split, which reads them anyway
+                if (r == INT_MIN && c0 + threadIdx.x + (long long)j * kBkThreads >= t1) continue;
+                if (r < 0 || r >= I.nrows) {
+                    bad = true;
+                    continue;
+                }
+                if (smem) atomicAdd(&hist[r >> kBkShift], 1u);
+                else atomicAdd(&bcount[I.bucket_base + (r >> kBkShift)], 1u);
+            }
         }
     }
     __syncthreads();
@@ -175,12 +181,32 @@ __global__ void bk_widen_kernel(const unsigned* __restrict__ c, long long* __res
         out[i] = c[i];
 }
 
-// Stage 3.
-constexpr int kSplitPer = kTileEntries / kBkThreads;  // 16 entries per thread
-// The tile's values are copied into shared memory with cp.async as soon as
-// the tile starts (8 bytes per copy, each thread the slots it later reads), so
-// no global load is left on the path from the reservations to the stores.
-constexpr size_t kSplitSmem = (size_t)kTileEntries * 8;  // 64 KB of values
+// Stage 3.  The tile is put into bucket order in shared memory before it is
+// written, so that a bucket's run leaves as consecutive records from
+// neighbouring lanes.
+//  * the values are copied into shared memory with cp.async as soon as the
+//    tile starts, and wait there in COO order;
+//  * an entry's place in bucket order (the exclusive scan of the tile's bucket
+//    counts, plus its rank) receives its key and, in one word, its bucket and
+//    its position in the tile;
+//  * the global reservations are in flight while that happens;
+//  * the words are then read back in order: record p of the tile goes to
+//    hist[bucket] + p, with hist[bucket] the run's first slot less its first
+//    place;
+//  * thread 0 asks for the next tile's entries to be brought into L2 meanwhile.
+// Written from COO order, a lane's record went to a bucket of its own: 32 write
+// requests of one sector per warp instruction, and those bounded the kernel.
+// 2.9e8 entries in 512 instances of 2^10 to 2^18 rows: 3.88 ms so (8192-entry
+// tiles), 2.77 ms in bucket order, 2.49 ms with the prefetch (reading and
+// writing 32 bytes per entry takes 1.37 ms at the copy rate).  Two blocks of
+// 512 threads with 6144 entries each fill an SM's shared memory; one block of
+// 1024 threads with 12288, whose runs are twice as long, has no second block to
+// fill its barriers and took 1% more of the whole pipeline.
+constexpr int kSplitPosBits = 14;
+static_assert(kTileEntries <= 1 << kSplitPosBits, "position in a tile");
+static_assert(kMaxSmemBuckets <= 1 << (32 - kSplitPosBits), "bucket beside the position");
+constexpr int kSplitBins = kMaxSmemBuckets / kSplitThreads;  // buckets per thread in the scan
+constexpr size_t kSplitSmem = (size_t)kTileEntries * 16 + (kMaxSmemBuckets + 4) * 4;
 
 __device__ __forceinline__ void cp_async_8(void* smem_dst, const void* gsrc) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(smem_dst)),
@@ -188,47 +214,71 @@ __device__ __forceinline__ void cp_async_8(void* smem_dst, const void* gsrc) {
                  : "memory");
 }
 
-__global__ void __launch_bounds__(kBkThreads, 2) bk_split_kernel(const BkInst* __restrict__ inst,
-                                                              const BkItem* __restrict__ items, unsigned nitems,
-                                                              unsigned* cursor, const long long* __restrict__ bstart,
-                                                              unsigned* __restrict__ bfill,
-                                                              uint4* __restrict__ rec_out, unsigned* err) {
-    __shared__ unsigned hist[kMaxSmemBuckets];
-    __shared__ unsigned gbase[kMaxSmemBuckets];  // batch-wide slots (< 2^32, checked on the host)
-    extern __shared__ __align__(16) double split_vals[];
-    unsigned it;
+__global__ void __launch_bounds__(kSplitThreads, kSplitPerSm) bk_split_kernel(
+    const BkInst* __restrict__ inst, const BkItem* __restrict__ items, unsigned nitems, unsigned* cursor,
+    const long long* __restrict__ bstart, unsigned* __restrict__ bfill, uint4* __restrict__ rec_out, unsigned* err) {
+    extern __shared__ __align__(16) double split_vals[];          // [kTileEntries], COO order
+    unsigned* skey = (unsigned*)(split_vals + kTileEntries);      // [kTileEntries], bucket order
+    unsigned* spos = skey + kTileEntries;                         // [kTileEntries], bucket << 14 | position
+    unsigned* hist = spos + kTileEntries;                         // [kMaxSmemBuckets + 1]
+    __shared__ unsigned warp_sum[kSplitThreads / 32];
+    __shared__ unsigned sh_it[2];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     bool bad = false;
-    while (bk_next(cursor, nitems, it)) {
+    unsigned next = 0u;  // thread 0's: the tile after the current one
+    if (threadIdx.x == 0) {
+        sh_it[0] = blockIdx.x;
+        next = gridDim.x + atomicAdd(cursor, 1u);
+    }
+    __syncthreads();
+    for (unsigned turn = 0;; turn ^= 1u) {
+        const unsigned it = sh_it[turn];
+        if (it >= nitems) break;
         const BkItem w = items[it];
         const BkInst I = inst[w.inst];
         const bool smem = I.nbuckets <= kMaxSmemBuckets;
         const long long t0 = (long long)w.tile * kTileEntries;
-        const long long t1 = t0 + kTileEntries < I.nnz ? t0 + kTileEntries : I.nnz;
+        const int tn = (int)(t0 + kTileEntries < I.nnz ? kTileEntries : I.nnz - t0);
+        // the rows and columns of all this thread's entries first (read-only
+        // loads, all in flight at once), then the values' copies
+        int bucket[kSplitPer];
+        unsigned key[kSplitPer], rank[kSplitPer];
 #pragma unroll
         for (int j = 0; j < kSplitPer; ++j) {
-            const int q = threadIdx.x + j * kBkThreads;
-            if (t0 + q < t1) cp_async_8(split_vals + q, I.vals + t0 + q);
+            const int q = threadIdx.x + j * kSplitThreads;
+            bucket[j] = q < tn ? __ldg(I.rows + t0 + q) : -1;
+            key[j] = q < tn ? (unsigned)__ldg(I.cols + t0 + q) : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < kSplitPer; ++j) {
+            const int q = threadIdx.x + j * kSplitThreads;
+            if (q < tn) cp_async_8(split_vals + q, I.vals + t0 + q);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
-        if (smem)
-            for (int b = threadIdx.x; b < I.nbuckets; b += kBkThreads) hist[b] = 0u;
-        __syncthreads();
-        unsigned key[kSplitPer], rank[kSplitPer];
-        int bucket[kSplitPer];
-        // the rows and columns of all this thread's entries first (read-only
-        // loads, all in flight at once), then the ranking atomics
-#pragma unroll
-        for (int j = 0; j < kSplitPer; ++j) {
-            const long long k = t0 + threadIdx.x + (long long)j * kBkThreads;
-            bucket[j] = k < t1 ? __ldg(I.rows + k) : -1;
-            key[j] = k < t1 ? (unsigned)__ldg(I.cols + k) : 0u;
+        if (threadIdx.x == 0) {
+            // the next tile's entries on their way to L2 while this one is sorted
+            sh_it[turn ^ 1u] = next;
+            if (next < nitems) {
+                const BkItem nw = items[next];
+                const BkInst N = inst[nw.inst];
+                const long long n0 = (long long)nw.tile * kTileEntries;
+                const long long nn = n0 + kTileEntries < N.nnz ? kTileEntries : N.nnz - n0;
+                l2_prefetch(N.rows + n0, nn * 4);
+                l2_prefetch(N.cols + n0, nn * 4);
+                l2_prefetch(N.vals + n0, nn * 8);
+                next = gridDim.x + atomicAdd(cursor, 1u);
+            }
         }
+        if (smem)
+            for (int b = threadIdx.x; b <= kMaxSmemBuckets / 4; b += kSplitThreads)
+                ((uint4*)hist)[b] = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();
 #pragma unroll
         for (int j = 0; j < kSplitPer; ++j) {
-            const long long k = t0 + threadIdx.x + (long long)j * kBkThreads;
+            const int q = threadIdx.x + j * kSplitThreads;
             const int r = bucket[j], c = (int)key[j];
             bucket[j] = -1;
-            if (k < t1) {
+            if (q < tn) {
                 if (c < 0 || c >= I.ncols) bad = true;                 // (rows were checked by the count)
                 if (r >= 0 && r < I.nrows && c >= 0 && c < I.ncols) {
                     bucket[j] = r >> kBkShift;
@@ -238,39 +288,92 @@ __global__ void __launch_bounds__(kBkThreads, 2) bk_split_kernel(const BkInst* _
             }
         }
         __syncthreads();
-        if (smem) {
-            // reserve this tile's run in every non-empty bucket; the atomics of
-            // one thread are independent, so they are all issued before any
-            // result is used (one memory round trip instead of eight)
-            constexpr int kPerThread = kMaxSmemBuckets / kBkThreads;
-            unsigned got[kPerThread];
+        if (!smem) {
+            // more buckets than the shared counts hold: one global atomic per
+            // entry, written where it lands
+            asm volatile("cp.async.wait_all;" ::: "memory");  // this thread's own copies
 #pragma unroll
-            for (int q = 0; q < kPerThread; ++q) {
-                const int b = threadIdx.x + q * kBkThreads;
-                const unsigned c = b < I.nbuckets ? hist[b] : 0u;
-                got[q] = c ? atomicAdd(&bfill[I.bucket_base + b], c) : 0u;
+            for (int j = 0; j < kSplitPer; ++j) {
+                if (bucket[j] < 0) continue;
+                const int q = threadIdx.x + j * kSplitThreads;
+                const double v = split_vals[q];
+                const long long pos =
+                    bstart[I.bucket_base + bucket[j]] + atomicAdd(&bfill[I.bucket_base + bucket[j]], 1u);
+                rec_out[pos] = make_uint4(key[j], (unsigned)(t0 + q), (unsigned)__double2loint(v),
+                                          (unsigned)__double2hiint(v));
             }
+            __syncthreads();
+            continue;
+        }
+        // exclusive scan of the counts in place; hist[kMaxSmemBuckets] = all
+        {
+            unsigned c[kSplitBins], sum = 0u;
 #pragma unroll
-            for (int q = 0; q < kPerThread; ++q) {
-                const int b = threadIdx.x + q * kBkThreads;
-                if (b < I.nbuckets && hist[b]) gbase[b] = (unsigned)(bstart[I.bucket_base + b] + got[q]);
+            for (int i = 0; i < kSplitBins; i += 4) {
+                const uint4 v = ((const uint4*)hist)[(threadIdx.x * kSplitBins + i) >> 2];
+                c[i] = v.x, c[i + 1] = v.y, c[i + 2] = v.z, c[i + 3] = v.w;
+                sum += v.x + v.y + v.z + v.w;
             }
+            unsigned incl = sum;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const unsigned o = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += o;
+            }
+            if (lane == 31) warp_sum[wid] = incl;
+            __syncthreads();
+            unsigned before = lane < kSplitThreads / 32 && lane < wid ? warp_sum[lane] : 0u;
+            before = __reduce_add_sync(0xffffffffu, before);
+            unsigned run = before + incl - sum;
+#pragma unroll
+            for (int i = 0; i < kSplitBins; i += 4) {
+                uint4 v;
+                v.x = run, run += c[i];
+                v.y = run, run += c[i + 1];
+                v.z = run, run += c[i + 2];
+                v.w = run, run += c[i + 3];
+                ((uint4*)hist)[(threadIdx.x * kSplitBins + i) >> 2] = v;
+            }
+            if (threadIdx.x == kSplitThreads - 1) hist[kMaxSmemBuckets] = run;
         }
         __syncthreads();
-        // this thread's values have landed in shared memory (its own copies)
-        asm volatile("cp.async.wait_all;" ::: "memory");
+        const int total = (int)hist[kMaxSmemBuckets];
+        // reserve this tile's run in every non-empty bucket; the atomics of
+        // one thread are independent, and their results are first needed after
+        // the placing below
+        unsigned first[kSplitBins];
+#pragma unroll
+        for (int i = 0; i < kSplitBins; ++i) {
+            const int b = threadIdx.x + i * kSplitThreads;
+            const unsigned c = hist[b + 1] - hist[b];
+            first[i] = c ? (unsigned)bstart[I.bucket_base + b] + atomicAdd(&bfill[I.bucket_base + b], c) : 0u;
+        }
 #pragma unroll
         for (int j = 0; j < kSplitPer; ++j) {
             if (bucket[j] < 0) continue;
-            const int q = threadIdx.x + j * kBkThreads;
-            const long long k = t0 + q;
+            const int p = (int)(hist[bucket[j]] + rank[j]);
+            skey[p] = key[j];
+            spos[p] = ((unsigned)bucket[j] << kSplitPosBits) | (unsigned)(threadIdx.x + j * kSplitThreads);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();  // every place is read and every value has landed
+#pragma unroll
+        for (int i = 0; i < kSplitBins; ++i) {
+            const int b = threadIdx.x + i * kSplitThreads;
+            hist[b] = first[i] - hist[b];  // batch-wide slots (< 2^32, checked on the host), modulo 2^32
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kSplitPer; ++j) {
+            const int p = threadIdx.x + j * kSplitThreads;
+            if (p >= total) break;
+            const unsigned e = spos[p];
+            const unsigned q = e & ((1u << kSplitPosBits) - 1u);
             const double v = split_vals[q];
-            const long long pos = smem ? (long long)gbase[bucket[j]] + rank[j]
-                                       : bstart[I.bucket_base + bucket[j]] +
-                                             atomicAdd(&bfill[I.bucket_base + bucket[j]], 1u);
             // one 16-byte record: the key, the entry's COO position (orders
             // equal (row, col) keys) and the value
-            rec_out[pos] = make_uint4(key[j], (unsigned)k, (unsigned)__double2loint(v), (unsigned)__double2hiint(v));
+            rec_out[hist[e >> kSplitPosBits] + (unsigned)p] =
+                make_uint4(skey[p], (unsigned)t0 + q, (unsigned)__double2loint(v), (unsigned)__double2hiint(v));
         }
         __syncthreads();
     }
@@ -1098,8 +1201,8 @@ int batch_pipeline_bucketed(std::vector<BatchInst>& bi, const char* key, cudaStr
     HYD_TRY(scan_i64_launch(wide, bstart, nb_total, 0, false, false, s));
     if (n_tiles) {
         HYD_TRY(configure_kernel((const void*)bk_split_kernel, d, false));
-        bk_split_kernel<<<grid, kBkThreads, kSplitSmem, s>>>(d_inst, d_tiles, (unsigned)n_tiles, cursors + 1, bstart,
-                                                             bfill, recs, d->d_err);
+        bk_split_kernel<<<(unsigned)(d->sm_count * kSplitPerSm), kSplitThreads, kSplitSmem, s>>>(
+            d_inst, d_tiles, (unsigned)n_tiles, cursors + 1, bstart, bfill, recs, d->d_err);
         HYD_TRY(launch_check("bk_split"));
     }
     // cursors: 2 the buckets of at most 1024 entries, 9 the larger ones (8: how
