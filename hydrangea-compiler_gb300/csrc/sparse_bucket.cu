@@ -23,11 +23,11 @@
 //             Buckets with clustered columns are sorted by a warp each, with a
 //             stable LSD radix sort of the packed keys; larger buckets by a
 //             block-wide bitonic network;
-//  5. spmv    one warp per 256-row chunk of an instance: the rows are ordered
+//  5. spmv    one warp per chunk of 32 to 256 rows of an instance: the rows are ordered
 //             by length in shared memory and each lane sums one row's fma
 //             chain in column order, 32 rows of similar length at a time.
 // The work lists of the stages (one item per (instance, tile), per (instance,
-// bucket) and per (instance, 256-row chunk)) are written on the device; only
+// bucket) and per (instance, chunk of rows)) are written on the device; only
 // the instance table crosses from the host.
 // Requires ncols < 2^24 (24-bit column field) and at most 256 entries per row.
 #include <climits>
@@ -58,7 +58,7 @@ struct BkInst {
     long long bucket_base;  // first bucket in the batch-wide bucket space
     long long nbuckets;
     long long tile_base;    // first entry tile in the batch-wide tile list
-    long long chunk_base;   // first 256-row SpMV chunk in the batch-wide chunk list
+    long long chunk_base;   // first SpMV chunk in the batch-wide chunk list
     long long scan_base;    // entries of all earlier instances
     const int* rows;
     const int* cols;
@@ -157,18 +157,19 @@ __global__ void __launch_bounds__(kBkThreads, kCountPerSm) bk_count_kernel(const
     if (bad) raise_error(err, ERRBIT_BOUNDS);
 }
 
-constexpr int kSpRows = 256;  // rows per SpMV chunk
+constexpr int kSpRows = 256;    // rows per SpMV chunk, at most
+constexpr int kSpMinRows = 32;  // and at least
 
 // The work lists of the count/split stages (one item per (instance, entry
 // tile)), of the bucket stage (one per (instance, bucket)) and of the SpMV
-// (one per (instance, 256-row chunk)), written on the device: block i writes
+// (one per (instance, chunk of rows)), written on the device: block i writes
 // instance i's items at its tile_base / bucket_base / chunk_base.
 __global__ void bk_items_kernel(const BkInst* __restrict__ inst, int64_t ninst, BkItem* __restrict__ tiles,
-                                BkItem* __restrict__ buckets, BkItem* __restrict__ chunks) {
+                                BkItem* __restrict__ buckets, BkItem* __restrict__ chunks, int chunk_rows) {
     for (int64_t i = blockIdx.x; i < ninst; i += gridDim.x) {
         const BkInst I = inst[i];
         const long long nt = (I.nnz + kTileEntries - 1) / kTileEntries;
-        const long long nc = (I.nrows + kSpRows - 1) / kSpRows;
+        const long long nc = (I.nrows + chunk_rows - 1) / chunk_rows;
         for (long long t = threadIdx.x; t < nt; t += blockDim.x) tiles[I.tile_base + t] = BkItem{(int)i, (int)t};
         for (long long b = threadIdx.x; b < I.nbuckets; b += blockDim.x)
             buckets[I.bucket_base + b] = BkItem{(int)i, (int)b};
@@ -987,10 +988,18 @@ __global__ void __launch_bounds__(kBkThreads) bk_bucket_kernel(const BkInst* __r
 // the finished CSR.  Each FP64 warp instruction holds the FP64 pipe for the
 // whole warp whatever its active lanes, so one lane per row only pays when
 // the 32 rows of a warp instruction have similar lengths: a warp takes a
-// 256-row chunk of one instance, counting-sorts its rows by length (256 bins,
+// chunk of one instance's rows, counting-sorts them by length (256 bins,
 // lengths above 255 share the last) in shared memory, and gives each lane one
 // row of every group of 32 consecutive rows in that order.  A lane reads its
 // row 4 entries at a time with 16-byte loads, ahead of the (in-order) chain.
+// Chunks have 256 rows, halved down to 32 while the batch has fewer chunks than
+// the chip has resident warps.  Whole pipeline: one instance of 2^13.5 to
+// 2^16.3 rows 197 -> 153 us, 24 of 2^10 to 2^14 rows 283 -> 232, 4 of 2^16 to
+// 2^18 rows 374 -> 351.  (Halving until there are four chunks per warp takes 64
+// instances of 2^12 to 2^16 rows from 676 to 723 us.)  Chunks above 256 rows
+// fill more lanes of the FP64 pipe, but their rows' entries no longer wait in
+// L1 and L2 for the neighbouring rows: 2.2 ms with 512 rows instead of 2.06 for
+// 2.9e8 entries, 3.0 ms with 1024.
 // Rows above 256 entries are outside the contract and reported.
 constexpr int kSpWarps = 8;
 constexpr int kSpPerSm = 4;
@@ -1003,7 +1012,7 @@ struct BkSpSmem {
 
 __global__ void __launch_bounds__(kSpWarps * 32, kSpPerSm)
     bk_spmv_kernel(const BkInst* __restrict__ inst, const BkItem* __restrict__ chunks, unsigned nchunks,
-                   unsigned* cursor, unsigned* err) {
+                   int chunk_rows, unsigned* cursor, unsigned* err) {
     __shared__ BkSpSmem sm_all[kSpWarps];
     const int lane = threadIdx.x & 31;
     BkSpSmem& sm = sm_all[threadIdx.x >> 5];
@@ -1015,8 +1024,8 @@ __global__ void __launch_bounds__(kSpWarps * 32, kSpPerSm)
         if (it >= nchunks) break;
         const BkItem w = chunks[it];
         const BkInst I = inst[w.inst];
-        const long long r0 = (long long)w.tile * kSpRows;
-        const int nr = (int)((I.nrows - r0) < kSpRows ? (I.nrows - r0) : kSpRows);
+        const long long r0 = (long long)w.tile * chunk_rows;
+        const int nr = (int)((I.nrows - r0) < chunk_rows ? (I.nrows - r0) : chunk_rows);
 #pragma unroll
         for (int j = 0; j < 8; ++j) sm.cnt[lane + 32 * j] = 0u;
         __syncwarp();
@@ -1115,7 +1124,10 @@ int batch_pipeline_bucketed(std::vector<BatchInst>& bi, const char* key, cudaStr
     Device* d = nullptr;
     HYD_TRY(device(&d));
     std::vector<BkInst> inst(bi.size());
-    long long nb_total = 0, entries = 0, nt_total = 0, nc_total = 0;
+    long long nb_total = 0, entries = 0, nt_total = 0, nc_total = 0, rows_total = 0;
+    for (const BatchInst& B : bi) rows_total += B.nrows;
+    int chunk_rows = kSpRows;
+    while (chunk_rows > kSpMinRows && rows_total < (long long)chunk_rows * kSpWarps * kSpPerSm * d->sm_count) chunk_rows /= 2;
     for (size_t i = 0; i < bi.size(); ++i) {
         const BatchInst& B = bi[i];
         if (B.ncols >= (1LL << 24) || B.nrows >= (1LL << 31)) return HYD_CUDA_ERR_UNSUPPORTED;
@@ -1137,7 +1149,7 @@ int batch_pipeline_bucketed(std::vector<BatchInst>& bi, const char* key, cudaStr
         I.tile_base = nt_total;
         I.chunk_base = nc_total;
         nt_total += (B.nnz + kTileEntries - 1) / kTileEntries;
-        nc_total += (B.nrows + kSpRows - 1) / kSpRows;
+        nc_total += (B.nrows + chunk_rows - 1) / chunk_rows;
         nb_total += I.nbuckets;
         entries += B.nnz;
     }
@@ -1183,7 +1195,7 @@ int batch_pipeline_bucketed(std::vector<BatchInst>& bi, const char* key, cudaStr
     {
         const int64_t ni = (int64_t)inst.size();
         const unsigned g = (unsigned)(ni < 4096 ? ni : 4096);
-        bk_items_kernel<<<g, 256, 0, s>>>(d_inst, ni, d_tiles, d_bk, d_chunks);
+        bk_items_kernel<<<g, 256, 0, s>>>(d_inst, ni, d_tiles, d_bk, d_chunks, chunk_rows);
         HYD_TRY(launch_check("bk_items"));
     }
     const size_t n_tiles = (size_t)nt_total, n_buckets = (size_t)nb_total;
@@ -1231,9 +1243,8 @@ int batch_pipeline_bucketed(std::vector<BatchInst>& bi, const char* key, cudaStr
                                                        recs, d->d_err);
     HYD_TRY(launch_check("bk_bucket_large"));
     if (nc_total) {
-        bk_spmv_kernel<<<(unsigned)(d->sm_count * kSpPerSm), kSpWarps * 32, 0, s>>>(d_inst, d_chunks,
-                                                                                  (unsigned)nc_total, cursors + 5,
-                                                                                  d->d_err);
+        bk_spmv_kernel<<<(unsigned)(d->sm_count * kSpPerSm), kSpWarps * 32, 0, s>>>(
+            d_inst, d_chunks, (unsigned)nc_total, chunk_rows, cursors + 5, d->d_err);
         HYD_TRY(launch_check("bk_spmv"));
     }
     if (!async_tables) HYD_CUDA_TRY(cudaStreamSynchronize(s));

@@ -1,9 +1,9 @@
 """GPU parity of the batched pipeline's entry tiles (6144 entries, put into
 bucket order in shared memory) at their edges: entry counts around one and two
 tiles, one bucket, 4096 buckets (the most a tile counts in shared memory) and
-one more, more tiles than blocks, values at 8-byte offsets.  CSR bit-exact
-(equal entries in COO order), y within the tolerance; an invalid column is
-reported and its neighbours are not."""
+one more, more tiles than blocks; and of the SpMV's chunks of rows at the
+totals where their size changes.  CSR bit-exact (equal entries in COO order),
+y within the tolerance; an invalid column is reported."""
 import numpy as np
 import pytest
 import torch
@@ -35,6 +35,19 @@ def test_bucket_count_edges(hc, orc, dev, n):
 def test_more_tiles_than_blocks(hc, orc, dev):
     rng = np.random.default_rng(3)
     _check(hc, orc, dev, [_random(40_001 + 64 * k, 30_000, 400_003 + 2 * k, rng) for k in range(8)])
+
+
+@pytest.mark.parametrize("chunk", [32, 64, 128, 256])
+@pytest.mark.parametrize("off", [-1, 0, 1])
+def test_chunk_sizes(hc, orc, dev, chunk, off):
+    # a chunk has 64, 128 or 256 rows once there is one such chunk per resident warp
+    rows = torch.cuda.get_device_properties(dev).multi_processor_count * 32 * chunk + off
+    rng = np.random.default_rng(chunk)
+    insts = []
+    for n in (rows // 3, 1, 33, rows - rows // 3 - 34):
+        r = np.concatenate([rng.integers(0, n, size=n // 2), np.full(150, n // 2), np.full(100, n - 1)])
+        insts.append((n, 999, rng.permutation(r).astype(np.int32), rng.integers(0, 999, size=len(r)).astype(np.int32)))
+    _check(hc, orc, dev, insts)
 
 
 def test_invalid_column_is_reported(hc, orc, dev):
