@@ -488,7 +488,7 @@ __device__ __forceinline__ void bk_rank_pass(const unsigned* src, unsigned* dst,
 }
 
 // The bucket sort of the 512-instance batch (2.9e8 entries): 5.22 + 0.21 ms with
-// the radix form for every bucket and the block-wide kernel, 1.77 + 0.70 + 0.04
+// the radix form for every bucket and the block-wide kernel, 1.56 + 0.65 + 0.04
 // ms now.  Buckets whose columns are not clustered take no rank chain: one
 // counting pass puts every entry into a bin, the bins being in (row, column)
 // order, and the few entries that share a bin are ordered by comparing them.
@@ -502,8 +502,11 @@ __device__ __forceinline__ void bk_rank_pass(const unsigned* src, unsigned* dst,
 //  * an entry's final place is its bin's start plus the number of entries in
 //    the bin that sort before it (equal keys: by COO position).
 // The bucket's records come to shared memory in one bulk copy, and four warps
-// share the bucket.  The L1 pipe bounds the kernel (about 55 wavefronts per 32
-// entries); with a warp per bucket shared memory left 14 warps per SM and the
+// share the bucket.  The L1 pipe bounds the kernel (about 41 wavefronts per 32
+// entries); a thread's at most eight keys, and the packed words made of them,
+// stay in registers from the first read to the last placing (kept in shared
+// memory, the keys a record apart, they took 14 wavefronts more: 1.77 + 0.70
+// ms); with a warp per bucket shared memory left 14 warps per SM and the
 // phases' latencies bound it, and reading the values from global memory in
 // sorted order, a line per lane, was a third of the pipe's work.  A bucket
 // whose bins overflow both ways goes to `clustered` (the radix form below), a
@@ -542,7 +545,7 @@ __global__ void __launch_bounds__(bk_place_threads<kCap>(), bk_place_per_sm<kCap
     __shared__ int sh_entries;    // ... its entries
     __shared__ long long sh_slot;  // and its first slot: read ahead by thread 0
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int T = bk_place_threads<kCap>(), kIdx = bk_place_idx_bits<kCap>();
+    constexpr int T = bk_place_threads<kCap>(), kIdx = bk_place_idx_bits<kCap>(), kPer = kCap / T;
     constexpr int kRankAt = kIdx + kBkColBits, kRankBits = 32 - kRankAt;
     constexpr unsigned kBinMax = 1u << kRankBits, kIdxMask = (1u << kIdx) - 1u;
     constexpr unsigned kColMask = (1u << kBkColBits) - 1u, kRankMask = (kBinMax - 1u) << kRankAt;
@@ -618,9 +621,16 @@ __global__ void __launch_bounds__(bk_place_threads<kCap>(), bk_place_per_sm<kCap
         }
         if (tid == 0) draw();  // (everyone has read the current one)
         bool big = !tried;
+        unsigned kk[kPer];  // this thread's keys, later their packed words
+        auto load_keys = [&]() {
+#pragma unroll
+            for (int j = 0; j < kPer; ++j) kk[j] = tid + j * T < E ? bk_key24(rec[tid + j * T].x, cbits) : 0u;
+        };
         if (fits && tried) {
-#pragma unroll 4
-            for (int p = tid; p < E; p += T) atomicAdd(&rowinfo[bk_key24(rec[p].x, cbits) >> cbits], 1u);
+            load_keys();
+#pragma unroll
+            for (int j = 0; j < kPer; ++j)
+                if (tid + j * T < E) atomicAdd(&rowinfo[kk[j] >> cbits], 1u);
             __syncthreads();
             if (warp == 0) {  // lane l owns rows 2l, 2l + 1
                 const unsigned n0 = rowinfo[2 * lane], n1 = rowinfo[2 * lane + 1];
@@ -638,15 +648,17 @@ __global__ void __launch_bounds__(bk_place_threads<kCap>(), bk_place_per_sm<kCap
             const float whole = 1.0f / (float)(cmask + 1u);  // a power of two: exact
             for (int tier = 0; tier < 2; ++tier) {
                 if (tier == 1) {  // the rows' own widths
+                    load_keys();
                     if (tid < kBkRows) {
                         rowmin[tid] = 0xFFFFFFFFu;
                         rowmax[tid] = 0u;
                     }
                     for (int i = tid; i < (E + 1) / 2; i += T) cntw[i] = 0u;
                     __syncthreads();
-#pragma unroll 4
-                    for (int p = tid; p < E; p += T) {
-                        const unsigned k = bk_key24(rec[p].x, cbits), r = k >> cbits, c = k & cmask;
+#pragma unroll
+                    for (int j = 0; j < kPer; ++j) {
+                        if (tid + j * T >= E) break;
+                        const unsigned r = kk[j] >> cbits, c = kk[j] & cmask;
                         atomicMin(&rowmin[r], c);
                         atomicMax(&rowmax[r], c);
                     }
@@ -659,9 +671,10 @@ __global__ void __launch_bounds__(bk_place_threads<kCap>(), bk_place_per_sm<kCap
                     __syncthreads();
                 }
                 big = false;
-#pragma unroll 4
-                for (int p = tid; p < E; p += T) {
-                    const unsigned k = bk_key24(rec[p].x, cbits), r = k >> cbits, c = k & cmask;
+#pragma unroll
+                for (int j = 0; j < kPer; ++j) {
+                    if (tid + j * T >= E) break;
+                    const unsigned r = kk[j] >> cbits, c = kk[j] & cmask;
                     const unsigned ri = rowinfo[r], L = ri >> 16;
                     const float f = tier == 0 ? (float)c * ((float)L * whole)
                                               : (float)(c - rowmin[r]) * __uint_as_float(rowmax[r]);
@@ -670,7 +683,7 @@ __global__ void __launch_bounds__(bk_place_threads<kCap>(), bk_place_per_sm<kCap
                     const unsigned sh = (bb & 1u) << 4;
                     const unsigned rank = (atomicAdd(&cntw[bb >> 1], 1u << sh) >> sh) & 0xFFFFu;
                     big |= rank >= kBinMax;
-                    ord[p] = rank << kRankAt | bb << kBkColBits | c;  // (the keys stay for a second try)
+                    kk[j] = rank << kRankAt | bb << kBkColBits | c;  // (a second try reads the keys again)
                 }
                 big = __syncthreads_or(big);
                 if (!big) break;
@@ -697,9 +710,6 @@ __global__ void __launch_bounds__(bk_place_threads<kCap>(), bk_place_per_sm<kCap
             if (lane >= o) incl += y;
         }
         if (lane == 31) sh_part[warp] = incl;
-        // the packed words take the place of the keys
-#pragma unroll 4
-        for (int p = tid; p < E; p += T) rec[p].x = ord[p];
         __syncthreads();
         unsigned run = incl - sum;
 #pragma unroll
@@ -710,9 +720,11 @@ __global__ void __launch_bounds__(bk_place_threads<kCap>(), bk_place_per_sm<kCap
             run = lo + (c >> 16);
         }
         __syncthreads();
-#pragma unroll 4
-        for (int p = tid; p < E; p += T) {
-            const unsigned v = rec[p].x, rank = v & kRankMask;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int p = tid + j * T;
+            if (p >= E) break;
+            const unsigned v = kk[j], rank = v & kRankMask;
             ord[start[(v >> kBkColBits) & kIdxMask] + (rank >> kRankAt)] = rank | (v & kColMask) << kIdx | (unsigned)p;
         }
         if (tid == 0) ord[E] = 0u;  // the end of the last bin
