@@ -11,9 +11,10 @@
 // One sweep of the keys counts every pass's digits; then each pass is one
 // launch that reads and writes every element once (a decoupled look-back per
 // digit; Adinets and Merrill, "Onesweep", 2022):
-//  * a tile ranks its elements by digit: each warp takes 32 at a time among
-//    the lanes holding the same digit (one ballot per digit bit, running
-//    counts per (warp, digit) in shared memory), in element order;
+//  * a tile ranks its elements by digit: each warp takes 32 at a time and ranks
+//    them among the lanes holding the same digit, which set their bits in a word
+//    of the (warp, digit) in shared memory (running counts beside it), in
+//    element order;
 //  * per digit, one thread publishes the tile's count and looks back over the
 //    earlier tiles' words for the digit's first output position;
 //  * the tile is put in digit order in shared memory and written out in runs.

@@ -295,10 +295,11 @@ int hyd_cuda_autotune_histogram(int64_t n, int64_t bins, int reps, int* best, do
  * scan / scan_inclusive / scanr / scanr_inclusive with (+) and initial value
  * `init` (Lowering.hs:3563-3612; the reference runs them as a serial fold):
  * reverse != 0 walks index n-1-k; inclusive != 0 writes the accumulator after
- * adding element k, otherwise before.  int64: single-pass decoupled look-back,
- * bit-exact.  float64: single pass, deterministic (a fixed warp scan within
- * blocks of 32 tiles, a left fold of the block totals): run-to-run identical
- * and within 1e-12 of the prefix sums of |x| of the serial fold. */
+ * adding element k, otherwise before.  int64: the sums of one range per warp,
+ * then the scans; bit-exact.  float64: the same up to 2^17 elements, above that
+ * a single pass (a fixed warp scan within blocks of 32 tiles, a left fold of
+ * the block totals); every order is fixed by n, so results are run-to-run
+ * identical, and within 1e-12 of the prefix sums of |x| of the serial fold. */
 int hyd_cuda_scan_i64(const int64_t* in, int64_t* out, int64_t n, int64_t init, int reverse,
                       int inclusive, void* stream);
 int hyd_cuda_scan_f64(const double* in, double* out, int64_t n, double init, int reverse,
