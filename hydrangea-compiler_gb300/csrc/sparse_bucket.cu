@@ -1003,7 +1003,9 @@ __global__ void __launch_bounds__(kBkThreads) bk_bucket_kernel(const BkInst* __r
 // chunk of one instance's rows, counting-sorts them by length (256 bins,
 // lengths above 255 share the last) in shared memory, and gives each lane one
 // row of every group of 32 consecutive rows in that order.  A lane reads its
-// row 4 entries at a time with 16-byte loads, ahead of the (in-order) chain.
+// row 4 entries at a time, ahead of the (in-order) chain.  Requests to L2 and
+// their latency bound it, most of them x (2.9e8 entries: 2.06 ms with the values
+// by 16-byte loads through L1 and x past it, 1.87 ms so).
 // Chunks have 256 rows, halved down to 32 while the batch has fewer chunks than
 // the chip has resident warps.  Whole pipeline: one instance of 2^13.5 to
 // 2^16.3 rows 197 -> 153 us, 24 of 2^10 to 2^14 rows 283 -> 232, 4 of 2^16 to
@@ -1091,23 +1093,26 @@ __global__ void __launch_bounds__(kSpWarps * 32, kSpPerSm)
             const int* __restrict__ rc = cols + a;
             const double* __restrict__ rv = vals + a;
             double acc = 0.0;
-            // x is gathered through L2 only, so that the random x lines do not
-            // evict the lanes' sequential row streams
-            auto xat = [&](unsigned c) { return c < ncols ? __ldcg(x + c) : 0.0; };
+            // x is gathered through L1: the values pass it by, a whole sector per
+            // load, and leave it to the columns' sectors, of two loads each, and x
+            auto xat = [&](unsigned c) { return c < ncols ? __ldg(x + c) : 0.0; };
             // entries one at a time until the columns are 16-byte aligned, then
-            // 4 per step: the columns by one 16-byte load, the values by two
-            // when they are 16-byte aligned too (the parity is fixed per row);
-            // the fma chain keeps the row's order throughout
+            // 4 per step: the columns by one 16-byte load, the values by one of
+            // 32 bytes or two of 16 where their alignment (fixed per row) lets
+            // it; the fma chain keeps the row's order throughout
             int k = 0;
             while (k < L && (reinterpret_cast<uintptr_t>(rc + k) & 15)) {
                 acc = fma(rv[k], xat((unsigned)rc[k]), acc);
                 ++k;
             }
-            const bool v16 = (reinterpret_cast<uintptr_t>(rv + k) & 15) == 0;
+            const unsigned va = (unsigned)reinterpret_cast<uintptr_t>(rv + k) & 31u;
             for (; k + 4 <= L; k += 4) {
                 const int4 c4 = *reinterpret_cast<const int4*>(rc + k);
                 double v0, v1, v2, v3;
-                if (v16) {
+                if (va == 0) {
+                    const f64x4 p = ldg_stream_f64x4(rv + k);
+                    v0 = p.x; v1 = p.y; v2 = p.z; v3 = p.w;
+                } else if (va == 16) {
                     const double2 p = *reinterpret_cast<const double2*>(rv + k);
                     const double2 q = *reinterpret_cast<const double2*>(rv + k + 2);
                     v0 = p.x; v1 = p.y; v2 = q.x; v3 = q.y;

@@ -50,6 +50,25 @@ def test_chunk_sizes(hc, orc, dev, chunk, off):
     _check(hc, orc, dev, insts)
 
 
+@pytest.mark.parametrize("vals_off", [0, 1, 2, 3])
+@pytest.mark.parametrize("cols_off", [0, 1, 2])
+def test_output_alignments(hc, dev, vals_off, cols_off):
+    """The SpMV reads the CSR by 4, 16 or 32 bytes, as it is aligned: the same bits."""
+    rng = np.random.default_rng(5)
+    n, ncols, r, c = _random(700, 800, 20_011, rng)
+    desc = np.array([[n, ncols, len(r)]], dtype=np.int64)
+    args = [torch.from_numpy(a).to(dev) for a in (r, c, rng.uniform(-1, 1, len(r)), rng.uniform(-1, 1, ncols))]
+    want = hc.batched_coo_csr_spmv(desc, *args)
+    got = [torch.empty(n + 1, dtype=torch.int64, device=dev),
+           torch.empty(len(r) + cols_off, dtype=torch.int32, device=dev)[cols_off:],
+           torch.empty(len(r) + vals_off, dtype=torch.float64, device=dev)[vals_off:],
+           torch.empty(n, dtype=torch.float64, device=dev)]
+    hc.call("hyd_cuda_batched_coo_csr_spmv_f64", 1, desc.ctypes.data, *(hc.ptr(t) for t in args + got),
+            hc.stream_handle(None))
+    hc.check(hc.device_check())
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 def test_invalid_column_is_reported(hc, orc, dev):
     rng = np.random.default_rng(4)
     n, ncols, r, c = _random(3000, 500, 13_000, rng)
