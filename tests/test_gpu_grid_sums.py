@@ -90,3 +90,27 @@ def test_jacobi1d_mean(hc, dev, values):
     with np.errstate(all="ignore"):
         want = ((np.concatenate([x[:1], x[:-1]]) + x) + np.concatenate([x[1:], x[-1:]])) / 3.0
     _same(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("dt", [1.0, 0.5])
+@pytest.mark.parametrize("values", KINDS)
+def test_gray_scott_laplacians(hc, dev, values, dt):
+    rng = np.random.default_rng(2)
+    u, v = (_values(values, 97 * 130, rng).reshape(97, 130) for _ in range(2))
+    p = hc.GrayScott(dt=dt)
+    src = [torch.from_numpy(x).to(dev) for x in (u, v)]
+    out = [torch.empty_like(x) for x in src]
+    hc.gray_scott_step(*src, *out, params=p)
+
+    def lap(x):
+        return ((np.roll(x, 1, 0) + np.roll(x, -1, 0)) + np.roll(x, 1, 1)) + np.roll(x, -1, 1) - 4.0 * x
+
+    with np.errstate(all="ignore"):
+        uvv = u * v * v
+        want = (u + dt * ((p.du * lap(u) - uvv) + p.feed * (1.0 - u)), v + dt * ((p.dv * lap(v) + uvv) - (p.feed + p.kill) * v))
+    # 4x is exact unless it overflows
+    fine = np.ones_like(u, dtype=bool)
+    for x in (u, v):
+        fine &= ~(np.abs(x) >= 1e307)
+    for got, w in zip(out, want):
+        _same(np.where(fine, got.cpu().numpy(), 0.0), np.where(fine, w, 0.0))
