@@ -60,9 +60,9 @@ struct MixReq {
 
 __device__ __forceinline__ double lap_body(double a, double b, double c, double d, double e) {
     // a + b + c + d + (e * -4.0), evaluated as the C backend does (4e exact);
-    // the first two additions on the integer pipe (exact, FP64 fallback)
-    const double t3 = __dadd_rn(dadd_pos(dadd_pos(a, b), c), d);
-    return __fma_rn(e, -4.0, t3);
+    // the sum of four on the integer pipe (exact, FP64 fallback)
+    // (eight requests of 4096^2 at once: 1060 -> 950 us)
+    return __fma_rn(e, -4.0, dsum4_pos(a, b, c, d));
 }
 
 __device__ __forceinline__ double block_sum_fixed(double v, double* sh) {

@@ -114,3 +114,41 @@ def test_gray_scott_laplacians(hc, dev, values, dt):
         fine &= ~(np.abs(x) >= 1e307)
     for got, w in zip(out, want):
         _same(np.where(fine, got.cpu().numpy(), 0.0), np.where(fine, w, 0.0))
+
+
+def _five(kind, p):
+    """One step from a field padded by one on every side."""
+    t = ((p[:-2, 1:-1] + p[2:, 1:-1]) + p[1:-1, :-2]) + p[1:-1, 2:]
+    u = p[1:-1, 1:-1]
+    return [t + u * -4.0, t / 4.0, u + 0.1 * (t - 4.0 * u), (t + u) / 5.0][kind]
+
+
+@pytest.mark.parametrize("boundary,pad", [(1, dict(mode="wrap")), (2, dict(mode="reflect")),
+                                          (3, dict(mode="constant", constant_values=0.25))])
+@pytest.mark.parametrize("values", KINDS)
+def test_boundary_bodies(hc, dev, values, boundary, pad):
+    u = _values(values, 75 * 101, np.random.default_rng(boundary)).reshape(75, 101)
+    src = torch.from_numpy(u).to(dev)
+    fine = ~(np.abs(u) >= 1e307)  # 4e is exact unless it overflows
+    with np.errstate(all="ignore"):
+        for kind in range(4):
+            out = torch.empty_like(src)
+            hc.stencil2d_bnd(kind, boundary, src, out, fill=0.25)
+            keep = fine if kind in (0, 2) else np.ones_like(fine)
+            _same(np.where(keep, out.cpu().numpy(), 0.0), np.where(keep, _five(kind, np.pad(u, 1, **pad)), 0.0))
+
+
+@pytest.mark.parametrize("values", KINDS)
+def test_served_laplacian(hc, dev, values):
+    u = _values(values, 130 * 257, np.random.default_rng(3)).reshape(130, 257)
+    src = torch.from_numpy(u).to(dev)
+    out = torch.empty_like(src)
+    torch.cuda.synchronize()
+    srv = hc.Server(budget_bytes=1 << 30)
+    st, ticket = srv.submit(hc.Request(hc.REQ_LAPLACIAN, 130, 257, src.data_ptr(), None, None, None, out.data_ptr()))
+    assert st == hc.OK
+    srv.wait(ticket)
+    fine = ~(np.abs(u) >= 1e307)
+    with np.errstate(all="ignore"):
+        want = _five(0, np.pad(u, 1, mode="edge"))
+    _same(np.where(fine, out.cpu().numpy(), 0.0), np.where(fine, want, 0.0))
