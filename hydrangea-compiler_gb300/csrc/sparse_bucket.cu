@@ -50,7 +50,7 @@ constexpr int kSplitThreads = 512;
 constexpr int kSplitPerSm = 2;
 constexpr int kSplitPer = 12;                // entries per thread of the split
 constexpr int kTileEntries = kSplitThreads * kSplitPer;  // entries per count/split work item
-constexpr int kCountEntries = kBkThreads * 12;           // entries the count loads at once
+static_assert(kTileEntries % kBkThreads == 0, "whole rounds of the count");
 constexpr int kMaxSmemBuckets = 4096;        // per instance (2^18 rows)
 
 struct BkInst {
@@ -128,29 +128,29 @@ __global__ void __launch_bounds__(kBkThreads, kCountPerSm) bk_count_kernel(const
         }
         const bool smem = cur_nb <= kMaxSmemBuckets;
         const long long t0 = (long long)w.tile * kTileEntries;
-        const long long t1 = t0 + kTileEntries < I.nnz ? t0 + kTileEntries : I.nnz;
+        const int tn = (int)(t0 + kTileEntries < I.nnz ? kTileEntries : I.nnz - t0);
+        const int* __restrict__ rows = I.rows + t0;
+        const unsigned nrows = (unsigned)I.nrows;  // below 2^31: a negative row is above it too
         // all of this thread's rows first (read-only loads, all in flight at
         // once), then the counting: a load next to an atomic would otherwise
         // wait for it, one memory round trip per entry
-        for (long long c0 = t0; c0 < t1; c0 += kCountEntries) {
-            int rr[kCountEntries / kBkThreads];
+        unsigned rr[kTileEntries / kBkThreads];
+        auto count = [&](bool full) {  // columns are checked by the split, which reads them anyway
 #pragma unroll
-            for (int j = 0; j < kCountEntries / kBkThreads; ++j) {
-                const long long k = c0 + threadIdx.x + (long long)j * kBkThreads;
-                rr[j] = k < t1 ? __ldg(I.rows + k) : INT_MIN;
+            for (int j = 0; j < kTileEntries / kBkThreads; ++j) {
+                const int q = threadIdx.x + j * kBkThreads;
+                if (full || q < tn) rr[j] = (unsigned)__ldg(rows + q);
             }
 #pragma unroll
-            for (int j = 0; j < kCountEntries / kBkThreads; ++j) {
-                const int r = rr[j];  // columns are checked by the split, which reads them anyway
-                if (r == INT_MIN && c0 + threadIdx.x + (long long)j * kBkThreads >= t1) continue;
-                if (r < 0 || r >= I.nrows) {
-                    bad = true;
-                    continue;
-                }
-                if (smem) atomicAdd(&hist[r >> kBkShift], 1u);
-                else atomicAdd(&bcount[I.bucket_base + (r >> kBkShift)], 1u);
+            for (int j = 0; j < kTileEntries / kBkThreads; ++j) {
+                if (!full && threadIdx.x + j * kBkThreads >= tn) break;
+                if (rr[j] >= nrows) bad = true;
+                else if (smem) atomicAdd(&hist[rr[j] >> kBkShift], 1u);
+                else atomicAdd(&bcount[cur_base + (rr[j] >> kBkShift)], 1u);
             }
-        }
+        };
+        if (tn == kTileEntries) count(true);
+        else count(false);
     }
     __syncthreads();
     flush();
