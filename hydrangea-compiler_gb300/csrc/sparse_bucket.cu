@@ -1005,7 +1005,8 @@ __global__ void __launch_bounds__(kBkThreads) bk_bucket_kernel(const BkInst* __r
 // row of every group of 32 consecutive rows in that order.  A lane reads its
 // row 4 entries at a time, ahead of the (in-order) chain.  Requests to L2 and
 // their latency bound it, most of them x (2.9e8 entries: 2.06 ms with the values
-// by 16-byte loads through L1 and x past it, 1.87 ms so).
+// by 16-byte loads through L1 and x past it, 1.89 ms so; one loop per alignment
+// of the values, as a choice inside the loop cost 0.07 ms).
 // Chunks have 256 rows, halved down to 32 while the batch has fewer chunks than
 // the chip has resident warps.  Whole pipeline: one instance of 2^13.5 to
 // 2^16.3 rows 197 -> 153 us, 24 of 2^10 to 2^14 rows 283 -> 232, 4 of 2^16 to
@@ -1105,26 +1106,31 @@ __global__ void __launch_bounds__(kSpWarps * 32, kSpPerSm)
                 acc = fma(rv[k], xat((unsigned)rc[k]), acc);
                 ++k;
             }
-            const unsigned va = (unsigned)reinterpret_cast<uintptr_t>(rv + k) & 31u;
-            for (; k + 4 <= L; k += 4) {
-                const int4 c4 = *reinterpret_cast<const int4*>(rc + k);
-                double v0, v1, v2, v3;
-                if (va == 0) {
-                    const f64x4 p = ldg_stream_f64x4(rv + k);
-                    v0 = p.x; v1 = p.y; v2 = p.z; v3 = p.w;
-                } else if (va == 16) {
-                    const double2 p = *reinterpret_cast<const double2*>(rv + k);
-                    const double2 q = *reinterpret_cast<const double2*>(rv + k + 2);
-                    v0 = p.x; v1 = p.y; v2 = q.x; v3 = q.y;
-                } else {
-                    v0 = rv[k]; v1 = rv[k + 1]; v2 = rv[k + 2]; v3 = rv[k + 3];
-                }
+            auto four = [&](double v0, double v1, double v2, double v3, const int4& c4) {
                 const double x0 = xat((unsigned)c4.x), x1 = xat((unsigned)c4.y);
                 const double x2 = xat((unsigned)c4.z), x3 = xat((unsigned)c4.w);
                 acc = fma(v0, x0, acc);
                 acc = fma(v1, x1, acc);
                 acc = fma(v2, x2, acc);
                 acc = fma(v3, x3, acc);
+            };
+            const unsigned va = (unsigned)reinterpret_cast<uintptr_t>(rv + k) & 31u;
+            if (va == 0) {
+                for (; k + 4 <= L; k += 4) {
+                    const int4 c4 = *reinterpret_cast<const int4*>(rc + k);
+                    const f64x4 p = ldg_stream_f64x4(rv + k);
+                    four(p.x, p.y, p.z, p.w, c4);
+                }
+            } else if (va == 16) {
+                for (; k + 4 <= L; k += 4) {
+                    const int4 c4 = *reinterpret_cast<const int4*>(rc + k);
+                    const double2 p = *reinterpret_cast<const double2*>(rv + k);
+                    const double2 q = *reinterpret_cast<const double2*>(rv + k + 2);
+                    four(p.x, p.y, q.x, q.y, c4);
+                }
+            } else {
+                for (; k + 4 <= L; k += 4)
+                    four(rv[k], rv[k + 1], rv[k + 2], rv[k + 3], *reinterpret_cast<const int4*>(rc + k));
             }
             for (; k < L; ++k) acc = fma(rv[k], xat((unsigned)rc[k]), acc);
             I.y[r0 + i] = acc;
