@@ -198,8 +198,9 @@ __global__ void bk_widen_kernel(const unsigned* __restrict__ c, long long* __res
 // Written from COO order, a lane's record went to a bucket of its own: 32 write
 // requests of one sector per warp instruction, and those bounded the kernel.
 // 2.9e8 entries in 512 instances of 2^10 to 2^18 rows: 3.88 ms so (8192-entry
-// tiles), 2.77 ms in bucket order, 2.49 ms with the prefetch (reading and
-// writing 32 bytes per entry takes 1.37 ms at the copy rate).  Two blocks of
+// tiles), 2.77 ms in bucket order, 2.49 ms with the prefetch, 2.27 ms since the
+// scan and the reservations stop at the instance's last bucket instead of 4096
+// (reading and writing 32 bytes per entry takes 1.37 ms at the copy rate).  Two blocks of
 // 512 threads with 6144 entries each fill an SM's shared memory; one block of
 // 1024 threads with 12288, whose runs are twice as long, has no second block to
 // fill its barriers and took 1% more of the whole pipeline.
@@ -219,9 +220,8 @@ __global__ void __launch_bounds__(kSplitThreads, kSplitPerSm) bk_split_kernel(
     const BkInst* __restrict__ inst, const BkItem* __restrict__ items, unsigned nitems, unsigned* cursor,
     const long long* __restrict__ bstart, unsigned* __restrict__ bfill, uint4* __restrict__ rec_out, unsigned* err) {
     extern __shared__ __align__(16) double split_vals[];          // [kTileEntries], COO order
-    unsigned* skey = (unsigned*)(split_vals + kTileEntries);      // [kTileEntries], bucket order
-    unsigned* spos = skey + kTileEntries;                         // [kTileEntries], bucket << 14 | position
-    unsigned* hist = spos + kTileEntries;                         // [kMaxSmemBuckets + 1]
+    uint2* sent = (uint2*)(split_vals + kTileEntries);  // [kTileEntries], bucket order: key; bucket << 14 | position
+    unsigned* hist = (unsigned*)(sent + kTileEntries);  // [kMaxSmemBuckets + 1]
     __shared__ unsigned warp_sum[kSplitThreads / 32];
     __shared__ unsigned sh_it[2];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -238,6 +238,9 @@ __global__ void __launch_bounds__(kSplitThreads, kSplitPerSm) bk_split_kernel(
         const BkItem w = items[it];
         const BkInst I = inst[w.inst];
         const bool smem = I.nbuckets <= kMaxSmemBuckets;
+        const int nb = smem ? (int)I.nbuckets : 0;
+        // threads of the counts' scan, whose counts reach one bucket past the last
+        const int threads_used = nb < kMaxSmemBuckets ? nb / kSplitBins + 1 : kSplitThreads;
         const long long t0 = (long long)w.tile * kTileEntries;
         const int tn = (int)(t0 + kTileEntries < I.nnz ? kTileEntries : I.nnz - t0);
         // the rows and columns of all this thread's entries first (read-only
@@ -271,7 +274,7 @@ __global__ void __launch_bounds__(kSplitThreads, kSplitPerSm) bk_split_kernel(
             }
         }
         if (smem)
-            for (int b = threadIdx.x; b <= kMaxSmemBuckets / 4; b += kSplitThreads)
+            for (int b = threadIdx.x; b < threads_used * (kSplitBins / 4); b += kSplitThreads)
                 ((uint4*)hist)[b] = make_uint4(0u, 0u, 0u, 0u);
         __syncthreads();
 #pragma unroll
@@ -306,12 +309,13 @@ __global__ void __launch_bounds__(kSplitThreads, kSplitPerSm) bk_split_kernel(
             __syncthreads();
             continue;
         }
-        // exclusive scan of the counts in place; hist[kMaxSmemBuckets] = all
+        // exclusive scan of the counts in place; hist[nb] = all
         {
             unsigned c[kSplitBins], sum = 0u;
 #pragma unroll
             for (int i = 0; i < kSplitBins; i += 4) {
-                const uint4 v = ((const uint4*)hist)[(threadIdx.x * kSplitBins + i) >> 2];
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                if ((int)threadIdx.x < threads_used) v = ((const uint4*)hist)[(threadIdx.x * kSplitBins + i) >> 2];
                 c[i] = v.x, c[i + 1] = v.y, c[i + 2] = v.z, c[i + 3] = v.w;
                 sum += v.x + v.y + v.z + v.w;
             }
@@ -333,12 +337,12 @@ __global__ void __launch_bounds__(kSplitThreads, kSplitPerSm) bk_split_kernel(
                 v.y = run, run += c[i + 1];
                 v.z = run, run += c[i + 2];
                 v.w = run, run += c[i + 3];
-                ((uint4*)hist)[(threadIdx.x * kSplitBins + i) >> 2] = v;
+                if ((int)threadIdx.x < threads_used) ((uint4*)hist)[(threadIdx.x * kSplitBins + i) >> 2] = v;
             }
             if (threadIdx.x == kSplitThreads - 1) hist[kMaxSmemBuckets] = run;
         }
         __syncthreads();
-        const int total = (int)hist[kMaxSmemBuckets];
+        const int total = (int)hist[nb];
         // reserve this tile's run in every non-empty bucket; the atomics of
         // one thread are independent, and their results are first needed after
         // the placing below
@@ -346,35 +350,35 @@ __global__ void __launch_bounds__(kSplitThreads, kSplitPerSm) bk_split_kernel(
 #pragma unroll
         for (int i = 0; i < kSplitBins; ++i) {
             const int b = threadIdx.x + i * kSplitThreads;
-            const unsigned c = hist[b + 1] - hist[b];
+            const unsigned c = b < nb ? hist[b + 1] - hist[b] : 0u;
             first[i] = c ? (unsigned)bstart[I.bucket_base + b] + atomicAdd(&bfill[I.bucket_base + b], c) : 0u;
         }
 #pragma unroll
         for (int j = 0; j < kSplitPer; ++j) {
             if (bucket[j] < 0) continue;
             const int p = (int)(hist[bucket[j]] + rank[j]);
-            skey[p] = key[j];
-            spos[p] = ((unsigned)bucket[j] << kSplitPosBits) | (unsigned)(threadIdx.x + j * kSplitThreads);
+            sent[p] = make_uint2(key[j], ((unsigned)bucket[j] << kSplitPosBits) |
+                                             (unsigned)(threadIdx.x + j * kSplitThreads));
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();  // every place is read and every value has landed
 #pragma unroll
         for (int i = 0; i < kSplitBins; ++i) {
             const int b = threadIdx.x + i * kSplitThreads;
-            hist[b] = first[i] - hist[b];  // batch-wide slots (< 2^32, checked on the host), modulo 2^32
+            if (b < nb) hist[b] = first[i] - hist[b];  // batch-wide slots (< 2^32, checked on the host), modulo 2^32
         }
         __syncthreads();
 #pragma unroll
         for (int j = 0; j < kSplitPer; ++j) {
             const int p = threadIdx.x + j * kSplitThreads;
             if (p >= total) break;
-            const unsigned e = spos[p];
-            const unsigned q = e & ((1u << kSplitPosBits) - 1u);
+            const uint2 e = sent[p];
+            const unsigned q = e.y & ((1u << kSplitPosBits) - 1u);
             const double v = split_vals[q];
             // one 16-byte record: the key, the entry's COO position (orders
             // equal (row, col) keys) and the value
-            rec_out[hist[e >> kSplitPosBits] + (unsigned)p] =
-                make_uint4(skey[p], (unsigned)t0 + q, (unsigned)__double2loint(v), (unsigned)__double2hiint(v));
+            rec_out[hist[e.y >> kSplitPosBits] + (unsigned)p] =
+                make_uint4(e.x, (unsigned)t0 + q, (unsigned)__double2loint(v), (unsigned)__double2hiint(v));
         }
         __syncthreads();
     }
