@@ -170,7 +170,13 @@ struct GuardedScatterI64Source {
 // then the scalar remainder.  Groups whose routes are all in range go to
 // fast(bin, val) with no per-element check; everything else goes to
 // checked(bin, val), which must handle an out-of-range bin.
-template <class Src, class F, class FF>
+// kDeep: the next two groups are loaded before the current two are applied.
+// That pays where the loads bound the kernel, with a mask for a route and the
+// bins in shared memory (2^27 elements, 64 bins 171 -> 165 us, 4096 bins 173 ->
+// 166; 2^26 elements, 16384 bins 144 -> 133); not with a remainder per element
+// (2e7 elements, 1000 bins: 36.9 us without, 37.3 with), nor beside global
+// atomics (4e6 elements, 65536 bins: 30.8 and 32.8), and other sources spill.
+template <bool kDeep, class Src, class F, class FF>
 __device__ __forceinline__ void for_each_element(const Src& src, int64_t n, bool vec, long long bins,
                                                  F checked, FF fast) {
     const int64_t S = (int64_t)gridDim.x * blockDim.x;
@@ -179,6 +185,31 @@ __device__ __forceinline__ void for_each_element(const Src& src, int64_t n, bool
     if (vec) {
         const int64_t nv = n >> 2;
         int64_t v = t;
+        if constexpr (kDeep) {
+            auto group = [&](const typename Src::Raw& q) {
+                long long b[4];
+                u64 w[4];
+                if (src.four(q, bins, b, w)) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) fast(b[k], w[k]);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) checked(b[k], w[k]);
+                }
+            };
+            if (v + S < nv) {
+                typename Src::Raw q0 = src.load4(v), q1 = src.load4(v + S);
+                for (v += 2 * S; v + S < nv; v += 2 * S) {
+                    const typename Src::Raw n0 = src.load4(v), n1 = src.load4(v + S);
+                    group(q0);
+                    group(q1);
+                    q0 = n0;
+                    q1 = n1;
+                }
+                group(q0);
+                group(q1);
+            }
+        }
         for (; v + S < nv; v += 2 * S) {
             long long b0[4], b1[4];
             u64 v0[4], v1[4];
@@ -241,7 +272,7 @@ __global__ void __launch_bounds__(kHistThreads, 2)
     unsigned* lo = sh_limbs + (((threadIdx.x >> 5) * 2 + ((threadIdx.x >> 4) & 1)) % copies) * bins * 2;
     unsigned* hi = lo + bins;
     bool bad = false;
-    for_each_element(
+    for_each_element<Src::kMaskRoute>(
         src, n, vec, bins,
         [&](long long b, u64 v) {
             const bool ok = (u64)b < (u64)bins;
@@ -953,7 +984,7 @@ __global__ void __launch_bounds__(kHistThreads, 2)
     hist_global_kernel(Src src, int64_t n, bool vec, long long bins, u64* __restrict__ hist,
                        unsigned* err) {
     bool bad = false;
-    for_each_element(
+    for_each_element<false>(
         src, n, vec, bins,
         [&](long long b, u64 v) {
             const bool ok = (u64)b < (u64)bins;
