@@ -25,7 +25,7 @@
 // segments of 2^U(0,16), 695 -> 317 us (3.4 TB/s); segments of 2^U(0,5), 783 ->
 // 579 us; of one value each, 1136 -> 1014 us.  Before, tiles of 4096 values took
 // 1.6 FP64 operations per value and waited for a look-back.  SpMV, 2^20 rows of
-// Zipf length, 12.9e6 entries: 198 -> 107 us; 8 lanes per row spent about seven
+// Zipf length, 12.9e6 entries: 198 -> 109 us; 8 lanes per row spent about seven
 // FP64 lane slots per entry.  Three blocks per SM (80 registers) beat four (64
 // and spills): 1014 against 1327 us on one-value segments.
 //
@@ -44,7 +44,7 @@ constexpr int kSegT = 256;
 constexpr int kSegWarps = kSegT / 32;
 constexpr int kSegPer = 8;                  // consecutive values per lane
 constexpr int kSegC = 32 * kSegPer;         // values per chunk
-constexpr int kSegCounterWord = 240;              // stream counters: +0 invalid offsets, +1 finished blocks
+constexpr int kSegCounterWord = 240;  // stream counters: +0 invalid offsets, +1 finished blocks, +2 rows by lanes
 // where a chunk's sum i sits: free of bank conflicts for a lane's 8 consecutive values
 __device__ __forceinline__ int seg_slot(int i) { return i ^ ((i >> 4) & 7); }
 
@@ -65,12 +65,14 @@ struct SegPartials {
     int64_t* closes;  // the boundary that ends that first piece, -1: none, or the piece is empty
     unsigned* bad;
     unsigned* done;
+    unsigned* by_lanes;  // SpMV: the second kernel takes the rows by lanes, the first does nothing
 };
 
 // ---- what a position of the array contributes ---------------------------------
 // Plain values; mac() adds one to a running sum.
 template <class T>
 struct SegPlain {
+    static constexpr bool kRows = false;
     static constexpr int kCtasPerSm = 3, kUnroll = 2;  // resident blocks; chunks in flight per warp
     static constexpr int kStageBytes = 0;
     static constexpr int kPos = kSegC + 32;  // boundaries of a chunk kept in shared memory; more are read again
@@ -106,6 +108,7 @@ template <class C>
 struct SegProduct {
     // chunks are staged in shared memory by cp.async, two ahead: the entries'
     // latency is off the chain entries -> x -> sums
+    static constexpr bool kRows = true;  // rows of even length may go by lanes
     static constexpr int kCtasPerSm = 3, kUnroll = 1;
     static constexpr int kStageBytes = kSegC * (8 + (int)sizeof(C));  // values, then columns
     // none: three blocks of two staged chunks per warp just fit the 196 KB
@@ -282,6 +285,70 @@ __device__ __forceinline__ void warp_lower_bound2(const int64_t* __restrict__ a,
 // with the range (lo, hi] takes the boundaries in it, the first warp those at
 // the array's very start too.  Positions and boundary numbers below are
 // relative to the warp's lo and first boundary b0.
+// ---- rows of even length --------------------------------------------------------
+// Where the rows of an SpMV are about equally long, 8 lanes per row waste little
+// and need no search, no scan and no staging.  Only the device knows the lengths:
+// every block looks at the same 256 groups of four neighbouring rows (what a warp
+// takes, with 8 lanes each) and so comes to the same answer.
+//
+// A group costs as many FP64 warp instructions as its longest row has eights of
+// entries, and three to combine.  Times in ns, fitted to measurements: by lanes
+// 5000 plus 0.0163 per row and instruction plus 0.002 per entry; by entries 22000
+// plus 0.008 per row plus 0.0054 per entry.  Uneven rows (the groups' longest well
+// above the average) are always split by entries.  2^20 rows, int64 columns, by 8
+// lanes without asking, by entries without asking, and now: 3 entries each 74, 47
+// and 52 us; 8 74, 68 and 77; 12 108, 96 and 101; 32 158, 200 and 162; 100 492, 580
+// and 494; Zipf
+// lengths 189, 102 and 105.
+// Called by all threads of a block of 256; sh: eight words.
+__device__ __forceinline__ bool seg_rows_by_lanes(const int64_t* __restrict__ row_ptr, int64_t nrows, unsigned* sh) {
+    const int64_t r = (int64_t)threadIdx.x * (nrows >> 2) / kSegT * 4;
+    const float rows = (float)nrows, entries = (float)(row_ptr[nrows] - row_ptr[0]);
+    int64_t p = row_ptr[r];
+    unsigned longest = 0;
+#pragma unroll
+    for (int k = 1; k <= 4; ++k) {
+        const int64_t e = r + k <= nrows ? row_ptr[r + k] : p, l = e - p;
+        const unsigned n = l < 0 ? 0u : (l > (1 << 20) ? 1u << 17 : (unsigned)(l + 7) >> 3);
+        longest = n > longest ? n : longest;
+        p = e;
+    }
+    longest = __reduce_add_sync(0xffffffffu, longest);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = longest;
+    __syncthreads();
+    unsigned sum = 0;
+#pragma unroll
+    for (int w = 0; w < kSegWarps; ++w) sum += sh[w];
+    __syncthreads();
+    const float eights = (float)sum * (1.0f / kSegT);
+    if (eights > entries / rows * (1.25f / 8.0f) + 1.25f) return false;
+    return 5000.0f + 0.0163f * rows * (eights + 3.0f) + 0.002f * entries < 22000.0f + 0.008f * rows + 0.0054f * entries;
+}
+
+// The rows by 8 lanes each, the sums of spmv_csr_kernel<8>, bit for bit.
+template <class Src>
+__device__ __forceinline__ void seg_rows(const Src& src, double* __restrict__ y, unsigned* err) {
+    const int sub = threadIdx.x & 7, group = (threadIdx.x & 31) >> 3;
+    const int64_t warps = (int64_t)gridDim.x * kSegWarps;
+    bool bad = false;
+    for (int64_t rb = ((int64_t)blockIdx.x * kSegWarps + (threadIdx.x >> 5)) * 4; rb < src.nrows; rb += warps * 4) {
+        const int64_t r = rb + group;
+        double acc = 0.0;
+        if (r < src.nrows) {
+            const long long s = src.row_ptr[r], e = src.row_ptr[r + 1];
+            for (long long k = s + sub; k < e; k += 8) {
+                const long long c = (long long)__ldg(src.cols + k);
+                if ((unsigned long long)c < (unsigned long long)src.ncols) acc = fma(__ldg(src.vals + k), __ldg(src.x + c), acc);
+                else bad = true;
+            }
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, 8);
+        if (sub == 0 && r < src.nrows) y[r] = acc;
+    }
+    if (bad) raise_error(err, ERRBIT_BOUNDS);
+}
+
 template <class T, class Src>
 __global__ void __launch_bounds__(kSegT, Src::kCtasPerSm)
     segsum_kernel(const Src src, const int64_t* __restrict__ offsets, const int64_t nseg, const T init,
@@ -297,6 +364,11 @@ __global__ void __launch_bounds__(kSegT, Src::kCtasPerSm)
     int* const pos = sh_pos[warp];
     const int w = blockIdx.x * kSegWarps + warp;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if constexpr (Src::kRows) {
+        const bool rows = seg_rows_by_lanes(offsets, nseg, &sh_bits[0][0]);
+        if (blockIdx.x == 0 && threadIdx.x == 0) *part.by_lanes = rows;
+        if (rows) return;  // the second kernel, of more and smaller warps, takes them
+    }
     const SegSplit sp(src.first(), src.end(), (int64_t)gridDim.x * kSegWarps);
     const int64_t lo = sp.base + w * sp.range;
     if (w > 0 && lo >= sp.hi_valid) {  // no values left for this warp
@@ -550,7 +622,7 @@ __device__ __forceinline__ bool seg_one(const SegProduct<C>& src, int64_t start,
 // one ends the piece that warp w of that one closed.  With invalid offsets it
 // computes every segment instead.
 template <class T, class Src>
-__global__ void __launch_bounds__(kSegT) segsum_finish_kernel(const Src src, const int64_t* __restrict__ offsets,
+__global__ void __launch_bounds__(kSegT, Src::kRows ? 8 : 1) segsum_finish_kernel(const Src src, const int64_t* __restrict__ offsets,
                                                               const int64_t nseg, const T init,
                                                               T* __restrict__ out, const SegPartials<T> part,
                                                               const int64_t nwarps, unsigned* err) {
@@ -558,10 +630,19 @@ __global__ void __launch_bounds__(kSegT) segsum_finish_kernel(const Src src, con
     const int64_t w = (int64_t)blockIdx.x * kSegWarps + warp;
     // launched while the first kernel runs: wait for its results
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if constexpr (Src::kRows) {
+        if (__ldcg(part.by_lanes) != 0u) {
+            seg_rows(src, out, err);
+            return;
+        }
+    }
+    // the blocks beyond the first kernel's were for the rows by lanes only
+    const unsigned nblocks = (unsigned)((nwarps + kSegWarps - 1) / kSegWarps);
+    if (blockIdx.x >= nblocks) return;
     const bool invalid = *(volatile const unsigned*)part.bad != 0u;
     if (invalid) {
         bool bad = false;
-        for (int64_t s = w; s < nseg; s += (int64_t)gridDim.x * kSegWarps)
+        for (int64_t s = w; s < nseg; s += (int64_t)nblocks * kSegWarps)
             bad |= !seg_one(src, offsets[s], offsets[s + 1], init, out + s);
         if (bad) raise_error(err, ERRBIT_BOUNDS);
     } else if (w < nwarps) {
@@ -582,7 +663,7 @@ __global__ void __launch_bounds__(kSegT) segsum_finish_kernel(const Src src, con
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        if (atomicAdd(part.done, 1u) == gridDim.x - 1) {
+        if (atomicAdd(part.done, 1u) == nblocks - 1) {
             *part.bad = 0u;
             *part.done = 0u;
         }
@@ -608,22 +689,25 @@ static int segsum_launch(const Src& src, const int64_t* offsets, int64_t nseg, i
     part.closes = reinterpret_cast<int64_t*>(part.tail + nwarps);
     part.bad = counters + kSegCounterWord;
     part.done = counters + kSegCounterWord + 1;
+    part.by_lanes = counters + kSegCounterWord + 2;
     auto k = segsum_kernel<T, Src>;
     constexpr size_t kSmem = kSegWarps * (size_t)(Src::kStageBytes ? 2 * Src::kStageBytes : kSegC * (int)sizeof(T));
     HYD_TRY(configure_kernel((const void*)k, d, false));
     k<<<(unsigned)blocks, kSegT, kSmem, s>>>(src, offsets, nseg, init, out, part, d->d_err);
     HYD_TRY(launch_check(what));
     // programmatic dependent launch: the second kernel's blocks are in place
-    // when the first one ends
+    // when the first one ends; not where it may have all the rows to do, which
+    // takes an L1 that the first kernel's shared memory has not cut down (100
+    // entries per row, 2^20 rows: 913 us so, 494 without)
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.gridDim = dim3((unsigned)(Src::kRows ? d->sm_count * 16 : blocks));
     cfg.blockDim = dim3(kSegT);
     cfg.stream = s;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = Src::kRows ? 0 : 1;
     HYD_CUDA_TRY(cudaLaunchKernelEx(&cfg, segsum_finish_kernel<T, Src>, src, offsets, nseg, init, out, part, nwarps,
                                     d->d_err));
     return launch_check(what);

@@ -339,14 +339,15 @@ __global__ void __launch_bounds__(256) spmv_csr_kernel(int64_t nrows, const long
 }
 
 // segsum.cu: the entries split evenly over the warps, whatever the rows'
-// lengths.  It searches the row pointers for each warp's share and launches
-// twice, so it pays on large matrices: on rows of Zipf length (12 entries on
-// average, int64 columns) 2^20 rows take 107 us against 198 with 8 lanes per
-// row, 2^18 rows 46 against 66, but 2^17 rows 37 against 33.
+// lengths, or, where the rows are even, 8 lanes per row after all: it looks.  It
+// launches twice and searches the row pointers, so it takes large matrices only.
+// 2^20 rows of Zipf length (12 entries on average, int64 columns) take 105 us
+// against 190 with 8 lanes per row, 2^19 rows 69 against 110, 2^18 rows 49
+// against 50; of 8 entries each 77 against 74, 45 against 39, 29 against 22.
 template <class C>
 int spmv_segsum(int64_t nrows, int64_t ncols, const long long* row_ptr, const C* cols, const double* vals,
                 const double* x, double* y, cudaStream_t s);
-constexpr int64_t kSpmvSegMinRows = 1 << 18;
+constexpr int64_t kSpmvSegMinRows = 3 << 18;
 
 template <class C>
 static int spmv_dispatch(int g, int64_t nrows, const long long* row_ptr, const C* col_idx, const double* vals,

@@ -68,7 +68,7 @@ def _spmv(hc, dev, row_ptr, cols, vals, x, dtype, lanes=0, shift=0):
 @pytest.mark.parametrize("dtype", [torch.int64, torch.int32])
 @pytest.mark.parametrize("kind,shift", [("zipf", 0), ("zipf", 1), ("empty", 0), ("long", 0)])
 def test_spmv_even_split(hc, orc, dev, kind, shift, dtype):
-    nrows, ncols = (1 << 18) + 37, 70_001
+    nrows, ncols = (3 << 18) + 37, 70_001
     row_ptr, cols, vals, x = _csr(np.random.default_rng(5), nrows, ncols, kind)
     y = _spmv(hc, dev, row_ptr, cols, vals, x, dtype, shift=shift)
     hc.check(hc.device_check())
@@ -83,7 +83,7 @@ def test_spmv_even_split_matches_the_lane_split(hc, dev, case):
     """Row pointers that do not start at 0 or do not ascend, and columns out of
     range, give what the lanes-per-row form gives (rows take what their two
     pointers span; a bad column is left out and reported)."""
-    nrows, ncols = 1 << 18, 5000
+    nrows, ncols = 3 << 18, 5000
     row_ptr, cols, vals, x = _csr(np.random.default_rng(6), nrows, ncols, "zipf")
     if case == "starts_later":
         row_ptr = row_ptr[1001:]
@@ -99,3 +99,21 @@ def test_spmv_even_split_matches_the_lane_split(hc, dev, case):
     want = _spmv(hc, dev, row_ptr, cols, vals, x, torch.int64, lanes=8)
     assert hc.device_check() == st == (hc.ERR_BOUNDS if case == "bad_column" else hc.OK)
     assert np.allclose(y.cpu().numpy(), want.cpu().numpy(), rtol=0, atol=1e-12 * 60_000)
+
+
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+@pytest.mark.parametrize("per_row,lanes", [(1, False), (5, False), (8, False), (40, True), (100, True)])
+def test_spmv_even_rows(hc, dev, per_row, lanes, dtype):
+    """Rows of one length go by entries or by lanes, whichever the model says is
+    faster; by lanes the sums are those of the lanes-per-row form, bit for bit."""
+    nrows, ncols = (3 << 18) + 3, 9001
+    rng = np.random.default_rng(per_row)
+    row_ptr = np.arange(nrows + 1, dtype=np.int64) * per_row
+    cols = rng.integers(0, ncols, size=nrows * per_row)
+    vals, x = rng.uniform(-1, 1, size=nrows * per_row), rng.uniform(-1, 1, size=ncols)
+    y = _spmv(hc, dev, row_ptr, cols, vals, x, dtype)
+    want = _spmv(hc, dev, row_ptr, cols, vals, x, dtype, lanes=8)
+    hc.check(hc.device_check())
+    if lanes:
+        assert torch.equal(y, want)
+    assert np.allclose(y.cpu().numpy(), want.cpu().numpy(), rtol=0, atol=1e-12 * per_row)
