@@ -7,9 +7,10 @@
 // array of values cut by ascending offsets (the segment offsets; row_ptr), one
 // sum per piece.  For the SpMV a value is the product vals[k] * x[col[k]].
 //
-// Every warp takes one contiguous range of values, equal shares of all values
-// whatever the segments' lengths, and walks it in chunks of 256:
-//  * a run of chunks with no boundary (the end of a segment) in it is added
+// Every warp takes one contiguous range of values and boundaries (the ends of
+// segments), equal shares of the two together whatever the segments' lengths
+// and however many of them are empty, and walks it in chunks of 256 values:
+//  * a run of chunks with no boundary in it is added
 //    into eight accumulators per lane, one operation per value;
 //  * a chunk with boundaries is summed by a segmented scan: each lane folds
 //    its 8 consecutive values, restarting at each head, one warp scan carries
@@ -22,12 +23,12 @@
 //
 // What bounds it: FP64.  GB300 adds 5.3e11 doubles/s, 254 us for 2^27, against
 // 158 us for reading them.  Measured (start -> now): 2^27 float64 values in
-// segments of 2^U(0,16), 695 -> 317 us (3.4 TB/s); segments of 2^U(0,5), 783 ->
-// 579 us; of one value each, 1136 -> 1014 us.  Before, tiles of 4096 values took
+// segments of 2^U(0,16), 695 -> 312 us (3.4 TB/s); segments of 2^U(0,5), 783 ->
+// 569 us; of one value each, 1136 -> 932 us.  Before, tiles of 4096 values took
 // 1.6 FP64 operations per value and waited for a look-back.  SpMV, 2^20 rows of
-// Zipf length, 12.9e6 entries: 198 -> 109 us; 8 lanes per row spent about seven
+// Zipf length, 12.9e6 entries: 198 -> 100 us; 8 lanes per row spent about seven
 // FP64 lane slots per entry.  Three blocks per SM (80 registers) beat four (64
-// and spills): 1014 against 1327 us on one-value segments.
+// and spills): 1014 against 1327 us on one-value segments when that was tried.
 //
 // Offsets that are not an ascending partition of [0, n_vals] are detected on
 // the way (every adjacent pair is looked at by exactly one warp); the second
@@ -44,6 +45,7 @@ constexpr int kSegT = 256;
 constexpr int kSegWarps = kSegT / 32;
 constexpr int kSegPer = 8;                  // consecutive values per lane
 constexpr int kSegC = 32 * kSegPer;         // values per chunk
+constexpr int kSegAlign = 32;               // a range's first chunk begins at a multiple of this
 constexpr int kSegCounterWord = 240;  // stream counters: +0 invalid offsets, +1 finished blocks, +2 rows by lanes
 // where a chunk's sum i sits: free of bank conflicts for a lane's 8 consecutive values
 __device__ __forceinline__ int seg_slot(int i) { return i ^ ((i >> 4) & 7); }
@@ -57,12 +59,15 @@ __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gsrc, in
 // lanes' reads of their own consecutive units meet few bank conflicts
 __device__ __forceinline__ int seg_unit(int u) { return u ^ ((u >> 3) & 3); }
 
+constexpr int64_t kSegNoBoundary = -1;  // none in the range
+constexpr int64_t kSegNoPiece = -2;     // some, but no piece was open at the range's start
+
 // One entry per warp of the first kernel.
 template <class T>
 struct SegPartials {
     T* head;          // the piece open at the range's start, up to its first boundary
     T* tail;          // after the last boundary (the whole range when it has none)
-    int64_t* closes;  // the boundary that ends that first piece, -1: none, or the piece is empty
+    int64_t* closes;  // the boundary that ends that first piece; kSegNoBoundary, kSegNoPiece
     unsigned* bad;
     unsigned* done;
     unsigned* by_lanes;  // SpMV: the second kernel takes the rows by lanes, the first does nothing
@@ -79,11 +84,16 @@ struct SegPlain {
     const T* vals;
     int64_t n;
     bool vec;  // 32-byte aligned base
+    int64_t share;  // a warp's, of values and boundaries
     struct Item {
         T x[kSegPer];
     };
     __device__ __forceinline__ int64_t first() const { return 0; }
     __device__ __forceinline__ int64_t end() const { return n; }
+    void set_share(int64_t nb, int64_t nwarps) {
+        share = (n + nb + nwarps - 1) / nwarps;
+        if (share < kSegC) share = kSegC;
+    }
     __device__ __forceinline__ bool check(const Item&) const { return true; }
     // positions base + i .. base + i + 7, those with i + j outside [lo, hi) zero
     __device__ __forceinline__ void load(Item& it, int64_t base, int i, int lo, int hi) const {
@@ -127,6 +137,8 @@ struct SegProduct {
     };
     __device__ __forceinline__ int64_t first() const { return row_ptr[0]; }
     __device__ __forceinline__ int64_t end() const { return row_ptr[nrows]; }
+    static constexpr int64_t share = 0;  // the device knows
+    void set_share(int64_t, int64_t) {}
     __device__ __forceinline__ bool check(const Item& it) const { return it.ok; }
     __device__ __forceinline__ void load(Item& it, int64_t base, int i, int lo, int hi) const {
         const C* const cols = this->cols + base;
@@ -228,39 +240,50 @@ struct SegProduct {
     }
 };
 
-// The split of [first, end) over the warps: ranges of `range` values from
-// `base` (a multiple of the chunk), the last ones possibly empty.  Positions
-// inside a range are kept in 32 bits.
+// The split of the values [first, end) and of the nb boundaries over the warps,
+// in equal shares of the two together: the boundaries are merged into the
+// values (boundary b comes before value offsets[b], as item offsets[b] - first +
+// b of the merged sequence), and warp w takes the items from w * per on.  With
+// shares of the values alone a run of empty segments, whose boundaries all
+// stand at one place, fell to one warp: 2^20 rows of Zipf length, half of them
+// empty in a run, took 10.0 ms and now 92 us (8 lanes per row: 138); 10^6 empty
+// segments between two of 500 values 16.5 ms and now 27 us.
 struct SegSplit {
-    int64_t base, range, lo_valid, hi_valid;
+    int64_t lo_valid, hi_valid, per;
     bool ok;
-    __device__ __forceinline__ SegSplit(int64_t first, int64_t end, int64_t nwarps) {
+    // share: `per` where the host knows it, else 0
+    __device__ __forceinline__ SegSplit(int64_t first, int64_t end, int64_t nb, int64_t nwarps, int64_t share) {
         ok = first >= 0 && end >= first;
         lo_valid = ok ? first : 0;
         hi_valid = ok ? end : 0;
-        base = lo_valid / kSegC * kSegC;
-        const int64_t chunks = (hi_valid - base + kSegC - 1) / kSegC;
-        const int64_t per = (chunks + nwarps - 1) / nwarps;
-        range = (per > 0 ? per : 1) * kSegC;
-        if (range > (1 << 30)) ok = false;
+        per = share ? share : (hi_valid - lo_valid + nb + nwarps - 1) / nwarps;
+        if (per > (1 << 29)) ok = false;  // positions inside a range are kept in 32 bits
     }
 };
+// Values before position p and boundaries before number b.
+struct SegCut {
+    int64_t p, b;
+};
 
-// First indices i in [0, m) with a[i] >= key, for two keys at once (m when
-// there is none).  Warp-wide: 32 probes per key and round narrow the range
-// 33-fold.  Monotone in `key` even for unsorted `a`, so the ranges of
-// different warps never overlap and together cover every boundary.
-__device__ __forceinline__ void warp_lower_bound2(const int64_t* __restrict__ a, int64_t m, int64_t key0,
-                                                  int64_t key1, int64_t& out0, int64_t& out1) {
+// The merged sequence's keys: strictly ascending where the offsets ascend.
+__device__ __forceinline__ int64_t seg_key(const int64_t* a, int64_t i) {
+    return (int64_t)((unsigned long long)a[i] + (unsigned long long)i);
+}
+// Narrows [0, m] to at most 33 numbers each, [lo, hi], that hold the first i with
+// seg_key(a, i) >= key (m when there is none), for two keys at once.  Warp-wide:
+// 32 probes per key and round narrow the range 33-fold.  The result depends on
+// the key alone.
+__device__ __forceinline__ void warp_narrow2(const int64_t* __restrict__ a, int64_t m, const int64_t (&key)[2],
+                                             int64_t (&lo)[2], int64_t (&hi)[2]) {
     const int lane = threadIdx.x & 31;
-    int64_t lo[2] = {0, 0}, hi[2] = {m, m};
-    const int64_t key[2] = {key0, key1};
+    lo[0] = lo[1] = 0;
+    hi[0] = hi[1] = m;
     while (hi[0] - lo[0] > 32 || hi[1] - lo[1] > 32) {
         int64_t v[2];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const int64_t p = lo[q] + (hi[q] - lo[q]) * (lane + 1) / 33;
-            v[q] = p < hi[q] ? a[p] : 0;
+            v[q] = p < hi[q] ? seg_key(a, p) : 0;
         }
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -274,17 +297,64 @@ __device__ __forceinline__ void warp_lower_bound2(const int64_t* __restrict__ a,
             }
         }
     }
-    int64_t v[2];
-#pragma unroll
-    for (int q = 0; q < 2; ++q) v[q] = lo[q] + lane < hi[q] ? a[lo[q] + lane] : key[q];
-    out0 = lo[0] + __popc(__ballot_sync(0xffffffffu, v[0] < key0));
-    out1 = lo[1] + __popc(__ballot_sync(0xffffffffu, v[1] < key1));
 }
 
-// Boundary b is offsets[b], 0 <= b <= nseg; it ends segment b - 1.  A warp
-// with the range (lo, hi] takes the boundaries in it, the first warp those at
-// the array's very start too.  Positions and boundary numbers below are
-// relative to the warp's lo and first boundary b0.
+// Where warp w's range begins, and where it ends (the next one's begin).
+// Warp-wide.  A cut is moved to the nearest whole chunk when no more than about
+// 32 boundaries and half a share lie between, with the boundaries at that very
+// place before it: ranges then begin and end with whole chunks as long as
+// boundaries are not dense (one chunk more for every warp cost 10^6 values 3 us
+// of 18).  A cut depends on its number alone, so both neighbours find the same
+// one; the cuts of valid offsets ascend.
+__device__ __forceinline__ void seg_cuts(const SegSplit& sp, const int64_t* __restrict__ a, int64_t nb, int64_t w,
+                                         int64_t nwarps, SegCut& from, SegCut& to) {
+    const int lane = threadIdx.x & 31;
+    const bool second = lane >= 16;  // the lower lanes work out `from`, the upper ones `to`
+    const int64_t d[2] = {sp.lo_valid + w * sp.per, sp.lo_valid + (w + 1) * sp.per};
+    int64_t lo[2], hi[2];
+    warp_narrow2(a, nb, d, lo, hi);
+    // the boundaries that may be the cut's, and 32 on either side of them
+    constexpr int kNear = 32, kLoads = 2 * kNear / 32 + 1;
+    int64_t x[2][kLoads];
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int k = 0; k < kLoads; ++k) {
+            const int64_t i = lo[q] - kNear + 32 * k + lane;
+            x[q][k] = i < 0 ? LLONG_MIN : (i < nb ? a[i] : LLONG_MAX);
+        }
+    int past[2], near[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int64_t i = lo[q] + lane;
+        const bool below = i < hi[q] && (int64_t)((unsigned long long)x[q][kNear / 32] + (unsigned long long)i) < d[q];
+        past[q] = __popc(__ballot_sync(0xffffffffu, below));
+    }
+    const int64_t item = second ? d[1] : d[0];
+    SegCut c;
+    c.b = second ? lo[1] + past[1] : lo[0] + past[0];
+    c.p = item - c.b;
+    c.p = c.p < sp.lo_valid ? sp.lo_valid : (c.p > sp.hi_valid ? sp.hi_valid : c.p);
+    int64_t edge = (c.p + kSegC / 2) / kSegC * kSegC;
+    edge = edge < sp.lo_valid ? sp.lo_valid : (edge > sp.hi_valid ? sp.hi_valid : edge);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {  // of those boundaries the ones up to the chunk's edge
+        const int64_t e = __shfl_sync(0xffffffffu, edge, 16 * q);
+        int n = 0;
+#pragma unroll
+        for (int k = 0; k < kLoads; ++k) n += x[q][k] <= e;
+        near[q] = __reduce_add_sync(0xffffffffu, n);
+    }
+    const int n = second ? near[1] : near[0], by = n - kNear - (second ? past[1] : past[0]);
+    const int64_t moved = (edge < c.p ? c.p - edge : edge - c.p) + (by < 0 ? -by : by);
+    if (n > 0 && n < 32 * kLoads && 2 * moved <= sp.per) c = SegCut{edge, c.b + by};
+    const int64_t number = second ? w + 1 : w;
+    if (number == 0) c = SegCut{sp.lo_valid, 0};
+    else if (number >= nwarps || item >= sp.hi_valid + nb) c = SegCut{sp.hi_valid, nb};
+    from = SegCut{__shfl_sync(0xffffffffu, c.p, 0), __shfl_sync(0xffffffffu, c.b, 0)};
+    to = SegCut{__shfl_sync(0xffffffffu, c.p, 16), __shfl_sync(0xffffffffu, c.b, 16)};
+}
+
 // ---- rows of even length --------------------------------------------------------
 // Where the rows of an SpMV are about equally long, 8 lanes per row waste little
 // and need no search, no scan and no staging.  Only the device knows the lengths:
@@ -349,6 +419,10 @@ __device__ __forceinline__ void seg_rows(const Src& src, double* __restrict__ y,
     if (bad) raise_error(err, ERRBIT_BOUNDS);
 }
 
+// Boundary b is offsets[b], 0 <= b <= nseg; it ends segment b - 1.  A warp takes
+// the values and the boundaries between its two cuts.  Positions and boundary
+// numbers below are relative to lo, the chunk that its first value is in, and to
+// its first boundary b0.
 template <class T, class Src>
 __global__ void __launch_bounds__(kSegT, Src::kCtasPerSm)
     segsum_kernel(const Src src, const int64_t* __restrict__ offsets, const int64_t nseg, const T init,
@@ -369,23 +443,22 @@ __global__ void __launch_bounds__(kSegT, Src::kCtasPerSm)
         if (blockIdx.x == 0 && threadIdx.x == 0) *part.by_lanes = rows;
         if (rows) return;  // the second kernel, of more and smaller warps, takes them
     }
-    const SegSplit sp(src.first(), src.end(), (int64_t)gridDim.x * kSegWarps);
-    const int64_t lo = sp.base + w * sp.range;
-    if (w > 0 && lo >= sp.hi_valid) {  // no values left for this warp
+    const int64_t nwarps = (int64_t)gridDim.x * kSegWarps;
+    const SegSplit sp(src.first(), src.end(), nseg + 1, nwarps, src.share);
+    SegCut from, to;
+    seg_cuts(sp, offsets, nseg + 1, w, nwarps, from, to);
+    const int64_t b0 = from.b;
+    if (sp.ok && from.p == to.p && b0 == to.b) {  // nothing left for this warp
         if (lane == 0) {
             part.tail[w] = T(0);
-            part.closes[w] = -1;
+            part.closes[w] = kSegNoBoundary;
         }
         return;
     }
-    const bool is_last = lo + sp.range >= sp.hi_valid;
-    int64_t b0, b1;
-    warp_lower_bound2(offsets, nseg + 1, lo + 1, lo + sp.range + 1, b0, b1);
-    if (w == 0) b0 = 0;
-    if (is_last) b1 = nseg + 1;
-    bool bad = !sp.ok || b1 < b0 || b1 - b0 > INT_MAX - 64;
+    const int64_t lo = from.p / kSegAlign * kSegAlign;
+    bool bad = !sp.ok || to.b < b0 || to.p < from.p || to.p - lo > (1 << 30);
     bool bad_item = false;
-    const int nb = bad ? 0 : (int)(b1 - b0);
+    const int nb = bad ? 0 : (int)(to.b - b0);
     const int64_t* const off = offsets + b0;  // [nb]
     T* const outb = out + b0 - 1;             // segment b0 - 1 + r ends at boundary r
     // a boundary's position: clamped below to "before the range"
@@ -393,8 +466,7 @@ __global__ void __launch_bounds__(kSegT, Src::kCtasPerSm)
         const int64_t r = x - lo;
         return r < 0 ? -1 : (r > INT_MAX ? INT_MAX : (int)r);
     };
-    const int vlo = (int)(sp.lo_valid > lo ? sp.lo_valid - lo : 0);                      // valid positions:
-    const int vhi = (int)(sp.hi_valid - lo < sp.range ? sp.hi_valid - lo : sp.range);  // [vlo, vhi)
+    const int vlo = (int)(from.p - lo), vhi = bad ? 0 : (int)(to.p - lo);  // valid positions: [vlo, vhi)
     const int stop_p = vhi;  // chunks start below this (the first one always runs)
     int bc = 0;                                      // first boundary not yet passed
     int prev = b0 > 0 ? rel(offsets[b0 - 1]) : -2;   // the one before it
@@ -465,7 +537,7 @@ __global__ void __launch_bounds__(kSegT, Src::kCtasPerSm)
             const int cnt = __popc(m);
             if (in) {
                 // ascending, inside the values, and not one that an earlier chunk should have met
-                bad |= xw < before || xw > vhi || xw < vlo || !(xw > p || (w == 0 && xw == 0));
+                bad |= xw < before || xw > vhi || xw < vlo || !(xw > p || p == 0);
                 if (xw > p && xw < p + kSegC) atomicOr(&bits[(xw - p) >> 5], 1u << ((xw - p) & 31));
                 at_end |= xw == p + kSegC;
                 if (total + lane < Src::kPos) pos[total + lane] = xw;
@@ -540,7 +612,7 @@ __global__ void __launch_bounds__(kSegT, Src::kCtasPerSm)
         // boundary 0 ends no segment; the piece that was open at lo goes to the partials
         auto finish = [&](int k, int x, int before) {
             const T s = x > p ? sums[seg_slot(x - 1 - p)] : T(0);
-            const bool open = before < 0 && before != x;
+            const bool open = before < vlo;
             if (open && (b0 > 0 || bc + k > 0)) {
                 part.head[w] = s;
                 part.closes[w] = b0;
@@ -581,7 +653,7 @@ __global__ void __launch_bounds__(kSegT, Src::kCtasPerSm)
     for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     const bool any = __any_sync(0xffffffffu, closes);
     if (lane == 0) {
-        if (!any) part.closes[w] = -1;
+        if (!any) part.closes[w] = nb > 0 ? kSegNoPiece : kSegNoBoundary;
         part.tail[w] = carry + a;
         if (bad) atomicOr(part.bad, 1u);
     }
@@ -648,12 +720,17 @@ __global__ void __launch_bounds__(kSegT, Src::kRows ? 8 : 1) segsum_finish_kerne
     } else if (w < nwarps) {
         const int64_t b = part.closes[w];
         if (b >= 0) {
-            const SegSplit sp(src.first(), src.end(), nwarps);
-            const int64_t start = offsets[b - 1];
-            // the warp whose range (lo, hi] holds the piece's start
-            const int64_t u0 = start > sp.base ? (start - 1 - sp.base) / sp.range : 0;
-            T s = T(0);
-            for (int64_t u = u0 + lane; u < w; u += 32) s += part.tail[u];
+            // the warp that took the boundary which opened the piece: the one whose
+            // share of the merged sequence it is in, or, where the cut there was
+            // moved, one beside it; between it and this warp none has a boundary
+            const SegSplit sp(src.first(), src.end(), nseg + 1, nwarps, src.share);
+            const unsigned long long item = seg_key(offsets, b - 1) - sp.lo_valid;
+            int64_t u = (item >> 32) == 0 ? (unsigned)item / (unsigned)sp.per : (int64_t)(item / sp.per);
+            u += lane - 1;
+            T s = u >= 0 && u < w ? part.tail[u] : T(0);
+            const bool has = lane < 3 && u >= 0 && u < w && part.closes[u] != kSegNoBoundary;
+            if (lane < 31 - __clz((int)__ballot_sync(0xffffffffu, has))) s = T(0);  // before the piece
+            for (u += 32; u < w; u += 32) s += part.tail[u];
 #pragma unroll
             for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
             if (lane == 0) out[b - 1] = init + (s + part.head[w]);
@@ -670,16 +747,25 @@ __global__ void __launch_bounds__(kSegT, Src::kRows ? 8 : 1) segsum_finish_kerne
     }
 }
 
-// `values`: the number of values, or an estimate of it when only the device knows.
+// `values`: their number, or an estimate of it when only the device knows.
 template <class T, class Src>
-static int segsum_launch(const Src& src, const int64_t* offsets, int64_t nseg, int64_t values, T init, T* out,
+static int segsum_launch(Src src, const int64_t* offsets, int64_t nseg, int64_t values, T init, T* out,
                          cudaStream_t s, const char* what) {
     Device* d = nullptr;
     HYD_TRY(device(&d));
-    int64_t blocks = (values + (int64_t)kSegC * kSegWarps - 1) / ((int64_t)kSegC * kSegWarps);
-    const int64_t cap = (int64_t)d->sm_count * Src::kCtasPerSm;
-    blocks = blocks < 1 ? 1 : (blocks > cap ? cap : blocks);
+    // a warp per 256 values and boundaries while there is a block per SM at most;
+    // then per 256 values, or 512 of both (3e5 values in 1.4e5 segments: 14.4 us,
+    // 16.4 with a warp per 256 of both; 4e4 in 1.9e4: 13.9 and 12.3)
+    const int64_t each = (int64_t)kSegC * kSegWarps, both = values + nseg + 1;
+    const int64_t some = values > both / 2 ? values : both / 2, cap = (int64_t)d->sm_count * Src::kCtasPerSm;
+    int64_t blocks = (both + each - 1) / each;
+    if (blocks > d->sm_count) {
+        blocks = (some + each - 1) / each;
+        if (blocks < d->sm_count) blocks = d->sm_count;
+    }
+    if (blocks > cap) blocks = cap;
     const int64_t nwarps = blocks * kSegWarps;
+    src.set_share(nseg + 1, nwarps);
     unsigned* counters = nullptr;
     void* scratch = nullptr;
     HYD_TRY(workspace(s, (size_t)nwarps * 24, &counters, &scratch));
@@ -737,7 +823,7 @@ static int segreduce_launch(const int64_t* offsets, int64_t n_offsets, const T* 
     HYD_CHECK_ARG(nseg == 0 || out != nullptr, "%s: null output", what);
     if (nseg == 0) return HYD_CUDA_OK;
     HYD_CHECK_ARG(n_vals <= (int64_t)4096 * 0x7fffffffLL, "%s: too many values", what);
-    const SegPlain<T> src{vals, n_vals, (reinterpret_cast<uintptr_t>(vals) & 31) == 0};
+    const SegPlain<T> src{vals, n_vals, (reinterpret_cast<uintptr_t>(vals) & 31) == 0, 0};
     return segsum_launch<T>(src, offsets, nseg, n_vals, init, out, as_stream(stream), what);
 }
 

@@ -117,3 +117,78 @@ def test_spmv_even_rows(hc, dev, per_row, lanes, dtype):
     if lanes:
         assert torch.equal(y, want)
     assert np.allclose(y.cpu().numpy(), want.cpu().numpy(), rtol=0, atol=1e-12 * per_row)
+
+
+def _with_empty_run(rng, n, where, filled):
+    """Lengths of n rows, `filled` of them (the others empty in one run, or two)."""
+    lens = np.zeros(n, dtype=np.int64)
+    at = {"front": n - filled, "end": 0, "middle": 0}[where]
+    lens[at:at + filled] = np.minimum(rng.zipf(1.5, size=filled), 256)
+    if where == "middle":  # half of the filled rows move to the other end
+        lens[n - filled // 2:], lens[filled // 2:filled] = lens[filled // 2:filled][-(filled // 2):].copy(), 0
+    return lens
+
+
+def _us(f, reps=5):
+    """Fastest of a few timed runs on the current stream."""
+    f()
+    best = float("inf")
+    for _ in range(reps):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        f()
+        b.record()
+        b.synchronize()
+        best = min(best, 1e3 * a.elapsed_time(b))
+    return best
+
+
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32])
+@pytest.mark.parametrize("where", ["front", "middle", "end"])
+@pytest.mark.parametrize("nrows,filled", [(1 << 20, 1 << 19), (4_000_001, 40_000), (1 << 20, 2)])
+def test_spmv_run_of_empty_rows(hc, orc, dev, nrows, filled, where, dtype):
+    """Rows that are empty in one run, whose boundaries all stand at one entry,
+    cost no more than they do with 8 lanes per row (twice that, for noise)."""
+    rng = np.random.default_rng(filled)
+    row_ptr = np.concatenate([[0], np.cumsum(_with_empty_run(rng, nrows, where, filled))]).astype(np.int64)
+    nnz, ncols = int(row_ptr[-1]), 70_001
+    cols, vals, x = rng.integers(0, ncols, size=nnz), rng.uniform(-1, 1, size=nnz), rng.uniform(-1, 1, size=ncols)
+    rp, ci = torch.from_numpy(row_ptr).to(dev), torch.from_numpy(cols).to(dev, dtype)
+    v, xt = torch.from_numpy(vals).to(dev), torch.from_numpy(x).to(dev)
+    y = torch.full((nrows,), -7.0, dtype=torch.float64, device=dev)
+    y8 = torch.empty_like(y)
+    now = _us(lambda: hc.spmv_csr(rp, ci, v, xt, y))
+    lanes = _us(lambda: hc.spmv_csr(rp, ci, v, xt, y8, lanes_per_row=8))
+    hc.check(hc.device_check())
+    bound = orc.spmv_csr(row_ptr, cols, np.abs(vals), np.abs(x))
+    assert np.all(np.abs(y.cpu().numpy() - orc.spmv_csr(row_ptr, cols, vals, x)) <= 1e-12 * bound)
+    assert now <= 2 * lanes
+
+
+@pytest.mark.parametrize("where", ["front", "middle", "end"])
+@pytest.mark.parametrize("nseg,filled", [(1_000_000, 2), (1 << 20, 1 << 19), (3_000_001, 100_000)])
+def test_run_of_empty_segments(hc, orc, dev, nseg, filled, where):
+    """Segments that are empty in one run cost about what as many cost with the
+    empty ones spread between the others (four times that, for noise and the
+    shares' unevenness)."""
+    rng = np.random.default_rng(nseg)
+    lens = _with_empty_run(rng, nseg, where, filled)
+    offsets = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    _seg(hc, orc, dev, offsets, int(offsets[-1]), 0)
+    spread = np.concatenate([[0], np.cumsum(rng.permutation(lens))]).astype(np.int64)
+    v = torch.rand(int(offsets[-1]), dtype=torch.float64, device=dev)
+    o = torch.empty(nseg, dtype=torch.float64, device=dev)
+    a, b = torch.from_numpy(offsets).to(dev), torch.from_numpy(spread).to(dev)
+    now = _us(lambda: hc.segmented_reduce(a, v, o, init=0.0))
+    assert now <= 4 * _us(lambda: hc.segmented_reduce(b, v, o, init=0.0))
+
+
+@pytest.mark.parametrize("nwords", [1, 37, 63, 64, 65, 129, 1000])
+@pytest.mark.parametrize("step", [1, 3, 64, 255, 256, 300])
+def test_equal_offsets_where_ranges_are_cut(hc, orc, dev, nwords, step):
+    """`nwords` equal offsets every `step` values: cuts between the warps fall
+    inside such a group, at its edges and around the 64 boundaries up to which
+    a cut moves to a whole chunk."""
+    ends = np.repeat(np.arange(0, 20_000, step, dtype=np.int64), nwords)[:1_500_000]
+    offsets = np.concatenate([ends, np.full(nwords, ends[-1] + 100)])
+    _seg(hc, orc, dev, offsets, int(offsets[-1]) + 100, 0)
