@@ -70,7 +70,7 @@ struct SegPartials {
     int64_t* closes;  // the boundary that ends that first piece; kSegNoBoundary, kSegNoPiece
     unsigned* bad;
     unsigned* done;
-    unsigned* by_lanes;  // SpMV: the second kernel takes the rows by lanes, the first does nothing
+    unsigned* by_lanes;  // SpMV: not 0: the second kernel takes the rows by lanes, the first does nothing
 };
 
 // ---- what a position of the array contributes ---------------------------------
@@ -118,7 +118,8 @@ template <class C>
 struct SegProduct {
     // chunks are staged in shared memory by cp.async, two ahead: the entries'
     // latency is off the chain entries -> x -> sums
-    static constexpr bool kRows = true;  // rows of even length may go by lanes
+    static constexpr bool kRows = true;  // rows of even length may go by lanes ...
+    static constexpr float kLanesMean = sizeof(C) == 8 ? 16.0f : 20.0f;  // ... from this many entries on average
     static constexpr int kCtasPerSm = 3, kUnroll = 1;
     static constexpr int kStageBytes = kSegC * (8 + (int)sizeof(C));  // values, then columns
     // none: three blocks of two staged chunks per warp just fit the 196 KB
@@ -361,61 +362,111 @@ __device__ __forceinline__ void seg_cuts(const SegSplit& sp, const int64_t* __re
 // every block looks at the same 256 groups of four neighbouring rows (what a warp
 // takes, with 8 lanes each) and so comes to the same answer.
 //
-// A group costs as many FP64 warp instructions as its longest row has eights of
-// entries, and three to combine.  Times in ns, fitted to measurements: by lanes
-// 5000 plus 0.0163 per row and instruction plus 0.002 per entry; by entries 22000
-// plus 0.008 per row plus 0.0054 per entry.  Uneven rows (the groups' longest well
-// above the average) are always split by entries.  2^20 rows, int64 columns, by 8
-// lanes without asking, by entries without asking, and now: 3 entries each 74, 47
-// and 52 us; 8 74, 68 and 77; 12 108, 96 and 101; 32 158, 200 and 162; 100 492, 580
-// and 494; Zipf
-// lengths 189, 102 and 105.
-// Called by all threads of a block of 256; sh: eight words.
-__device__ __forceinline__ bool seg_rows_by_lanes(const int64_t* __restrict__ row_ptr, int64_t nrows, unsigned* sh) {
+// By lanes go rows of 16 entries and more on average (20 with int32 columns, which
+// the entry split reads at less cost), unless they are uneven: the groups' longest
+// rows well above the average, or the average well above that of the sampled rows
+// (what the sample did not see must then be long).  2^20 rows, int64 / int32
+// columns, by 8 lanes and by entries, us: 8 entries each 74 and 71 / 82 and 66; 12
+// 108 and 92 / 107 and 86; 16 95 and 112 / 103 and 105; 20 115 and 134 / 121 and 125;
+// 32 157 and 194 / 160 and 181; 100 491 and 539 / 463 and 506; 16 to 48 178 and 194 /
+// 179 and 181; Zipf lengths 191 and 97 / 182 and 90.  (Looking takes 2 us.)
+// Returns 0, or, for the rows by lanes, how many entries make one of them long.
+// Called by all threads of a block of 256; sh: sixteen words.
+template <class Src>
+__device__ __forceinline__ unsigned seg_rows_by_lanes(const int64_t* __restrict__ row_ptr, int64_t nrows, unsigned* sh) {
     const int64_t r = (int64_t)threadIdx.x * (nrows >> 2) / kSegT * 4;
-    const float rows = (float)nrows, entries = (float)(row_ptr[nrows] - row_ptr[0]);
+    const float mean = (float)(row_ptr[nrows] - row_ptr[0]) / (float)nrows;
     int64_t p = row_ptr[r];
-    unsigned longest = 0;
+    unsigned longest = 0, len = 0;
 #pragma unroll
     for (int k = 1; k <= 4; ++k) {
         const int64_t e = r + k <= nrows ? row_ptr[r + k] : p, l = e - p;
-        const unsigned n = l < 0 ? 0u : (l > (1 << 20) ? 1u << 17 : (unsigned)(l + 7) >> 3);
+        const unsigned n = l < 0 ? 0u : (l > (1 << 20) ? 1u << 20 : (unsigned)l);
         longest = n > longest ? n : longest;
+        len += n;
         p = e;
     }
-    longest = __reduce_add_sync(0xffffffffu, longest);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = longest;
+    longest = __reduce_add_sync(0xffffffffu, (longest + 7) >> 3);
+    len = __reduce_add_sync(0xffffffffu, len);
+    if ((threadIdx.x & 31) == 0) {
+        sh[threadIdx.x >> 5] = longest;
+        sh[kSegWarps + (threadIdx.x >> 5)] = len;
+    }
     __syncthreads();
-    unsigned sum = 0;
+    unsigned eights = 0, sampled = 0;  // of 256 groups, of 1024 rows
 #pragma unroll
-    for (int w = 0; w < kSegWarps; ++w) sum += sh[w];
+    for (int w = 0; w < kSegWarps; ++w) {
+        eights += sh[w];
+        sampled += sh[kSegWarps + w];
+    }
     __syncthreads();
-    const float eights = (float)sum * (1.0f / kSegT);
-    if (eights > entries / rows * (1.25f / 8.0f) + 1.25f) return false;
-    return 5000.0f + 0.0163f * rows * (eights + 3.0f) + 0.002f * entries < 22000.0f + 0.008f * rows + 0.0054f * entries;
+    const bool even = mean >= Src::kLanesMean && (float)eights * (1.0f / kSegT) <= mean * (1.25f / 8.0f) + 1.25f &&
+                      mean <= (float)sampled * (1.25f / (4 * kSegT));
+    return even ? (mean < 128.0f ? 1024u : (unsigned)(8.0f * mean)) : 0u;  // (mean below 1.25 * 2^20)
 }
 
-// The rows by 8 lanes each, the sums of spmv_csr_kernel<8>, bit for bit.
+// The rows by 8 lanes each, the sums of spmv_csr_kernel<8>, bit for bit, but for
+// rows of more than 1024 entries and eight times the average: the first eight
+// that a warp meets wait for the whole block.  The sample sees one row in a
+// thousand, and 8 lanes take 0.42 us per 8 entries of a long one: 2^20 rows of 32
+// and one of 10^6 entries 55.6 ms, now 2.3.
+constexpr int kSegLongKept = 8;
 template <class Src>
-__device__ __forceinline__ void seg_rows(const Src& src, double* __restrict__ y, unsigned* err) {
-    const int sub = threadIdx.x & 7, group = (threadIdx.x & 31) >> 3;
+__device__ __forceinline__ void seg_rows(const Src& src, double* __restrict__ y, unsigned limit, unsigned* err) {
+    __shared__ int64_t sh_row[kSegWarps][kSegLongKept];
+    __shared__ int sh_kept[kSegWarps];
+    __shared__ double sh_sum[kSegWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = threadIdx.x & 7, group = lane >> 3;
     const int64_t warps = (int64_t)gridDim.x * kSegWarps;
     bool bad = false;
-    for (int64_t rb = ((int64_t)blockIdx.x * kSegWarps + (threadIdx.x >> 5)) * 4; rb < src.nrows; rb += warps * 4) {
+    int kept = 0;
+    for (int64_t rb = ((int64_t)blockIdx.x * kSegWarps + warp) * 4; rb < src.nrows; rb += warps * 4) {
         const int64_t r = rb + group;
+        const long long s = r < src.nrows ? src.row_ptr[r] : 0, e = r < src.nrows ? src.row_ptr[r + 1] : 0;
+        const unsigned far = __ballot_sync(0xffffffffu, e - s > (long long)limit && sub == 0);  // the groups with a long row
+        const int at = kept + __popc(far & ((1u << (8 * group)) - 1u));
+        const bool later = e - s > (long long)limit && at < kSegLongKept;
+        kept += __popc(far);
         double acc = 0.0;
-        if (r < src.nrows) {
-            const long long s = src.row_ptr[r], e = src.row_ptr[r + 1];
-            for (long long k = s + sub; k < e; k += 8) {
-                const long long c = (long long)__ldg(src.cols + k);
-                if ((unsigned long long)c < (unsigned long long)src.ncols) acc = fma(__ldg(src.vals + k), __ldg(src.x + c), acc);
-                else bad = true;
-            }
+        for (long long k = s + sub; k < e && !later; k += 8) {
+            const long long c = (long long)__ldg(src.cols + k);
+            if ((unsigned long long)c < (unsigned long long)src.ncols) acc = fma(__ldg(src.vals + k), __ldg(src.x + c), acc);
+            else bad = true;
         }
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, 8);
-        if (sub == 0 && r < src.nrows) y[r] = acc;
+        if (sub == 0 && r < src.nrows) {
+            if (later) sh_row[warp][at] = r;
+            else y[r] = acc;
+        }
     }
+    if (lane == 0) sh_kept[warp] = kept < kSegLongKept ? kept : kSegLongKept;
+    __syncthreads();
+    for (int w = 0; w < kSegWarps; ++w)
+        for (int i = 0; i < sh_kept[w]; ++i) {
+            const int64_t r = sh_row[w][i];
+            const long long e = src.row_ptr[r + 1];
+            double acc = 0.0;
+#pragma unroll 4
+            for (long long k = src.row_ptr[r] + threadIdx.x; k < e; k += kSegT) {
+                const long long c = (long long)__ldg(src.cols + k);
+                const bool ok = (unsigned long long)c < (unsigned long long)src.ncols;
+                const double v = __ldg(src.vals + k), x = ok ? __ldg(src.x + c) : 0.0;
+                if (ok) acc = fma(v, x, acc);
+                bad |= !ok;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane == 0) sh_sum[warp] = acc;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                acc = 0.0;
+#pragma unroll
+                for (int u = 0; u < kSegWarps; ++u) acc += sh_sum[u];
+                y[r] = acc;
+            }
+            __syncthreads();
+        }
     if (bad) raise_error(err, ERRBIT_BOUNDS);
 }
 
@@ -439,9 +490,9 @@ __global__ void __launch_bounds__(kSegT, Src::kCtasPerSm)
     const int w = blockIdx.x * kSegWarps + warp;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if constexpr (Src::kRows) {
-        const bool rows = seg_rows_by_lanes(offsets, nseg, &sh_bits[0][0]);
-        if (blockIdx.x == 0 && threadIdx.x == 0) *part.by_lanes = rows;
-        if (rows) return;  // the second kernel, of more and smaller warps, takes them
+        const unsigned limit = seg_rows_by_lanes<Src>(offsets, nseg, &sh_bits[0][0]);
+        if (blockIdx.x == 0 && threadIdx.x == 0) *part.by_lanes = limit;
+        if (limit) return;  // the second kernel, of more and smaller warps, takes them
     }
     const int64_t nwarps = (int64_t)gridDim.x * kSegWarps;
     const SegSplit sp(src.first(), src.end(), nseg + 1, nwarps, src.share);
@@ -703,8 +754,8 @@ __global__ void __launch_bounds__(kSegT, Src::kRows ? 8 : 1) segsum_finish_kerne
     // launched while the first kernel runs: wait for its results
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if constexpr (Src::kRows) {
-        if (__ldcg(part.by_lanes) != 0u) {
-            seg_rows(src, out, err);
+        if (const unsigned limit = __ldcg(part.by_lanes)) {
+            seg_rows(src, out, limit, err);
             return;
         }
     }

@@ -341,9 +341,10 @@ __global__ void __launch_bounds__(256) spmv_csr_kernel(int64_t nrows, const long
 // segsum.cu: the entries split evenly over the warps, whatever the rows'
 // lengths, or, where the rows are even, 8 lanes per row after all: it looks.  It
 // launches twice and searches the row pointers, so it takes large matrices only.
-// 2^20 rows of Zipf length (12 entries on average, int64 columns) take 105 us
-// against 190 with 8 lanes per row, 2^19 rows 69 against 110, 2^18 rows 49
-// against 50; of 8 entries each 77 against 74, 45 against 39, 29 against 22.
+// Rows of Zipf length (12 entries on average, int64 columns), so and by 8 lanes
+// each: 2^20 rows 97 and 204 us, 3 * 2^18 79 and 149, 2^19 61 and 104, 2^18 43 and
+// 54; rows of 8 entries 71 and 74, 60 and 58, 47 and 39, 37 and 22.  From 3 * 2^18
+// rows on no kind of row loses more than 5%; below, even rows lose more.
 template <class C>
 int spmv_segsum(int64_t nrows, int64_t ncols, const long long* row_ptr, const C* cols, const double* vals,
                 const double* x, double* y, cudaStream_t s);

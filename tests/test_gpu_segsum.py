@@ -192,3 +192,33 @@ def test_equal_offsets_where_ranges_are_cut(hc, orc, dev, nwords, step):
     ends = np.repeat(np.arange(0, 20_000, step, dtype=np.int64), nwords)[:1_500_000]
     offsets = np.concatenate([ends, np.full(nwords, ends[-1] + 100)])
     _seg(hc, orc, dev, offsets, int(offsets[-1]) + 100, 0)
+
+
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32])
+@pytest.mark.parametrize("per_row,long,count", [(8, 1_000_000, 1), (32, 1_000_000, 1), (32, 10_000_000, 1), (32, 1025, 9),
+                                                (32, 5000, 3000), (100, 20_000, 70)])
+def test_spmv_even_rows_and_a_few_long_ones(hc, orc, dev, per_row, long, count, dtype):
+    """Rows of one length but for a few long ones that a sample of the rows does
+    not show (neighbours among them): right, the same over runs, and the long
+    rows are not left to 8 lanes each (a fifth of the time those take for the
+    longest, 0.4 us per 8 entries, beside the time for the even rows alone)."""
+    nrows, ncols = (3 << 18) + 3, 9001
+    rng = np.random.default_rng(count)
+    lens = np.full(nrows, per_row, dtype=np.int64)
+    at = 4 * rng.integers(0, nrows // 4 - 1, size=count) + 1
+    at[count // 2:] = at[:count - count // 2] + 1
+    lens[np.minimum(at, nrows - 1)] = long
+    row_ptr = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    nnz = int(row_ptr[-1])
+    cols, vals, x = rng.integers(0, ncols, size=nnz), rng.uniform(-1, 1, size=nnz), rng.uniform(-1, 1, size=ncols)
+    y = _spmv(hc, dev, row_ptr, cols, vals, x, dtype)
+    assert torch.equal(y, _spmv(hc, dev, row_ptr, cols, vals, x, dtype))
+    hc.check(hc.device_check())
+    ref = orc.spmv_csr(row_ptr, cols, vals, x)
+    bound = orc.spmv_csr(row_ptr, cols, np.abs(vals), np.abs(x))
+    assert np.all(np.abs(y.cpu().numpy() - ref) <= 1e-12 * bound)
+    rp, ci = torch.from_numpy(row_ptr).to(dev), torch.from_numpy(cols).to(dev, dtype)
+    v, xt = torch.from_numpy(vals).to(dev), torch.from_numpy(x).to(dev)
+    even = torch.arange(nrows + 1, device=dev) * per_row
+    now = _us(lambda: hc.spmv_csr(rp, ci, v, xt, y))
+    assert now <= 2 * _us(lambda: hc.spmv_csr(even, ci, v, xt, y)) + long / 8 * 0.4 / 5
