@@ -68,6 +68,10 @@ struct Device {
     std::unordered_map<cudaStream_t, Workspace> ws;
     // runtime-owned device buffers (staging for host-pointer entry points)
     std::unordered_map<std::string, Workspace> bufs;
+    // the SpMV's own scratch per stream, of one size, and what keeps its two
+    // launches together
+    std::mutex spmv_mu;
+    std::unordered_map<cudaStream_t, Workspace> spmv_ws;
     cudaStream_t side[2] = {nullptr, nullptr};  // pipelining streams
 };
 

@@ -212,6 +212,8 @@ void hyd_cuda_cleanup(void) {
             if (kv.second.base) cudaFree(kv.second.base);
         for (auto& kv : d->bufs)
             if (kv.second.base) cudaFree(kv.second.base);
+        for (auto& kv : d->spmv_ws)
+            if (kv.second.base) cudaFree(kv.second.base);
         for (cudaStream_t s : d->side)
             if (s) cudaStreamDestroy(s);
         if (d->d_err) cudaFree(d->d_err);

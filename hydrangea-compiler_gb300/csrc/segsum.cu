@@ -46,7 +46,7 @@ constexpr int kSegWarps = kSegT / 32;
 constexpr int kSegPer = 8;                  // consecutive values per lane
 constexpr int kSegC = 32 * kSegPer;         // values per chunk
 constexpr int kSegAlign = 32;               // a range's first chunk begins at a multiple of this
-constexpr int kSegCounterWord = 240;  // stream counters: +0 invalid offsets, +1 finished blocks, +2 rows by lanes
+constexpr int kSegCounterWord = 240;  // of the segmented reduce among the stream's counters
 // where a chunk's sum i sits: free of bank conflicts for a lane's 8 consecutive values
 __device__ __forceinline__ int seg_slot(int i) { return i ^ ((i >> 4) & 7); }
 
@@ -68,8 +68,8 @@ struct SegPartials {
     T* head;          // the piece open at the range's start, up to its first boundary
     T* tail;          // after the last boundary (the whole range when it has none)
     int64_t* closes;  // the boundary that ends that first piece; kSegNoBoundary, kSegNoPiece
-    unsigned* bad;
-    unsigned* done;
+    unsigned* bad;   // invalid offsets were met
+    unsigned* done;  // finished blocks of the second kernel
     unsigned* by_lanes;  // SpMV: not 0: the second kernel takes the rows by lanes, the first does nothing
 };
 
@@ -798,12 +798,10 @@ __global__ void __launch_bounds__(kSegT, Src::kRows ? 8 : 1) segsum_finish_kerne
     }
 }
 
-// `values`: their number, or an estimate of it when only the device knows.
-template <class T, class Src>
-static int segsum_launch(Src src, const int64_t* offsets, int64_t nseg, int64_t values, T init, T* out,
-                         cudaStream_t s, const char* what) {
-    Device* d = nullptr;
-    HYD_TRY(device(&d));
+// Blocks of the first kernel.  `values`: their number, or an estimate of it when
+// only the device knows.
+template <class Src>
+static int64_t segsum_blocks(const Device* d, int64_t nseg, int64_t values) {
     // a warp per 256 values and boundaries while there is a block per SM at most;
     // then per 256 values, or 512 of both (3e5 values in 1.4e5 segments: 14.4 us,
     // 16.4 with a warp per 256 of both; 4e4 in 1.9e4: 13.9 and 12.3)
@@ -814,19 +812,23 @@ static int segsum_launch(Src src, const int64_t* offsets, int64_t nseg, int64_t 
         blocks = (some + each - 1) / each;
         if (blocks < d->sm_count) blocks = d->sm_count;
     }
-    if (blocks > cap) blocks = cap;
+    return blocks > cap ? cap : blocks;
+}
+// `counters`: three words, zero the first time; scratch: segsum_bytes(blocks).
+static size_t segsum_bytes(int64_t blocks) { return (size_t)blocks * kSegWarps * 24; }
+
+template <class T, class Src>
+static int segsum_launch(Src src, const int64_t* offsets, int64_t nseg, T init, T* out, const Device* d,
+                         int64_t blocks, unsigned* counters, void* scratch, cudaStream_t s, const char* what) {
     const int64_t nwarps = blocks * kSegWarps;
     src.set_share(nseg + 1, nwarps);
-    unsigned* counters = nullptr;
-    void* scratch = nullptr;
-    HYD_TRY(workspace(s, (size_t)nwarps * 24, &counters, &scratch));
     SegPartials<T> part;
     part.head = static_cast<T*>(scratch);
     part.tail = part.head + nwarps;
     part.closes = reinterpret_cast<int64_t*>(part.tail + nwarps);
-    part.bad = counters + kSegCounterWord;
-    part.done = counters + kSegCounterWord + 1;
-    part.by_lanes = counters + kSegCounterWord + 2;
+    part.bad = counters;
+    part.done = counters + 1;
+    part.by_lanes = counters + 2;
     auto k = segsum_kernel<T, Src>;
     constexpr size_t kSmem = kSegWarps * (size_t)(Src::kStageBytes ? 2 * Src::kStageBytes : kSegC * (int)sizeof(T));
     HYD_TRY(configure_kernel((const void*)k, d, false));
@@ -851,13 +853,47 @@ static int segsum_launch(Src src, const int64_t* offsets, int64_t nseg, int64_t 
 }
 
 // The SpMV with the default row split (sparse.cu checks the arguments).
+// HYD_CUDA_ERR_UNSUPPORTED, with nothing launched, where 8 lanes per row have to
+// do: that form is one launch without scratch, so that calls may overlap in any
+// way.  This one's scratch lies between its two launches.  Threads that share a
+// stream take turns with both, and no other call uses the scratch; but a graph
+// may be replayed on any stream, and a handle of the per-thread default stream
+// stands for many.
 template <class C>
 int spmv_segsum(int64_t nrows, int64_t ncols, const long long* row_ptr, const C* cols, const double* vals,
                 const double* x, double* y, cudaStream_t s) {
     const bool vec = ((reinterpret_cast<uintptr_t>(cols) | reinterpret_cast<uintptr_t>(vals)) & 31) == 0;
     const SegProduct<C> src{cols, vals, x, row_ptr, nrows, ncols, vec};
-    return segsum_launch<double>(src, reinterpret_cast<const int64_t*>(row_ptr), nrows, INT64_MAX / 2, 0.0, y, s,
-                                 "spmv_csr");
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (s == cudaStreamPerThread || cudaStreamIsCapturing(s, &capturing) != cudaSuccess) {
+        cudaGetLastError();
+        return HYD_CUDA_ERR_UNSUPPORTED;
+    }
+    if (capturing != cudaStreamCaptureStatusNone) return HYD_CUDA_ERR_UNSUPPORTED;
+    Device* d = nullptr;
+    HYD_TRY(device(&d));
+    const int64_t blocks = segsum_blocks<SegProduct<C>>(d, nrows, INT64_MAX / 2);
+    constexpr size_t kCounters = 256;
+    std::lock_guard<std::mutex> lock(d->spmv_mu);
+    Workspace& w = d->spmv_ws[s];
+    if (!w.base) {
+        const size_t bytes = kCounters + segsum_bytes((int64_t)d->sm_count * SegProduct<C>::kCtasPerSm);
+        // (relaxed: a capture that another thread has under way is not disturbed)
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        void* p = nullptr;
+        const cudaError_t e = cudaMalloc(&p, bytes);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return HYD_CUDA_ERR_UNSUPPORTED;
+        }
+        w.base = static_cast<unsigned char*>(p);
+        w.bytes = bytes;
+        HYD_CUDA_TRY(cudaMemsetAsync(p, 0, kCounters, s));
+    }
+    return segsum_launch<double>(src, reinterpret_cast<const int64_t*>(row_ptr), nrows, 0.0, y, d, blocks,
+                                 reinterpret_cast<unsigned*>(w.base), w.base + kCounters, s, "spmv_csr");
 }
 template int spmv_segsum<long long>(int64_t, int64_t, const long long*, const long long*, const double*,
                                     const double*, double*, cudaStream_t);
@@ -875,7 +911,14 @@ static int segreduce_launch(const int64_t* offsets, int64_t n_offsets, const T* 
     if (nseg == 0) return HYD_CUDA_OK;
     HYD_CHECK_ARG(n_vals <= (int64_t)4096 * 0x7fffffffLL, "%s: too many values", what);
     const SegPlain<T> src{vals, n_vals, (reinterpret_cast<uintptr_t>(vals) & 31) == 0, 0};
-    return segsum_launch<T>(src, offsets, nseg, n_vals, init, out, as_stream(stream), what);
+    Device* d = nullptr;
+    HYD_TRY(device(&d));
+    const int64_t blocks = segsum_blocks<SegPlain<T>>(d, nseg, n_vals);
+    unsigned* counters = nullptr;
+    void* scratch = nullptr;
+    HYD_TRY(workspace(as_stream(stream), segsum_bytes(blocks), &counters, &scratch));
+    return segsum_launch<T>(src, offsets, nseg, init, out, d, blocks, counters + kSegCounterWord, scratch,
+                            as_stream(stream), what);
 }
 
 }  // namespace hyd

@@ -354,7 +354,10 @@ template <class C>
 static int spmv_dispatch(int g, int64_t nrows, const long long* row_ptr, const C* col_idx, const double* vals,
                          const double* x, int64_t ncols, double* y, const Device* d, cudaStream_t stream) {
     if (g == 0) {
-        if (nrows >= kSpmvSegMinRows) return spmv_segsum<C>(nrows, ncols, row_ptr, col_idx, vals, x, y, stream);
+        if (nrows >= kSpmvSegMinRows) {
+            const int st = spmv_segsum<C>(nrows, ncols, row_ptr, col_idx, vals, x, y, stream);
+            if (st != HYD_CUDA_ERR_UNSUPPORTED) return st;
+        }
         g = 8;
     }
     int64_t blocks = (nrows * g + 255) / 256;

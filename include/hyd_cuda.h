@@ -352,7 +352,8 @@ int hyd_cuda_csr_from_sorted_coo_i64(int64_t nrows, int64_t nnz, const int64_t* 
 /* SpMV y = A x over CSR (bench/spmv/spmv.hyd:30-40): lanes_per_row lanes (power
  * of two <= 32) share a row with fma partial sums and a fixed xor tree; 0
  * chooses: 8 lanes per row, or from 3 * 2^18 rows on, where their lengths are
- * uneven, an even split of the entries over the GPU.  Every form is deterministic and within
+ * uneven, an even split of the entries over the GPU (not while the stream is
+ * being captured).  Every form is deterministic and within
  * 1e-12 of sum |v*x| of the sequential C sum.
  * A column outside [0, ncols) is skipped and reported. */
 int hyd_cuda_spmv_csr_f64(int64_t nrows, int64_t ncols, const int64_t* row_ptr, const int64_t* col_idx,

@@ -222,3 +222,80 @@ def test_spmv_even_rows_and_a_few_long_ones(hc, orc, dev, per_row, long, count, 
     even = torch.arange(nrows + 1, device=dev) * per_row
     now = _us(lambda: hc.spmv_csr(rp, ci, v, xt, y))
     assert now <= 2 * _us(lambda: hc.spmv_csr(even, ci, v, xt, y)) + long / 8 * 0.4 / 5
+
+
+def _big_matrix(dev, seed):
+    """Row pointers, columns and values of an uneven matrix that the even split takes."""
+    rng = np.random.default_rng(seed)
+    nrows = (3 << 18) + 5
+    row_ptr, cols, vals, x = _csr(rng, nrows, 9001, "zipf")
+    return (torch.from_numpy(row_ptr).to(dev), torch.from_numpy(cols).to(dev), torch.from_numpy(vals).to(dev),
+            torch.from_numpy(x).to(dev))
+
+
+def test_spmv_first_call_on_a_stream_is_captured(hc, dev):
+    """A captured SpMV needs nothing prepared, keeps no scratch of the stream it
+    was captured on, and gives the sums of 8 lanes per row."""
+    rp, ci, v, x = _big_matrix(dev, 8)
+    y = torch.full((len(rp) - 1,), -7.0, dtype=torch.float64, device=dev)
+    want = torch.empty_like(y)
+    hc.spmv_csr(rp, ci, v, x, want, lanes_per_row=8)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=torch.cuda.Stream()):
+        hc.spmv_csr(rp, ci, v, x, y)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+
+
+def test_spmv_does_not_disturb_a_capture_on_another_stream(hc, dev):
+    rp, ci, v, x = _big_matrix(dev, 9)
+    y, one = torch.empty(len(rp) - 1, dtype=torch.float64, device=dev), torch.zeros(1, device=dev)
+    other = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=torch.cuda.Stream()):
+        one.add_(1)
+        hc.spmv_csr(rp, ci, v, x, y, stream=other)  # the first call on that stream
+    g.replay()
+    torch.cuda.synchronize()
+    want = torch.empty_like(y)
+    hc.spmv_csr(rp, ci, v, x, want)
+    assert float(one) == 1.0 and torch.equal(y, want)
+
+
+def test_spmv_from_two_threads_on_one_stream(hc, dev):
+    """Calls of several threads on one stream, with calls that use the stream's
+    workspace between them, give what they give alone."""
+    import threading
+    rp, ci, v, x = _big_matrix(dev, 10)
+    xs = [x, x * 3.0, x - 0.25]
+    alone = []
+    for xk in xs:
+        y = torch.empty(len(rp) - 1, dtype=torch.float64, device=dev)
+        hc.spmv_csr(rp, ci, v, xk, y)
+        alone.append(y)
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    got = [[torch.empty_like(alone[0]) for _ in range(30)] for _ in xs]
+    out = torch.zeros(1, dtype=torch.float64, device=dev)
+
+    def work(k):
+        torch.cuda.set_device(dev)
+        for y in got[k]:
+            hc.spmv_csr(rp, ci, v, xs[k], y, stream=stream)
+
+    def sums():
+        torch.cuda.set_device(dev)
+        for _ in range(60):
+            hc.dot_f64(v, v, out, stream=stream)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(xs))] + [threading.Thread(target=sums)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for k, ys in enumerate(got):
+        assert all(torch.equal(y, alone[k]) for y in ys)
