@@ -71,18 +71,22 @@ __device__ __forceinline__ void coo_load8(const long long* __restrict__ a, int64
 }
 
 // Tile word: {state | heads << 2, sum since the last head}; state 1 the tile's
-// own, 2 of all entries up to the tile's end (TileWord, one 16-byte access).
+// own, 2 of all entries up to the tile's end (TileWord, one 16-byte access), 3
+// none: the tile's look-back gave up.  Such a tile has no place to write to: it
+// writes nothing, nor do those that wait for it, and when the last one is among
+// them the count is 0 (the caller learns of it from the error word).
 __global__ void __launch_bounds__(kCooT, 3)
     coo_sum_kernel(const long long* __restrict__ rows, const long long* __restrict__ cols,
                    const long long* __restrict__ vals, int64_t nnz, bool vec, long long* __restrict__ out_rows,
                    long long* __restrict__ out_cols, long long* __restrict__ out_vals, long long* __restrict__ out_nnz,
-                   TileWord* words, unsigned* ticket, unsigned* err) {
+                   TileWord* words, unsigned* ticket, unsigned limit, unsigned* err) {
     __shared__ long long sh_out[kCooTile];
     __shared__ long long sh_sum[kCooT / 32];   // per warp: the sum since its last head
     __shared__ int sh_heads[kCooT / 32];
     __shared__ long long sh_carry, sh_before;  // of the tile: the open run's sum, the heads before
     __shared__ unsigned sh_tile;
     __shared__ int sh_head0, sh_end;
+    __shared__ bool sh_known;  // the look-back came to its end
     typedef unsigned long long U;  // sums wrap
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) sh_tile = atomicAdd(ticket, 1u);
@@ -162,6 +166,7 @@ __global__ void __launch_bounds__(kCooT, 3)
     }
     if (warp == 0) {
         U before = 0, carry = 0;
+        bool known = true;
         if (tile > 0) {
             if (lane == 0) tile_word_store(&words[tile], 1ull | (U)heads << 2, tsum);
             bool open = true;  // the carry is not complete
@@ -171,15 +176,12 @@ __global__ void __launch_bounds__(kCooT, 3)
                 U f = 2ull, b = 0ull;  // before the first tile: no heads, no sum
                 if (q >= 0) tile_word_load(&words[q], f, b);
                 unsigned spins = 0;
-                bool ok = true;
-                while (__any_sync(0xffffffffu, (f & 3ull) == 0ull)) {
-                    if (++spins > kSpinLimit) {
-                        ok = false;
-                        break;
-                    }
+                while (known && __any_sync(0xffffffffu, (f & 3ull) == 0ull)) {
+                    known = ++spins <= limit;
                     if ((f & 3ull) == 0ull) tile_word_load(&words[q], f, b);
                 }
-                if (!ok) {
+                known = known && !__any_sync(0xffffffffu, (f & 3ull) == 3ull);
+                if (!known) {
                     if (lane == 0) raise_error(err, ERRBIT_TIMEOUT);
                     break;
                 }
@@ -203,13 +205,16 @@ __global__ void __launch_bounds__(kCooT, 3)
             }
         }
         if (lane == 0) {
-            tile_word_store(&words[tile], 2ull | (before + (U)heads) << 2, heads ? tsum : carry + tsum);
+            if (known) tile_word_store(&words[tile], 2ull | (before + (U)heads) << 2, heads ? tsum : carry + tsum);
+            else tile_word_store(&words[tile], 3ull, 0ull);
             sh_before = (long long)before;
             sh_carry = (long long)carry;
-            if (base + kCooTile >= nnz) *out_nnz = (long long)before + heads;
+            sh_known = known;
+            if (base + kCooTile >= nnz) *out_nnz = known ? (long long)before + heads : 0;
         }
     }
     __syncthreads();
+    if (!sh_known) return;
     const int head0 = sh_head0;
     const int nruns = heads - head0 + sh_end;                            // runs that end here
     const int64_t at = sh_before - (head0 ? 0 : 1);                      // the first of them
@@ -700,6 +705,34 @@ static size_t batch_pipeline_rows_table_bytes(const std::vector<BatchInst>& inst
 using namespace hyd;
 
 // ------------------------------------------------------------------ C ABI
+// `left_out`: tiles at the start that no block takes (0 but for the self-test).
+static int coo_sum_launch(const int64_t* rows, const int64_t* cols, const int64_t* vals, int64_t nnz,
+                          int64_t* out_rows, int64_t* out_cols, int64_t* out_vals, int64_t* out_nnz, int left_out,
+                          unsigned limit, cudaStream_t s) {
+    Device* d = nullptr;
+    HYD_TRY(device(&d));
+    const int64_t ntiles = (nnz + kCooTile - 1) / kCooTile;
+    HYD_CHECK_ARG(ntiles <= 0x7fffffffLL, "coo_sum_duplicates: too long");
+    const size_t bytes = 256 + sizeof(TileWord) * (size_t)ntiles;  // the ticket, then the tile words
+    void* scratch = nullptr;
+    HYD_TRY(workspace(s, bytes, nullptr, &scratch));
+    HYD_CUDA_TRY(cudaMemsetAsync(scratch, 0, bytes, s));
+    if (left_out) HYD_CUDA_TRY(cudaMemsetAsync(scratch, left_out, 1, s));  // the first ticket's lowest byte
+    const bool vec = ((reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(cols) |
+                       reinterpret_cast<uintptr_t>(vals)) & 31) == 0;
+    coo_sum_kernel<<<(unsigned)(ntiles - left_out), kCooT, 0, s>>>(
+        (const long long*)rows, (const long long*)cols, (const long long*)vals, nnz, vec, (long long*)out_rows,
+        (long long*)out_cols, (long long*)out_vals, (long long*)out_nnz,
+        reinterpret_cast<TileWord*>(static_cast<unsigned char*>(scratch) + 256), static_cast<unsigned*>(scratch),
+        limit, d->d_err);
+    HYD_TRY(launch_check("coo_sum_duplicates"));
+    int64_t blocks = (nnz + 255) / 256;
+    if (blocks > d->sm_count * 8) blocks = d->sm_count * 8;
+    coo_zero_tail_kernel<<<(unsigned)blocks, 256, 0, s>>>((long long*)out_rows, (long long*)out_cols,
+                                                          (long long*)out_vals, nnz, (const long long*)out_nnz);
+    return launch_check("coo_sum_duplicates");
+}
+
 extern "C" int hyd_cuda_coo_sum_duplicates_i64(const int64_t* rows, const int64_t* cols, const int64_t* vals,
                                                int64_t nnz, int64_t* out_rows, int64_t* out_cols, int64_t* out_vals,
                                                int64_t* out_nnz, void* stream) {
@@ -712,27 +745,18 @@ extern "C" int hyd_cuda_coo_sum_duplicates_i64(const int64_t* rows, const int64_
         HYD_CUDA_TRY(cudaMemsetAsync(out_nnz, 0, 8, s));
         return HYD_CUDA_OK;
     }
-    Device* d = nullptr;
-    HYD_TRY(device(&d));
-    const int64_t ntiles = (nnz + kCooTile - 1) / kCooTile;
-    HYD_CHECK_ARG(ntiles <= 0x7fffffffLL, "coo_sum_duplicates: too long");
-    const size_t bytes = 256 + sizeof(TileWord) * (size_t)ntiles;  // the ticket, then the tile words
-    void* scratch = nullptr;
-    HYD_TRY(workspace(s, bytes, nullptr, &scratch));
-    HYD_CUDA_TRY(cudaMemsetAsync(scratch, 0, bytes, s));
-    const bool vec = ((reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(cols) |
-                       reinterpret_cast<uintptr_t>(vals)) & 31) == 0;
-    coo_sum_kernel<<<(unsigned)ntiles, kCooT, 0, s>>>(
-        (const long long*)rows, (const long long*)cols, (const long long*)vals, nnz, vec, (long long*)out_rows,
-        (long long*)out_cols, (long long*)out_vals, (long long*)out_nnz,
-        reinterpret_cast<TileWord*>(static_cast<unsigned char*>(scratch) + 256), static_cast<unsigned*>(scratch),
-        d->d_err);
-    HYD_TRY(launch_check("coo_sum_duplicates"));
-    int64_t blocks = (nnz + 255) / 256;
-    if (blocks > d->sm_count * 8) blocks = d->sm_count * 8;
-    coo_zero_tail_kernel<<<(unsigned)blocks, 256, 0, s>>>((long long*)out_rows, (long long*)out_cols,
-                                                          (long long*)out_vals, nnz, (const long long*)out_nnz);
-    return launch_check("coo_sum_duplicates");
+    return coo_sum_launch(rows, cols, vals, nnz, out_rows, out_cols, out_vals, out_nnz, 0, kSpinLimit, s);
+}
+
+extern "C" int hyd_cuda_selftest_coo_timeout(const int64_t* rows, const int64_t* cols, const int64_t* vals,
+                                             int64_t nnz, int64_t* out_rows, int64_t* out_cols, int64_t* out_vals,
+                                             int64_t* out_nnz, uint32_t poll_limit, void* stream) {
+    HYD_CHECK_ARG(nnz > kCooTile, "selftest_coo_timeout: needs more than %d entries", kCooTile);
+    HYD_CHECK_ARG(rows && cols && vals && out_rows && out_cols && out_vals && out_nnz,
+                  "selftest_coo_timeout: null buffer");
+    HYD_CHECK_ARG(poll_limit >= 1 && poll_limit <= (1u << 20), "selftest_coo_timeout: poll limit outside 1..2^20");
+    return coo_sum_launch(rows, cols, vals, nnz, out_rows, out_cols, out_vals, out_nnz, 1, poll_limit,
+                          as_stream(stream));
 }
 
 extern "C" int hyd_cuda_csr_from_sorted_coo_i64(int64_t nrows, int64_t nnz, const int64_t* rows, const int64_t* cols,

@@ -57,6 +57,7 @@ SIGNATURES = {
     "hyd_cuda_selftest_div": (_i, [_p, _i, _p, _p, _i64, _p]),
     "hyd_cuda_probe_fp64_rate": (_i, [_i64, _p, C.POINTER(C.c_int64), _p]),
     "hyd_cuda_selftest_timeout": (_i, [_i, C.c_uint32, _p]),
+    "hyd_cuda_selftest_coo_timeout": (_i, [_p, _p, _p, _i64, _p, _p, _p, _p, C.c_uint32, _p]),
     "hyd_cuda_iterate_stencil2d_f64_variant": (_i, [_i, _p, _p, _i64, _i64, _i64, _i, C.POINTER(C.c_int), _p]),
     "hyd_cuda_tune_cache_path": (C.c_char_p, []),
     "hyd_cuda_tune_set_cache_path": (_i, [C.c_char_p]),

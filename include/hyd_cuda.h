@@ -217,6 +217,13 @@ int hyd_cuda_probe_fp64_rate(int64_t iters, double* sink, int64_t* fma_count, vo
  * hyd_cuda_check(stream) returns HYD_CUDA_ERR_TIMEOUT, and the device stays
  * usable.  No counterpart in the reference; for tests. */
 int hyd_cuda_selftest_timeout(int which, uint32_t poll_limit, void* stream);
+/* The same for hyd_cuda_coo_sum_duplicates_i64 (more than 2048 entries): its first
+ * tile of 2048 is left out, so every other one waits for it, at most poll_limit
+ * (1..2^20) polls.  Outputs are zeros and a count of 0, nothing outside them is
+ * written, and the next hyd_cuda_check(stream) returns HYD_CUDA_ERR_TIMEOUT. */
+int hyd_cuda_selftest_coo_timeout(const int64_t* rows, const int64_t* cols, const int64_t* vals, int64_t nnz,
+                                  int64_t* out_rows, int64_t* out_cols, int64_t* out_vals, int64_t* out_nnz,
+                                  uint32_t poll_limit, void* stream);
 /* ---- fused map / zipwith / generate chains -------------------------------------
  * The element loop of a fused chain (bench/map_chain/map_chain.hyd; the C
  * backend's loop body, CodegenC.hs:1328-1353 for the reduced form) with its
