@@ -212,11 +212,13 @@ __global__ void __launch_bounds__(kRangeT, kRangeCtasPerSm)
     for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
     if (lane == 0) sh_part[warp] = part;
     __syncthreads();
-    T carry = T(0);
-#pragma unroll
-    for (int u = 0; u < kRangeWarps; ++u) carry += sh_part[u];
-    for (int u = 0; u < warp; ++u) carry += __ldcg(sums + (int64_t)blockIdx.x * kRangeWarps + u);
-    carry = init + carry;
+    // the prefix is `carry` plus, for the first step, `near`: every addition to the
+    // whole prefix rounds at its size, so the small sums are added to each other first
+    static_assert(kRangeWarps == 8, "the sum below");
+    T carry = init + (((sh_part[0] + sh_part[1]) + (sh_part[2] + sh_part[3])) +
+                      ((sh_part[4] + sh_part[5]) + (sh_part[6] + sh_part[7])));
+    T near = T(0);
+    for (int u = 0; u < warp; ++u) near += __ldcg(sums + (int64_t)blockIdx.x * kRangeWarps + u);
     for (int64_t k = lo; k < end; k += kRangeStep) {
         // to blocked: lane l then holds elements k + 8l .. k + 8l + 7
 #pragma unroll
@@ -231,8 +233,9 @@ __global__ void __launch_bounds__(kRangeT, kRangeCtasPerSm)
         for (int j = 1; j < kRangePer; ++j) x[j] = x[j - 1] + x[j];
         const T incl = warp_inclusive_scan(x[kRangePer - 1]);
         const T left = __shfl_up_sync(0xffffffffu, incl, 1);
-        const T p = lane == 0 ? carry : carry + left;
-        carry = carry + __shfl_sync(0xffffffffu, incl, 31);
+        const T p = carry + (lane == 0 ? near : near + left);
+        carry = carry + (near + __shfl_sync(0xffffffffu, incl, 31));
+        near = T(0);
         if (inclusive) {
 #pragma unroll
             for (int j = 0; j < kRangePer; ++j) x[j] = p + x[j];
@@ -367,7 +370,7 @@ __global__ void __launch_bounds__(kScanT, kScanCtasPerSm) scan_fold_kernel(const
     __shared__ T sh_total[kScanWarps];  // the warps' totals, then their offsets in the tile
     __shared__ T sh_fold[kFoldBuf];
     __shared__ unsigned sh_tile_id;
-    __shared__ T sh_within, sh_before;
+    __shared__ T sh_before;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
         sh_tile_id = atomicAdd(st.tile_counter, 1u);
@@ -386,7 +389,7 @@ __global__ void __launch_bounds__(kScanT, kScanCtasPerSm) scan_fold_kernel(const
     const T incl = warp_inclusive_scan(items[kScanIPT - 1]);
     if (lane == 31) sh_total[warp] = incl;
     __syncthreads();
-    T off = T(0), total = T(0);
+    T off = T(0), total = T(0), within = T(0);  // (within: of the block's tiles before this one)
     if (warp == 0) {
         T agg;
         off = scan_warp_totals(sh_total, agg);
@@ -405,12 +408,9 @@ __global__ void __launch_bounds__(kScanT, kScanCtasPerSm) scan_fold_kernel(const
         }
         if (!ok && lane == 0) raise_error(err, ERRBIT_TIMEOUT);
         const T sc = warp_inclusive_scan(lane < pos ? from_bits<T>(bits) : (lane == pos ? agg : T(0)));
-        const T within = __shfl_sync(0xffffffffu, sc, pos > 0 ? pos - 1 : 0);
+        within = __shfl_sync(0xffffffffu, sc, pos > 0 ? pos - 1 : 0);
         total = __shfl_sync(0xffffffffu, sc, 31);
-        if (lane == 0) {
-            if (pos == 31) tile_word_store(&bst.word[blk], 1ull, to_bits(total));
-            sh_within = within;
-        }
+        if (lane == 0 && pos == 31) tile_word_store(&bst.word[blk], 1ull, to_bits(total));
     } else if (warp == 1) {
         T before = init;  // B(blk - 1)
         if (!lookback_fold(bst, blk, init, sh_fold, before) && lane == 0) raise_error(err, ERRBIT_TIMEOUT);
@@ -420,8 +420,8 @@ __global__ void __launch_bounds__(kScanT, kScanCtasPerSm) scan_fold_kernel(const
     if (warp == 0) {
         const T before = sh_before;
         if (pos == 31 && lane == 0) tile_word_store(&bst.word[blk], 2ull, to_bits(before + total));
-        const T prefix = pos == 0 ? before : before + sh_within;
-        if (lane < kScanWarps) sh_total[lane] = prefix + off;
+        // the two small sums first: an addition to the whole prefix rounds at its size
+        if (lane < kScanWarps) sh_total[lane] = before + (pos == 0 ? off : within + off);
     }
     __syncthreads();
     // outputs: the thread's prefix plus its running sums (one addition each)
