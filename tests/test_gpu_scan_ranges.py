@@ -32,3 +32,21 @@ def test_scan_sizes(hc, orc, dev, n, shift):
         assert np.array_equal(oi.cpu().numpy(), orc.scan_i64(xi, -3, rev, inc))
         bound = orc.scan_f64(np.abs(xf), 0.5, rev, inc)
         assert np.all(np.abs(of.cpu().numpy() - orc.scan_f64(xf, 0.5, rev, inc)) <= 1e-12 * np.maximum(bound, 1.0))
+
+
+@pytest.mark.parametrize("n,limit", [(50_000, 2.7), (300_000, 3.4)])
+def test_scan_f64_rounds_few_times_at_the_prefix_size(hc, dev, n, limit):
+    """The largest error of a scan of n positive elements, in units of 2^-53 of
+    the last value, on average over 10 arrays.  A value takes about four
+    roundings at its own size, whatever the tile's (2.2 and 3.0 measured; five
+    and more, with the small sums added to the prefix one by one, gave 3.6 and
+    3.7)."""
+    worst = []
+    for seed in range(10):
+        x = np.random.default_rng(seed).uniform(0, 1, n)
+        t = torch.from_numpy(x).to(dev)
+        out = torch.empty_like(t)
+        hc.scan(t, out, inclusive=True)
+        exact = np.cumsum(x.astype(np.longdouble))
+        worst.append(float(np.abs(out.cpu().numpy().astype(np.longdouble) - exact).max() / exact[-1]) * 2.0 ** 53)
+    assert float(np.mean(worst)) <= limit
