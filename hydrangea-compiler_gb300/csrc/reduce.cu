@@ -132,10 +132,13 @@ __global__ void __launch_bounds__(kRedThreads, kRedBlocksPerSM)
 
 // Short arrays, by one block: no partials through memory and no completion
 // counter.  What counts here is the FP64 pipe of the one SM (a warp instruction
-// holds it for 19 cycles), so there are few warps and each thread keeps one
-// chain of multiply-adds, all its loads in flight.  Per call: 4099 elements 8.2
-// -> 4.1 us, 8192 9.4 -> 6.1, 16384 9.7 -> 8.2 (512 or 1024 threads with eight
-// accumulators each and a tree in every warp: 8.2 at 4099).
+// holds it for 19 cycles), so there are few warps, with all their loads in flight,
+// and no more accumulators per thread than the rounding asks for: four.  With one,
+// 16000 elements in [-1, 1) came out with an error of 0.029 units of 2^-53 of
+// sum |xy| (root mean square), with four 0.019, as in the form for long arrays
+// (0.019); the three additions more cost 0.2 us.  Back to back, against that form
+// with eight accumulators and a tree in every warp: 4099 elements 6.2 -> 3.2 us,
+// 8192 7.7 -> 4.4, 16384 7.7 -> 6.5.
 constexpr int kRedOneThreads = 256;
 constexpr int64_t kRedOneBlock = 16384;
 template <bool kDot, bool kVec>
@@ -145,7 +148,7 @@ __global__ void __launch_bounds__(kRedOneThreads) reduce_one_kernel(const double
     __shared__ double sh[kRedOneThreads];
     constexpr int T = kRedOneThreads, kIn = 4;
     const int t = threadIdx.x;
-    double acc = 0.0;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
     if (kVec) {
         const int nv = n >> 2;
         const bool tail = 4 * nv + t < n;
@@ -161,19 +164,24 @@ __global__ void __launch_bounds__(kRedOneThreads) reduce_one_kernel(const double
 #pragma unroll
             for (int u = 0; u < kIn; ++u)
                 if (v + u * T < nv) {
-                    acc = kDot ? fma(x[u].x, y[u].x, acc) : acc + x[u].x;
-                    acc = kDot ? fma(x[u].y, y[u].y, acc) : acc + x[u].y;
-                    acc = kDot ? fma(x[u].z, y[u].z, acc) : acc + x[u].z;
-                    acc = kDot ? fma(x[u].w, y[u].w, acc) : acc + x[u].w;
+                    acc[0] = kDot ? fma(x[u].x, y[u].x, acc[0]) : acc[0] + x[u].x;
+                    acc[1] = kDot ? fma(x[u].y, y[u].y, acc[1]) : acc[1] + x[u].y;
+                    acc[2] = kDot ? fma(x[u].z, y[u].z, acc[2]) : acc[2] + x[u].z;
+                    acc[3] = kDot ? fma(x[u].w, y[u].w, acc[3]) : acc[3] + x[u].w;
                 }
         }
-        if (tail) acc = kDot ? fma(tx, ty, acc) : acc + tx;
+        if (tail) acc[0] = kDot ? fma(tx, ty, acc[0]) : acc[0] + tx;
     } else {
-#pragma unroll 8
-        for (int i = t; i < n; i += T) acc = kDot ? fma(__ldg(xs + i), __ldg(ys + i), acc) : acc + __ldg(xs + i);
+#pragma unroll 2
+        for (int i = t; i < n; i += 4 * T) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i + u * T < n)
+                    acc[u] = kDot ? fma(__ldg(xs + i + u * T), __ldg(ys + i + u * T), acc[u]) : acc[u] + __ldg(xs + i + u * T);
+        }
     }
-    acc = block_sum<T>(acc, sh);
-    if (t == 0) *out = acc;
+    const double sum = block_sum<T>((acc[0] + acc[1]) + (acc[2] + acc[3]), sh);
+    if (t == 0) *out = sum;
 }
 
 // Blocks for n elements on `sms` SMs: two vectors per thread until every SM has
