@@ -59,3 +59,12 @@ def test_whole_job_aggregate_is_weak_scaling():
     assert abs(bench.whole_job_gbs(4, 2_147_483_648, 10, 0.01) - 4 * one) < 1e-6
     # the aggregate uses the slowest replica's time
     assert bench.whole_job_gbs(2, 100, 1, 2.0) == 2 * 100 / 2.0 / 1e9
+
+
+def test_heat_operation_count_is_the_kernel_s():
+    sys.path.insert(0, ROOT)
+    import bench
+    grid, small, sms = 8192 * 8192, 512 * 512, 152
+    assert [bench.heat_fp64_ops(v, grid, sms) for v in (0, 6, 7, 13, 14, 19)] == [6, 6, 4, 4, 3, 3]
+    assert bench.heat_fp64_ops(20, grid, sms) == 2.75  # `- 4e` of one row in four goes to the integer pipe too
+    assert bench.heat_fp64_ops(20, small, sms) == 3    # one row per thread
