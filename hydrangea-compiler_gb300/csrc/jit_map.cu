@@ -84,13 +84,14 @@ static std::string map_source(const std::string& body, int nin, bool i64, bool w
     // without a reduction no element is added up: FP64 additions bind these
     // kernels before memory does (see map_launch)
     auto add = [&](const std::string& v) { return with_sum ? "acc += (" + A + ")" + v + ";" : std::string(";"); };
+    const std::string BT = std::to_string(kMapThreads), BW = std::to_string(kMapThreads / 32);
     std::string s;
     s += "__device__ __forceinline__ " + T + " hyd_elem(long long i";
     for (int k = 0; k < kMapMaxInputs; ++k) s += ", " + T + " x" + std::to_string(k);
     s += ") {\n  " + T + " v = " + zero + ";\n  (void)i;\n";
     for (int k = 0; k < kMapMaxInputs; ++k) s += "  (void)x" + std::to_string(k) + ";\n";
     s += "  {\n" + body + "\n  }\n  return v;\n}\n";
-    s += "extern \"C\" __global__ void __launch_bounds__(256) hyd_map_kernel(";
+    s += "extern \"C\" __global__ void __launch_bounds__(" + BT + ") hyd_map_kernel(";
     for (int k = 0; k < kMapMaxInputs; ++k) s += "const " + T + "* __restrict__ p" + std::to_string(k) + ", ";
     s += "long long n, " + T + "* __restrict__ out, " + A + "* __restrict__ partials, unsigned int* counter, " + A +
          "* __restrict__ sum, int vec) {\n"
@@ -101,7 +102,7 @@ static std::string map_source(const std::string& body, int nin, bool i64, bool w
          "    const long long nq = n >> 2;\n"
          "    long long q = 2LL * blockIdx.x * blockDim.x + threadIdx.x;\n"
          "    for (; q < nq; q += 2 * nt) {\n"
-         "      const bool two = q + 256 < nq;\n";
+         "      const bool two = q + " + BT + " < nq;\n";
     // 32-byte vectors, two per lane per step (8 elements), all loads first
     const std::string LD = i64 ? "ld.global.nc.L1::no_allocate.v4.u64" : "ld.global.nc.L1::no_allocate.v4.f64";
     const std::string ST = i64 ? "st.global.v4.u64" : "st.global.v4.f64";
@@ -116,7 +117,7 @@ static std::string map_source(const std::string& body, int nin, bool i64, bool w
                      " {%0,%1,%2,%3}, [%4];\" : \"=" + RC + "\"(a" + ks + "[" + std::to_string(4 * h) + "]), \"=" + RC +
                      "\"(a" + ks + "[" + std::to_string(4 * h + 1) + "]), \"=" + RC + "\"(a" + ks + "[" +
                      std::to_string(4 * h + 2) + "]), \"=" + RC + "\"(a" + ks + "[" + std::to_string(4 * h + 3) +
-                     "]) : \"l\"(p" + ks + " + 4 * (q + " + hs + " * 256)));\n";
+                     "]) : \"l\"(p" + ks + " + 4 * (q + " + hs + " * " + BT + ")));\n";
                 if (h) s += "      else { a" + ks + "[4] = a" + ks + "[5] = a" + ks + "[6] = a" + ks + "[7] = " + zero + "; }\n";
             }
         } else {
@@ -125,13 +126,13 @@ static std::string map_source(const std::string& body, int nin, bool i64, bool w
     }
     s += "      " + T + " w[8];\n"
          "      #pragma unroll\n"
-         "      for (int u = 0; u < 8; ++u) w[u] = hyd_elem(4 * (q + (u >> 2) * 256) + (u & 3)";
+         "      for (int u = 0; u < 8; ++u) w[u] = hyd_elem(4 * (q + (u >> 2) * " + BT + ") + (u & 3)";
     for (int k = 0; k < kMapMaxInputs; ++k) s += ", a" + std::to_string(k) + "[u]";
     s += ");\n"
          "      if (out) {\n"
          "        asm volatile(\"" + ST + " [%0], {%1,%2,%3,%4};\" :: \"l\"(out + 4 * q), \"" + RC + "\"(w[0]), \"" +
          RC + "\"(w[1]), \"" + RC + "\"(w[2]), \"" + RC + "\"(w[3]) : \"memory\");\n"
-         "        if (two) asm volatile(\"" + ST + " [%0], {%1,%2,%3,%4};\" :: \"l\"(out + 4 * (q + 256)), \"" + RC +
+         "        if (two) asm volatile(\"" + ST + " [%0], {%1,%2,%3,%4};\" :: \"l\"(out + 4 * (q + " + BT + ")), \"" + RC +
          "\"(w[4]), \"" + RC + "\"(w[5]), \"" + RC + "\"(w[6]), \"" + RC + "\"(w[7]) : \"memory\");\n"
          "      }\n"
          "      #pragma unroll\n"
@@ -184,14 +185,14 @@ static std::string map_source(const std::string& body, int nin, bool i64, bool w
          "  }\n"
          "  if (sum == 0) return;\n"
          // fixed shuffle tree per warp, warps in order per block, blocks in order by the last block
-         "  __shared__ " + A + " wsum[8];\n"
+         "  __shared__ " + A + " wsum[" + BW + "];\n"
          "  __shared__ bool last;\n"
          "  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);\n"
          "  if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = acc;\n"
          "  __syncthreads();\n"
          "  if (threadIdx.x == 0) {\n"
          "    " + A + " b = 0;\n"
-         "    for (int w = 0; w < 8; ++w) b += wsum[w];\n"
+         "    for (int w = 0; w < " + BW + "; ++w) b += wsum[w];\n"
          "    partials[blockIdx.x] = b;\n"
          "    __threadfence();\n"
          "    last = atomicAdd(counter, 1u) == gridDim.x - 1;\n"
