@@ -133,12 +133,12 @@ __global__ void __launch_bounds__(kRedThreads, kRedBlocksPerSM)
 // Short arrays, by one block: no partials through memory and no completion
 // counter.  What counts here is the FP64 pipe of the one SM (a warp instruction
 // holds it for 19 cycles), so there are few warps, with all their loads in flight,
-// and no more accumulators per thread than the rounding asks for: four.  With one,
-// 16000 elements in [-1, 1) came out with an error of 0.029 units of 2^-53 of
-// sum |xy| (root mean square), with four 0.019, as in the form for long arrays
-// (0.019); the three additions more cost 0.2 us.  Back to back, against that form
-// with eight accumulators and a tree in every warp: 4099 elements 6.2 -> 3.2 us,
-// 8192 7.7 -> 4.4, 16384 7.7 -> 6.5.
+// and each thread adds 16 elements in one chain before it adds the chain to the
+// ones before: with one chain for all, 16000 elements in [-1, 1) came out with an
+// error of 0.029 units of 2^-53 of sum |xy| (root mean square), so with 0.019, as
+// in the form for long arrays (0.019).  Per call: 4099 elements 8.2 -> 4.1 us (four
+// accumulators all along: 5.8), 8192 9.4 -> 6.1, 16384 9.7 -> 8.2 (512 or 1024
+// threads with eight accumulators each and a tree in every warp: 8.2 at 4099).
 constexpr int kRedOneThreads = 256;
 constexpr int64_t kRedOneBlock = 16384;
 template <bool kDot, bool kVec>
@@ -148,12 +148,12 @@ __global__ void __launch_bounds__(kRedOneThreads) reduce_one_kernel(const double
     __shared__ double sh[kRedOneThreads];
     constexpr int T = kRedOneThreads, kIn = 4;
     const int t = threadIdx.x;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    double acc = 0.0;
     if (kVec) {
         const int nv = n >> 2;
         const bool tail = 4 * nv + t < n;
         const double tx = tail ? xs[4 * nv + t] : 0.0, ty = kDot && tail ? ys[4 * nv + t] : 0.0;
-        for (int v = t; v < nv; v += kIn * T) {
+        auto chain = [&](int v) {
             f64x4 x[kIn], y[kIn];
 #pragma unroll
             for (int u = 0; u < kIn; ++u)
@@ -161,27 +161,33 @@ __global__ void __launch_bounds__(kRedOneThreads) reduce_one_kernel(const double
                     x[u] = ldg_stream_f64x4(xs + 4 * (v + u * T));
                     if (kDot) y[u] = ldg_stream_f64x4(ys + 4 * (v + u * T));
                 }
+            double c = 0.0;
 #pragma unroll
             for (int u = 0; u < kIn; ++u)
                 if (v + u * T < nv) {
-                    acc[0] = kDot ? fma(x[u].x, y[u].x, acc[0]) : acc[0] + x[u].x;
-                    acc[1] = kDot ? fma(x[u].y, y[u].y, acc[1]) : acc[1] + x[u].y;
-                    acc[2] = kDot ? fma(x[u].z, y[u].z, acc[2]) : acc[2] + x[u].z;
-                    acc[3] = kDot ? fma(x[u].w, y[u].w, acc[3]) : acc[3] + x[u].w;
+                    c = kDot ? fma(x[u].x, y[u].x, c) : c + x[u].x;
+                    c = kDot ? fma(x[u].y, y[u].y, c) : c + x[u].y;
+                    c = kDot ? fma(x[u].z, y[u].z, c) : c + x[u].z;
+                    c = kDot ? fma(x[u].w, y[u].w, c) : c + x[u].w;
                 }
-        }
-        if (tail) acc[0] = kDot ? fma(tx, ty, acc[0]) : acc[0] + tx;
+            return c;
+        };
+        if (t < nv) acc = chain(t);
+        for (int v = t + kIn * T; v < nv; v += kIn * T) acc += chain(v);
+        if (tail) acc = kDot ? fma(tx, ty, acc) : acc + tx;
     } else {
-#pragma unroll 2
-        for (int i = t; i < n; i += 4 * T) {
+        for (int i0 = t; i0 < n; i0 += 4 * kIn * T) {
+            double c = 0.0;
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (i + u * T < n)
-                    acc[u] = kDot ? fma(__ldg(xs + i + u * T), __ldg(ys + i + u * T), acc[u]) : acc[u] + __ldg(xs + i + u * T);
+            for (int u = 0; u < 4 * kIn; ++u) {
+                const int i = i0 + u * T;
+                if (i < n) c = kDot ? fma(__ldg(xs + i), __ldg(ys + i), c) : c + __ldg(xs + i);
+            }
+            acc += c;
         }
     }
-    const double sum = block_sum<T>((acc[0] + acc[1]) + (acc[2] + acc[3]), sh);
-    if (t == 0) *out = sum;
+    acc = block_sum<T>(acc, sh);
+    if (t == 0) *out = acc;
 }
 
 // Blocks for n elements on `sms` SMs: two vectors per thread until every SM has
