@@ -744,7 +744,7 @@ def suite_segmented_reduce(hc, torch, peak, steps=20):
                      "values (seed 43), longest %d" % (nseg, int(lens.max())),
            "segments": nseg, "ms": round(ms, 4), "GB_s": round(gbs, 1), "frac_of_hbm_peak": round(gbs / peak, 3),
            "algorithmic_bytes": alg, "run_to_run_identical": bool(torch.equal(first, outv)),
-           "launches_per_step": 2, "note": "the values by equal shares per warp, then a kernel that adds the pieces crossing warps"}
+           "launches_per_step": 2, "note": "values and segment ends by equal shares per warp, then a kernel that adds the pieces crossing warps"}
     try:
         from oracle import oracle as O
         hv = vals.cpu().numpy()

@@ -151,8 +151,8 @@ __device__ __forceinline__ void raise_error(unsigned* err, unsigned bit) { atomi
 // integers using multiplication", 1994): with 2^(l-1) < d < 2^l and
 // m = floor(2^(63+l) / d) + 1 (below 2^64), floor(u / d) is the high word of
 // m * u shifted right by l - 1 for every u <= 2^63; and the same with 31 for 63
-// in 32 bits.  (The compiler's 64-bit division is a loop of about a hundred
-// instructions: it, not memory, bound the histogram over 1000 bins.)
+// in 32 bits.  (The 64-bit division that `%` compiles to, not memory, bound the
+// histogram over 1000 bins: 2e7 values 54 us with it, 37 so.)
 struct DivMod64 {
     long long d;
     unsigned long long mask;

@@ -10,7 +10,9 @@
 // the FP64 instructions):
 //  * a fixed grid of 2 blocks x 512 threads per SM; thread t owns the 32-byte
 //    vectors t, t+S, t+2S, ... (S = total threads) in two chains of
-//    multiply-adds, with four 256-bit loads in flight per thread;
+//    multiply-adds, with four 256-bit loads in flight per thread (eight
+//    accumulators round no better: 3e5 elements in [-1, 1) 0.0048 units of 2^-53
+//    of sum |xy| with them, 0.0041 so, root mean square);
 //  * per-thread order, the halving through shared memory, the last warp's tree
 //    and the final combine are all fixed, so a given (n, device) always produces the
 //    same bits (the C backend's result instead depends on the thread count);

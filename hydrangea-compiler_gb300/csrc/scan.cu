@@ -26,12 +26,15 @@
 // tree).  A parallel prefix cannot reproduce the serial fold's roundings; the
 // tolerance is |gpu - c| <= 1e-12 * prefix sum of |x| (stated in the tests).
 // FP64 bounds it: 2.3 additions per element (15 + 5 + 2 + 16 per thread of 16),
-// 586 us of the 744 us at 2^27 (812 with 8 per thread, 2.6 additions, the two
-// levels of the look-back one after the other and no prefetch).
+// 586 us of the 735 us at 2^27 (812 with 8 per thread, 2.6 additions, the two
+// levels of the look-back one after the other and no prefetch).  The chains of 16
+// do not show in the errors, whose size the few additions to the whole prefix
+// set: largest one of 2^24 positive elements 4.5 units of 2^-53 of the last value
+// with 8 per thread, 4.4 now.
 //
 // Tiles pass through shared memory padded with one slot per 16 elements, so
-// the blocked (8 consecutive elements per thread) and striped accesses are
-// free of bank conflicts.
+// the blocked (16 consecutive elements per thread, 8 per lane in the two-launch
+// form) and striped accesses are free of bank conflicts.
 //
 // Reverse scans read and write index n-1-k for logical position k, exactly the
 // ix the reference's lowering computes.
@@ -256,7 +259,7 @@ __global__ void __launch_bounds__(kRangeT, kRangeCtasPerSm)
     }
 }
 
-// Bytes of scratch, and the launches (`scratch`: 8-byte aligned).
+// Blocks, and the launches (`scratch`: one 8-byte word per warp).
 static int64_t range_blocks(const Device* d, int64_t n) {
     const int64_t want = (n + kRangeStep * kRangeWarps - 1) / (kRangeStep * kRangeWarps);
     const int64_t cap = (int64_t)d->sm_count * kRangeCtasPerSm;

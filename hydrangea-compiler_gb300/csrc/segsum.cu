@@ -30,6 +30,11 @@
 // FP64 lane slots per entry.  Three blocks per SM (80 registers) beat four (64
 // and spills): 1014 against 1327 us on one-value segments when that was tried.
 //
+// Errors, root mean square in units of 2^-53 of a sum's magnitudes, against
+// tiles with a look-back (segments) and 8 lanes per row: segments of 300 positive
+// values 0.88 and 0.80, of 10^6 4.4 and 0.77; rows of 12 positive products 0.67
+// and 0.73, of Zipf length 0.59 and 0.60, of Zipf length with signs 0.42 and 0.39.
+//
 // Offsets that are not an ascending partition of [0, n_vals] are detected on
 // the way (every adjacent pair is looked at by exactly one warp); the second
 // kernel then computes every segment on its own, with the reference's

@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(bk_place_threads<kCap>(), bk_place_per_sm<kCap
     constexpr unsigned kColMask = (1u << kBkColBits) - 1u, kRankMask = (kBinMax - 1u) << kRankAt;
     static_assert(kCap <= (1 << kIdx), "entry and bin numbers must fit their field");
     uint4* const rec = reinterpret_cast<uint4*>(bkw_smem);
-    unsigned* const ord = reinterpret_cast<unsigned*>(rec + kCap);  // rank << 29 | col << 11 | entry, by bin
+    unsigned* const ord = reinterpret_cast<unsigned*>(rec + kCap);  // rank | column | entry number, by bin (kRankAt, kIdx)
     unsigned* const cntw = ord + kCap + 4;                          // two 16-bit counts per word
     const unsigned short* const start = reinterpret_cast<const unsigned short*>(cntw);
     unsigned* const rowinfo = cntw + kCap / 2;  // start | length << 16
@@ -924,7 +924,7 @@ __global__ void __launch_bounds__(kBkWarps * 32, kBkWarpPerSm) bk_bucket_radix_k
 
 // Large buckets (up to 64 rows x 256): one CTA sorts the bucket's keys with a
 // block-wide bitonic network in shared memory.  Reads its item count from
-// device memory (filled by the warp sort).
+// device memory (filled by the placing kernels).
 constexpr size_t kBkSmem = (size_t)kBkCap * 6 + 1024;
 
 __global__ void __launch_bounds__(kBkThreads) bk_bucket_kernel(const BkInst* __restrict__ inst,

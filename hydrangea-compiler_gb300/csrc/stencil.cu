@@ -15,14 +15,15 @@
 // is exact -- `t3 - 4e` and `t3 + e*-4` are one fma because 4e is exact (for
 // |e| < DBL_MAX/4), and /4.0 is *0.25 (both correctly rounded, same value).
 //
-// GB300 design.  FP64 runs at 1.7 operations per clock and SM on this part, so
+// GB300 design.  FP64 runs at 1.68 operations per clock and SM on this part, so
 // a 5-point fp64 step is bound by the FP64 pipe (6 operations per point for
 // HEAT: 768 us per step at 8192^2), not by HBM (158 us).  The default kernel
 // therefore does the neighbour sum on the integer pipe, exactly (fp64_emu.cuh),
 // sweeping rows of a column per thread: HEAT 369 us per step, its FP64 pipe
-// (2.75 operations per point) and its ALU pipe both near 90% busy, JACOBI 312,
-// HEAT_EXAMPLE 415; with two additions emulated one by one they took 528, 418
-// and 895.  The tiled kernels bring each tile through shared memory:
+// (2.75 operations per point) 80% and its ALU pipe 76% busy (the first step on
+// random data 450: some operands lie outside the grid and take the FP64 unit),
+// JACOBI 312, HEAT_EXAMPLE 415; with two additions emulated one by one they took
+// 528, 418 and 895.  The tiled kernels bring each tile through shared memory:
 //  * a persistent grid walks 16 x 128 output tiles; each tile plus its halo
 //    (rows -1..+1, columns -2..+2 so the TMA x coordinate stays 16-byte
 //    aligned) is brought into shared memory by a 2-D TMA load
